@@ -271,7 +271,8 @@ PKCUDA_API int pk_system_adjoint_step(pk_system* sys, const pk_step_params* para
 PKCUDA_API int pk_system_set_refinement(pk_system* sys, int passes);
 /* The PCG kernel of the last solve: 0 ring-staged, 1 TMA-staged, 2 unstaged, 3
  * part-resident, 4 per-body batch kernel, 5 part-resident with one group of parts per body
- * (batched solve); -1 before the first solve (or a negative PK_ERR_*).
+ * (batched solve); where the whole matrix fits the SMs' on-chip memory, the resident
+ * kernel runs as 3 and 5 (FP32 storage) and as 0 (FP64); -1 before the first solve (or a negative PK_ERR_*).
  * blocks (may be NULL) receives the blocks it ran on. */
 PKCUDA_API int pk_system_pcg_kernel(pk_system* sys, int* blocks);
 /* Stream form of the part-resident kernel's layout in the last solve: 0 full symmetric
@@ -364,6 +365,16 @@ PKCUDA_API int pk_slab_plan_selfcheck(int n, const int* row_start, const int* co
 PKCUDA_API int pk_slab_plan_batched_selfcheck(int n, const int* row_start, const int* col_index, const double* values,
                                               const double* x, const double* coords, const int* segment_row_start,
                                               int segment_count, int max_blocks, int form, double* y, int* info);
+
+/* CPU self-check of the resident PCG kernel's layout (its rows stay on chip for the whole
+ * solve): builds it for the upper BSR of segment_count bodies on at most max_blocks blocks
+ * in the precision's storage, checks what the kernel checks, and evaluates y = A x as its
+ * lanes do.  info (may be NULL) receives {parts, most rows of a part, lanes per row, bytes
+ * of shared memory}.  PK_ERR_UNSUPPORTED when the matrix does not fit on chip.  No
+ * counterpart in the reference (it checks this library's own layout). */
+PKCUDA_API int pk_res_plan_selfcheck(int n, const int* row_start, const int* col_index, const double* values,
+                                     const double* x, const double* coords, const int* segment_row_start,
+                                     int segment_count, int max_blocks, int precision, double* y, int* info);
 
 /* Builds the transposed index of an upper BSR: for row r the blocks (c, r), c < r.
  * lt_start[n+1]; lt_row / lt_block sized nnz - n.  Host-only, no device needed. */

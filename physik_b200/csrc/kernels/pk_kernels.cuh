@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include "pk_math.cuh"
+#include "pk_res_plan.h"
 #include "pk_slab_plan.h"
 
 namespace pk {
@@ -406,6 +407,52 @@ struct SlabPcgArgs {
     int sym;
 };
 
+// ------------------------------------------------------------------ resident PCG
+// The resident PCG kernel (pk_pcg_res.cu; layout in pk_res_plan.h): one block per part,
+// the part's rows on chip for the whole solve, one exchange per iteration.
+template <class Real>
+struct ResPcgArgs {
+    int n;
+    int lpr;                         // lanes per row: 1, 2, 4 or 8
+    int nslots;                      // slots per thread
+    int max_halo;                    // most halo rows of a part (clusters: the inbox's rows)
+    const int* part_info;            // [grid] x kResPartInts
+    const int* perm;                 // part order -> dynamic row
+    const int* halo_src;
+    int halo_count;
+    const int2* send;                // rows to send {row of the part, place}, part by part
+    const unsigned* src;             // [part's slots][thread]
+    const unsigned short* col;
+    int slot_count;
+    int nnz;
+    unsigned smem_bytes;             // dynamic shared memory of the launch
+    const Real* values;              // the assembled system
+    const Real* b;
+    const Real* minv;
+    Real* x;                         // per dynamic row: delta-v out
+    // exchange through global memory (not in clusters)
+    unsigned char* rows_in;          // [2][halo_count] tagged q rows (16 bytes each; 32 in FP64)
+    unsigned char* sums_in;          // [2][grid][sender] x kResSlotBytes: tagged sums
+    size_t sums_stride;              // bytes of one block's inbox: the largest group's senders
+    unsigned* epoch;                 // [grid] tag base of the group starting at each block
+    int max_iterations;
+    double tolerance;
+    int skip_on_flags;
+    int integrate;
+    Real dt;
+    const int* dyn_to_node;
+    Real* node_x;
+    Real* node_v;
+    unsigned* flags;
+    DevStats* stats;
+    // per-body solves (see SlabPcgArgs)
+    int grouped;
+    int nbodies;
+    BatchBodyStats* body_stats;
+    unsigned* missing;
+};
+constexpr int kResSlotBytes = 64;    // four 16-byte packets
+
 // ------------------------------------------------------------------ FP64 refinement
 // Kernels of the outer true-residual refinement (pk_refine.cu).
 constexpr int kRefineThreads = 256;
@@ -553,6 +600,14 @@ int pcg_slab_max_grid();
 cudaError_t launch_slab_fill_kernel(const float* values, int nnz, const int* tile_desc, const int* tile_entry0,
                                     int ntiles, const unsigned* fill_src, int nentries, float* stream,
                                     unsigned long long stream_floats, int sym, cudaStream_t stream_);
+
+// Resident PCG (pk_pcg_res.cu): `grid` blocks of `threads`, in clusters of `cluster` blocks
+// or, with 0, as a cooperative launch.
+template <class Real>
+cudaError_t launch_pcg_res_kernel(const ResPcgArgs<Real>& args, int threads, int cluster, int grid,
+                                  cudaStream_t stream);
+template <class Real>
+ResLimits pcg_res_limits();
 
 constexpr int kPcgThreads = 512;
 

@@ -1,0 +1,973 @@
+// pk_pcg_res.cu -- the resident cooperative block-Jacobi PCG kernel.
+//
+// The solve of the other PCG kernels (SolvePreconditionedConjugateGradient,
+// src/Core/Solvers/Linear/ConjugateGradientSolver.cpp:114-241, with the SpMV of
+// SparseBlockMatrix::Multiply, src/Math/SparseBlockMatrix.cpp:209-268, and
+// World::IntegrateImplicitEuler, src/Core/World/World.cpp:644-695, fused at the end) for
+// systems whose matrix fits the SMs' on-chip memory (pk_res_plan.h).  Such a solve is bound
+// by latency, not by bytes: an iteration of the streaming kernels spends most of its time
+// in two grid exchanges and the loads around them.  Here
+//
+// * every block loads its part's rows once, straight from the assembled blocks, into
+//   shared memory and registers; x, r, s, d and M^-1 of a row stay in the registers of the
+//   lane that owns it.
+// * an iteration has one exchange.  The blocks publish, with the partial sums of d.q, the
+//   rows of q = A d that other parts' windows hold; every block then knows alpha and beta
+//   and updates r, s = M^-1 r and d of its halo rows itself, with the same operations as
+//   their owners (so all copies of a row agree bit for bit).  beta needs r'.s' of the
+//   updated vectors before they exist; it is predicted from sums of the same exchange,
+//       r'.s' = r.s - alpha (q.s + r.z) + alpha^2 q.z,   z = M^-1 q, r' = r - alpha q
+//   (exact in exact arithmetic for any M), and the true r'.s' of the updated vectors is
+//   summed with the next exchange and used for alpha, for the stopping test and for the
+//   next prediction ("predict and recompute", Chen and Carson 2020).  Where the prediction
+//   would cancel (r'.s' below a sixteenth of r.s), near the stopping target and in the last
+//   iteration the true sum is exchanged at once.
+// * through global memory an exchange needs no fence: every value travels in a 16-byte packet with a tag (the
+//   exchange's number), written and read whole.  A sender writes into the inbox of every
+//   reader, so that a reader polls lines nobody else reads, and reads them coalesced.  Two
+//   buffers by parity: a block overwrites exchange g's packets in g + 2, after it has seen
+//   every block's sums of g + 1, which a block sends only when it has read all of g.  Tags
+//   go on from solve to solve (epoch), so nothing is cleared between solves.
+//
+// Measured per CG iteration against the streaming kernels (part-resident stream for FP32
+// storage, ring for FP64): 8x8x8 box FP32 1.8 us (7.2), 32x8x8 beam FP64 3.0 us (13.3),
+// 64x16x16 beam 3.3 us mixed (10.9) and 4.2 us FP64 (18.5).  What is left is a chain of
+// latencies: about 3,000 cycles of a block's own work (product, two sets of FP64 sums by
+// shuffles, the scalars, the updates; 8.6 cycles an FP64 add, 24 a shuffle, 45 a barrier of
+// 512 threads) and the exchange.
+//
+// All sums keep one fixed order: warp shuffles, then the block's warps, then the group's
+// blocks, the same in every block; a run repeats bit for bit.  Sums and scalars are FP64 in
+// every precision.  Every wait is bounded; one that gives up sets the timeout flag, which
+// ends the other blocks' waits.
+#include <cuda_runtime.h>
+#include <float.h>
+#include <math.h>
+#include <stdint.h>
+
+#include <mutex>
+#include <type_traits>
+
+#include "pk_device.cuh"
+
+namespace pk {
+namespace {
+
+constexpr int kResMaxWarps = kResMaxThreads / 32;
+constexpr int kResSums = 4;  // d.q, q.s + r.z, q.z, r.s; at the end r.r in the first
+constexpr int kResSendRegs = 2;
+constexpr unsigned kResSpinLimit = 1u << 22;  // polls of one wait: seconds
+
+struct Packet {
+    unsigned long long lo, hi;
+};
+__device__ __forceinline__ void st_packet(void* p, Packet v)
+{
+    asm volatile(
+        "{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p), "l"(v.lo),
+        "l"(v.hi)
+        : "memory");
+}
+__device__ __forceinline__ Packet ld_packet(const void* p)
+{
+    Packet v;
+    asm volatile(
+        "{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+        : "=l"(v.lo), "=l"(v.hi)
+        : "l"(p)
+        : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned packet_tag(Packet v) { return (unsigned)(v.hi >> 32); }
+
+// A row of q with its tag: one packet in FP32; two in FP64 (96 bits of data and a tag each).
+__device__ __forceinline__ void st_row(unsigned char* p, V3<float> q, unsigned tag)
+{
+    st_packet(p, {(unsigned long long)__float_as_uint(q.x) | ((unsigned long long)__float_as_uint(q.y) << 32),
+                  (unsigned long long)__float_as_uint(q.z) | ((unsigned long long)tag << 32)});
+}
+__device__ __forceinline__ void st_row(unsigned char* p, V3<double> q, unsigned tag)
+{
+    const unsigned long long x = __double_as_longlong(q.x), y = __double_as_longlong(q.y),
+                             z = __double_as_longlong(q.z), t = (unsigned long long)tag << 32;
+    st_packet(p, {x, (y & 0xffffffffull) | t});
+    st_packet(p + 16, {(y >> 32) | (z << 32), (z >> 32) | t});
+}
+__device__ __forceinline__ bool ld_row(const unsigned char* p, unsigned tag, V3<float>& q)
+{
+    const Packet a = ld_packet(p);
+    q = V3<float>{__uint_as_float((unsigned)a.lo), __uint_as_float((unsigned)(a.lo >> 32)),
+                  __uint_as_float((unsigned)a.hi)};
+    return packet_tag(a) == tag;
+}
+__device__ __forceinline__ bool ld_row(const unsigned char* p, unsigned tag, V3<double>& q)
+{
+    const Packet a = ld_packet(p), b = ld_packet(p + 16);
+    q = V3<double>{__longlong_as_double((long long)a.lo),
+                   __longlong_as_double((long long)((a.hi & 0xffffffffull) | (b.lo << 32))),
+                   __longlong_as_double((long long)((b.lo >> 32) | (b.hi << 32)))};
+    return packet_tag(a) == tag && packet_tag(b) == tag;
+}
+
+// The row updates, with every rounding spelled out: owners and halo copies must agree.
+template <class Real>
+__device__ __forceinline__ V3<Real> fma3(Real a, V3<Real> b, V3<Real> c)
+{
+    return V3<Real>{fma(a, b.x, c.x), fma(a, b.y, c.y), fma(a, b.z, c.z)};
+}
+__device__ __forceinline__ V3<float> fma3(float a, V3<float> b, V3<float> c)
+{
+    return V3<float>{__fmaf_rn(a, b.x, c.x), __fmaf_rn(a, b.y, c.y), __fmaf_rn(a, b.z, c.z)};
+}
+template <class Real>
+__device__ __forceinline__ V3<Real> apply_minv(const Real (&m)[9], V3<Real> v)
+{
+    V3<Real> r{m[0] * v.x, m[1] * v.x, m[2] * v.x};
+    r = V3<Real>{fma(m[3], v.y, r.x), fma(m[4], v.y, r.y), fma(m[5], v.y, r.z)};
+    return V3<Real>{fma(m[6], v.z, r.x), fma(m[7], v.z, r.y), fma(m[8], v.z, r.z)};
+}
+// c + a b with the FP64 scalar a: in FP32 a is split into two floats (see SplitAlpha in
+// pk_pcg_slab.cu: within an ulp of the FP64 update, without conversions).
+template <class Real>
+struct Scale;
+template <>
+struct Scale<float> {
+    float hi, lo;
+    __device__ __forceinline__ explicit Scale(double a) : hi(float(a)), lo(float(a - double(float(a)))) {}
+    __device__ __forceinline__ Scale(float h, float l) : hi(h), lo(l) {}
+    __device__ __forceinline__ Scale negated() const { return Scale(-hi, -lo); }
+    __device__ __forceinline__ V3<float> axpy(V3<float> b, V3<float> c) const { return fma3(lo, b, fma3(hi, b, c)); }
+};
+template <>
+struct Scale<double> {
+    double a;
+    __device__ __forceinline__ explicit Scale(double v) : a(v) {}
+    __device__ __forceinline__ Scale negated() const { return Scale(-a); }
+    __device__ __forceinline__ V3<double> axpy(V3<double> b, V3<double> c) const { return fma3(a, b, c); }
+};
+
+// ------------------------------------------------------------------ cluster exchange
+__device__ __forceinline__ unsigned cluster_map(const void* p, unsigned rank)
+{
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_async16(unsigned dst, Packet v, unsigned bar)
+{
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(dst),
+                 "l"(v.lo), "l"(v.hi), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void st_async8(unsigned dst, unsigned long long v, unsigned bar)
+{
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst), "l"(v),
+                 "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void st_async_row(unsigned dst, V3<float> q, unsigned bar)
+{
+    st_async16(dst, {(unsigned long long)__float_as_uint(q.x) | ((unsigned long long)__float_as_uint(q.y) << 32),
+                     (unsigned long long)__float_as_uint(q.z)},
+               bar);
+}
+__device__ __forceinline__ void st_async_row(unsigned dst, V3<double> q, unsigned bar)
+{
+    st_async16(dst, {(unsigned long long)__double_as_longlong(q.x), (unsigned long long)__double_as_longlong(q.y)}, bar);
+    st_async8(dst + 16, (unsigned long long)__double_as_longlong(q.z), bar);
+}
+template <class Real>
+constexpr unsigned row_tx_bytes()
+{
+    return sizeof(Real) == 4 ? 16 : 24;
+}
+// Bounded wait for the phase with the given parity, seeing what cluster peers wrote.
+__device__ __forceinline__ bool cluster_wait(unsigned long long* bar, unsigned parity)
+{
+    for (unsigned i = 0; i < kMbarSpinLimit; ++i) {
+        unsigned ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_addr(bar)), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// MAXT: threads per block at most (256 leaves a thread twice the registers of 512).
+// CL: exchange inside a cluster (else through global memory).
+template <class Real, int MAXT, bool CL>
+__global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
+{
+    constexpr int KR = res_reg_slots(sizeof(Real), MAXT);
+    constexpr int NH = kResHaloPerThread;
+    constexpr int RB = (int)res_row_packet(sizeof(Real));
+    extern __shared__ __align__(128) unsigned char dyn[];
+    // the owner warps' partials and the group's sums, by exchange parity
+    __shared__ double sh_part[2][kResSums * kResMaxWarps];
+    __shared__ double sh_sum[2][kResSums];
+    __shared__ unsigned sh_bits[3], sh_gbits[3];  // flags by exchange number
+    __shared__ __align__(8) unsigned long long sh_bar[2];
+    __shared__ int s_fail;
+
+    const int T = blockDim.x, W = T >> 5, lpr = P.lpr;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, blk = blockIdx.x;
+    const int* pi = P.part_info + (size_t)kResPartInts * blk;
+    const int row0 = __ldg(pi + 0), halo0 = __ldg(pi + 2), slot0 = __ldg(pi + 4), body = __ldg(pi + 8),
+              send0 = __ldg(pi + 9);
+    int m = __ldg(pi + 1), h = __ldg(pi + 3), gfirst = __ldg(pi + 6), gsize = __ldg(pi + 7), sends_n = __ldg(pi + 10);
+    const unsigned in_flags = *(volatile unsigned*)P.flags;
+    const bool skip = P.skip_on_flags && (in_flags & (kFlagPrecomputeFailed | kFlagSingularDiag));
+    const bool idle = CL && gsize == 0;  // a block its cluster has left over
+    unsigned cl_size = 1;
+    if (CL) asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(cl_size));
+    const int cl0 = CL ? blk - blk % (int)cl_size : 0;
+    unsigned bad0 = 0;
+    // A part that does not fit the launch (the host never builds one) is emptied and
+    // reports a breakdown; a block outside its group works alone.
+    if (!idle &&
+        (gfirst < 0 || gsize < 1 || gsize > (CL ? kResMaxCluster : kResMaxParts) || gfirst + gsize > (int)gridDim.x ||
+         blk < gfirst || blk >= gfirst + gsize || (P.grouped && (unsigned)body >= (unsigned)P.nbodies) ||
+         (!P.grouped && (gfirst != 0 || (!CL && gsize != (int)gridDim.x))) ||
+         (CL && (gfirst < cl0 || gfirst + gsize > cl0 + (int)cl_size)))) {
+        gfirst = blk;
+        gsize = 1;
+        bad0 = 4u;
+    }
+    int nslots = P.nslots;
+    if (m < 0 || m * lpr > T || h < 0 || h > NH * T || h > P.max_halo || row0 < 0 || row0 + m > P.n || halo0 < 0 ||
+        halo0 + h > P.halo_count || sends_n < 0 || send0 < 0 || send0 + sends_n > P.halo_count || nslots < 0 || slot0 < 0 || slot0 + nslots > P.slot_count ||
+        res_smem_bytes(sizeof(Real), T, m, h, nslots, CL ? 1 : 0, P.max_halo) > P.smem_bytes) {
+        m = h = nslots = sends_n = 0;
+        bad0 = 4u;
+    }
+    const bool leader = !idle && blk == gfirst;
+    BatchBodyStats* const bs = P.grouped ? P.body_stats + ((unsigned)body < (unsigned)P.nbodies ? body : 0) : nullptr;
+    if (skip) {
+        if (leader && tid == 0) {
+            if (P.grouped) {
+                bs->iterations = 0;
+                bs->converged = 0;
+                bs->residual_norm = 0.0;
+                bs->flags = 0;
+            } else {
+                P.stats->iterations = 0;
+                P.stats->converged = 0;
+                P.stats->residual_norm = 0.0;
+            }
+        }
+        return;
+    }
+    // Inboxes of a cluster (at the same place in every block): sums [parity][sender][sum],
+    // halo rows [parity][row].
+    unsigned char* const sums_in = dyn;
+    unsigned char* const rows_in = dyn + 2 * kResMaxCluster * kResSlotBytes;
+    size_t off = CL ? 2 * (size_t)kResMaxCluster * kResSlotBytes + 2 * (size_t)P.max_halo * RB : 0;
+    const int wn = m + h;
+    Real* const win = reinterpret_cast<Real*>(dyn + off);
+    off += res_align(3 * (size_t)wn * sizeof(Real));
+    Real* const hr = reinterpret_cast<Real*>(dyn + off);  // halo r: [3][h], then M^-1: [9][h]
+    Real* const hm = hr + 3 * (size_t)h;
+    off += res_align(12 * (size_t)h * sizeof(Real));
+    Real* const qbuf = reinterpret_cast<Real*>(dyn + off);  // q of the part's rows
+    off += res_align(3 * (size_t)m * sizeof(Real));
+    // [slot][thread][element]: nine words apart, so a warp's reads hit different banks
+    Real* const vals = reinterpret_cast<Real*>(dyn + off);
+    off += res_align((size_t)max(0, nslots - KR) * T * 9 * sizeof(Real));
+    unsigned short* const cols = reinterpret_cast<unsigned short*>(dyn + off);
+    if (tid == 0) {
+        for (int i = 0; i < 3; ++i) sh_bits[i] = sh_gbits[i] = 0u;
+        s_fail = 0;
+        if (CL) {
+            mbar_init(&sh_bar[0], 1);
+            mbar_init(&sh_bar[1], 1);
+            mbar_fence_init();
+        }
+    }
+    unsigned epoch = 0u;
+    if (!CL && gsize > 1) epoch = *(volatile unsigned*)(P.epoch + gfirst);
+    if (CL)
+        cluster_barrier();  // every block's barriers exist before anybody writes to them
+    else
+        __syncthreads();
+    if (idle) {
+        cluster_barrier();
+        return;
+    }
+
+    // Thread i < m owns row i: its vectors and M^-1 stay in its registers.  Packing the rows
+    // into the first warps keeps the FP64 work of the sums off the others.  The last threads
+    // hold the halo rows.
+    const bool has = tid < m;
+    const int owner_warps = (m + 31) / 32;
+    const int htid = T - 1 - tid;
+    const V3<Real> zero{Real(0), Real(0), Real(0)};
+    int cidx = -1;
+    // the rows this thread sends {row, place}: the first few in registers
+    int2 send[kResSendRegs];
+#pragma unroll
+    for (int u = 0; u < kResSendRegs; ++u)
+        send[u] = tid + u * T < sends_n ? __ldg(P.send + send0 + tid + u * T) : make_int2(-1, -1);
+    V3<Real> xv = zero, rv = zero, sv = zero, dv = zero, qv = zero;
+    Real mi[9];
+#pragma unroll
+    for (int e = 0; e < 9; ++e) mi[e] = Real(0);
+    unsigned bad = bad0;
+    if (has) {
+        cidx = __ldg(P.perm + row0 + tid);
+        if ((unsigned)cidx >= (unsigned)P.n) {
+            cidx = -1;
+            bad |= 4u;
+        } else {
+            rv = ld3(P.b, cidx);
+#pragma unroll
+            for (int e = 0; e < 9; ++e) mi[e] = __ldg(P.minv + 9 * (size_t)cidx + e);
+        }
+    }
+    // Halo rows: r = b and M^-1 in shared memory, d = s in the window.
+#pragma unroll
+    for (int u = 0; u < NH; ++u) {
+        const int j = htid + u * T;
+        if (j < h) {
+            const int g = __ldg(P.halo_src + halo0 + j);
+            int c = 0;
+            if ((unsigned)g < (unsigned)P.n) c = __ldg(P.perm + g);
+            if ((unsigned)g >= (unsigned)P.n || (unsigned)c >= (unsigned)P.n) {
+                c = 0;
+                bad |= 4u;
+            }
+            const V3<Real> b = ld3(P.b, c);
+            Real hmi[9];
+#pragma unroll
+            for (int e = 0; e < 9; ++e) {
+                hmi[e] = __ldg(P.minv + 9 * (size_t)c + e);
+                hm[(size_t)e * h + j] = hmi[e];
+            }
+            hr[j] = b.x;
+            hr[h + j] = b.y;
+            hr[2 * h + j] = b.z;
+            const V3<Real> s = apply_minv(hmi, b);
+            Real* d = win + 3 * (m + j);
+            d[0] = s.x;
+            d[1] = s.y;
+            d[2] = s.z;
+        }
+    }
+    // The part's blocks: the first KR slots in registers, the others in shared memory.
+    Real rval[KR > 0 ? KR : 1][9];
+    int rcol[KR > 0 ? KR : 1];
+    auto load_entry = [&](int slot, Real (&v)[9]) -> int {
+        const size_t at = (size_t)(slot0 + slot) * T + tid;
+        const unsigned s = __ldg(P.src + at);
+        const int c = __ldg(P.col + at);
+        const unsigned k = s & ~kSlabLowerBit;
+        const bool live = s != kSlabNoPos && k < (unsigned)P.nnz;
+        const Real* q = P.values + 9 * (size_t)(live ? k : 0u);
+        Real t[9];
+#pragma unroll
+        for (int e = 0; e < 9; ++e) t[e] = live ? __ldg(q + e) : Real(0);
+        const bool tr = (s & kSlabLowerBit) != 0u;
+#pragma unroll
+        for (int e = 0; e < 9; ++e) v[e] = tr ? t[3 * (e % 3) + e / 3] : t[e];
+        return c + 2 < 3 * wn ? c : 0;
+    };
+#pragma unroll
+    for (int k = 0; k < KR; ++k) {
+        rcol[k] = 0;
+#pragma unroll
+        for (int e = 0; e < 9; ++e) rval[k][e] = Real(0);
+        if (k < nslots) rcol[k] = load_entry(k, rval[k]);
+    }
+#pragma unroll 2
+    for (int k = KR; k < nslots; ++k) {
+        Real v[9];
+        const size_t at = (size_t)(k - KR) * T + tid;
+        cols[at] = (unsigned short)load_entry(k, v);
+#pragma unroll
+        for (int e = 0; e < 9; ++e) vals[9 * at + e] = v[e];
+    }
+
+    unsigned fl = 0;
+    int iterations = 0, it = 0, node = 0;
+    bool converged = false, have_x = true, timed_out = false;
+    bool ran = false;      // the iteration was entered: the residual norm is reported
+    bool pending = false;  // the last iteration's r.s comes with the next exchange
+    double residual = 0.0, delta = 0.0, target = 0.0, rs_next = 0.0;
+    unsigned sbad = 0, gen = 0;
+    V3<Real> hq[NH], hs[NH], nx = zero, nv = zero;
+#pragma unroll
+    for (int u = 0; u < NH; ++u) hq[u] = hs[u] = zero;
+    if (has && cidx >= 0) {
+        if (!finite3(rv)) bad |= 1u;
+        sv = apply_minv(mi, rv);
+        bool fin = finite3(sv);
+#pragma unroll
+        for (int e = 0; e < 9; ++e) fin = fin && isfinite(mi[e]);
+        if (!fin) bad |= 2u;
+        dv = sv;
+        rs_next = dot_acc<double>(rv, sv);
+    }
+    if (has) {
+        Real* d = win + 3 * tid;
+        d[0] = dv.x;
+        d[1] = dv.y;
+        d[2] = dv.z;
+    }
+
+    // The end of an iteration whose r.s is known: false ends the solve.
+    auto close = [&](double new_delta, unsigned broken, int done) -> bool {
+        if (broken) {
+            fl |= kFlagBreakdown;
+            return false;
+        }
+        const double old = delta;
+        delta = new_delta;
+        // (the last test: delta / old overflows)
+        if (!isfinite(delta) || !isfinite(old) || old <= 0.0 || (old < 1.0 && fabs(delta) > DBL_MAX * old)) {
+            fl |= kFlagBreakdown;
+            return false;
+        }
+        iterations = done;
+        return true;
+    };
+
+    // One exchange per turn, whatever it is for: the first residual, an iteration's
+    // products, a true r.s at once, the end.
+    enum Turn { kFirst, kProducts, kConfirm, kEnd };
+    Turn turn = kFirst;
+    for (;;) {
+        double v[kResSums] = {0.0, 0.0, 0.0, 0.0};
+        unsigned bits = 0;
+        if (turn == kProducts) {
+            // q = A d for the part's rows.
+            V3<Real> acc = zero;
+            auto mul_regs = [&](auto count) {
+#pragma unroll
+                for (int k = 0; k < decltype(count)::value; ++k) {
+                    const Real* d = win + rcol[k];
+                    const Real dx = d[0], dy = d[1], dz = d[2];
+                    acc.x += rval[k][0] * dx + rval[k][3] * dy + rval[k][6] * dz;
+                    acc.y += rval[k][1] * dx + rval[k][4] * dy + rval[k][7] * dz;
+                    acc.z += rval[k][2] * dx + rval[k][5] * dy + rval[k][8] * dz;
+                }
+            };
+            if (KR > 0) {  // (a slot the plan does not have is a zero block)
+                if (nslots > KR / 2)
+                    mul_regs(std::integral_constant<int, KR>{});
+                else if (nslots > KR / 4)
+                    mul_regs(std::integral_constant<int, KR / 2>{});
+                else
+                    mul_regs(std::integral_constant<int, (KR + 3) / 4>{});
+            }
+            {
+                const unsigned short* cp = cols + tid;
+                const Real* e = vals + 9 * tid;
+#pragma unroll 4
+                for (int k = KR; k < nslots; ++k, cp += T, e += 9 * T) {
+                    const Real* d = win + *cp;
+                    const Real dx = d[0], dy = d[1], dz = d[2];
+                    acc.x += e[0] * dx + e[3] * dy + e[6] * dz;
+                    acc.y += e[1] * dx + e[4] * dy + e[7] * dz;
+                    acc.z += e[2] * dx + e[5] * dy + e[8] * dz;
+                }
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1)
+                if (lpr > o) {
+                    acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+                    acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+                    acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o);
+                }
+            const int row = tid / lpr;
+            if (tid % lpr == 0 && row < m) {
+                Real* q = qbuf + 3 * row;
+                q[0] = acc.x;
+                q[1] = acc.y;
+                q[2] = acc.z;
+            }
+            __syncthreads();
+            bits = sbad;
+            // The rows other parts hold, spread over all threads (a corner row has many
+            // readers: sent by its owner alone it held the block up by 1,500 cycles).
+            auto send_row = [&](int2 s) {
+                if ((unsigned)s.x >= (unsigned)m) return;
+                const V3<Real> q{qbuf[3 * s.x], qbuf[3 * s.x + 1], qbuf[3 * s.x + 2]};
+                if (CL) {
+                    const unsigned rank = (unsigned)s.y >> 16, j = (unsigned)s.y & 0xffffu;
+                    if (rank < cl_size && j < (unsigned)P.max_halo)
+                        st_async_row(cluster_map(rows_in + ((size_t)(it & 1) * P.max_halo + j) * RB, rank), q,
+                                     cluster_map(&sh_bar[(gen + 1u) & 1u], rank));
+                } else if ((unsigned)s.y < (unsigned)P.halo_count) {
+                    st_row(P.rows_in + ((size_t)(it & 1) * P.halo_count + s.y) * RB, q, epoch + gen + 1u);
+                }
+            };
+#pragma unroll
+            for (int u = 0; u < kResSendRegs; ++u) send_row(send[u]);
+            for (int e = tid + kResSendRegs * T; e < sends_n; e += T) send_row(__ldg(P.send + send0 + e));
+            if (has) {
+                qv = V3<Real>{qbuf[3 * tid], qbuf[3 * tid + 1], qbuf[3 * tid + 2]};
+                if (!finite3(qv)) bits |= 1u;
+                const V3<Real> z = apply_minv(mi, qv);
+                v[0] = dot_acc<double>(dv, qv);
+                v[1] = dot_acc<double>(qv, sv) + dot_acc<double>(rv, z);
+                v[2] = dot_acc<double>(qv, z);
+                v[3] = rs_next;
+            }
+        } else if (turn == kEnd) {
+            // delta-v back in dynamic-row order; the solve succeeds when it is present and
+            // finite; integration is all-or-nothing.
+            if (has) v[0] = dot_acc<double>(rv, rv);
+            if (has && cidx >= 0) {
+                if (!have_x) xv = zero;
+                st3(P.x, cidx, xv);
+                if (!finite3(xv)) bits |= 1u;
+                if (P.integrate) {
+                    node = __ldg(P.dyn_to_node + cidx);
+                    const V3<Real> xo = ldplain3(P.node_x, node), vo = ldplain3(P.node_v, node);
+                    nv = vo + xv;
+                    nx = xo + nv * P.dt;
+                    if (!finite3(xo) || !finite3(vo) || !finite3(nv) || !finite3(nx)) bits |= 2u;
+                }
+            }
+        } else {
+            v[3] = rs_next;
+            bits = turn == kFirst ? bad : sbad;
+        }
+
+        // ---- the exchange: the group's sums of v and the OR of bits; with the products,
+        // also the halo rows of q (hq)
+        {
+            const bool rows = turn == kProducts;
+            ++gen;
+            // The owner warps' four sums, each in one butterfly: two steps that halve the
+            // values a lane carries, then (lane >> 3) holds its own sum.
+            if (warp < owner_warps) {
+                const bool up = (lane & 16) != 0, right = (lane & 8) != 0;
+                double k0 = up ? v[2] : v[0], k1 = up ? v[3] : v[1];
+                k0 += __shfl_xor_sync(0xffffffffu, up ? v[0] : v[2], 16);
+                k1 += __shfl_xor_sync(0xffffffffu, up ? v[1] : v[3], 16);
+                double t = right ? k1 : k0;
+                t += __shfl_xor_sync(0xffffffffu, right ? k0 : k1, 8);
+                t += __shfl_xor_sync(0xffffffffu, t, 4);
+                t += __shfl_xor_sync(0xffffffffu, t, 2);
+                t += __shfl_xor_sync(0xffffffffu, t, 1);
+                if ((lane & 7) == 0) sh_part[gen & 1u][(lane >> 3) * kResMaxWarps + warp] = t;
+            }
+            if (bits) atomicOr(&sh_bits[gen % 3u], bits);
+            if (CL && gsize > 1 && tid == 0)
+                mbar_arrive_expect_tx(&sh_bar[gen & 1u], (unsigned)gsize * kResSlotBytes +
+                                                             (rows ? (unsigned)h * row_tx_bytes<Real>() : 0u));
+            __syncthreads();
+            if (tid == 0) sh_bits[(gen + 2u) % 3u] = 0u;
+            // The block's sums: lane (k, i) takes the partials of sum k of owner warps i and
+            // i + 8, then a butterfly over i as far as there are any.  Warps that send do it
+            // each for itself; a group of one block needs nothing else.
+            const bool sends = gsize > 1 && 8 * warp < gsize;
+            if (gsize == 1 || sends) {
+                const double* q = sh_part[gen & 1u] + (lane >> 3) * kResMaxWarps + (lane & 7);
+                double t = (lane & 7) < owner_warps ? q[0] : 0.0;
+                if (owner_warps > 8) t += (lane & 7) + 8 < owner_warps ? q[8] : 0.0;
+                if (owner_warps > 4) t += __shfl_xor_sync(0xffffffffu, t, 4);
+                if (owner_warps > 2) t += __shfl_xor_sync(0xffffffffu, t, 2);
+                if (owner_warps > 1) t += __shfl_xor_sync(0xffffffffu, t, 1);
+                const unsigned w = sh_bits[gen % 3u];
+                if (gsize == 1) {
+#pragma unroll
+                    for (int k = 0; k < kResSums; ++k) v[k] = __shfl_sync(0xffffffffu, t, 8 * k);
+                    bits = w;
+                } else {
+                    // warp w's lane (k, i) sends sum k to the group's blocks 8 w + i, + 8 W, ...
+                    t = __shfl_sync(0xffffffffu, t, lane & 24);
+                    const unsigned long long lo = (unsigned long long)__double_as_longlong(t);
+                    if (CL) {
+                        const int d = 8 * warp + (lane & 7);
+                        if (d < gsize) {
+                            const unsigned rank = (unsigned)(gfirst - cl0 + d);
+                            st_async16(cluster_map(sums_in + ((gen & 1u) * kResMaxCluster + (unsigned)(blk - gfirst)) *
+                                                                 kResSlotBytes + 16 * (lane >> 3),
+                                                   rank),
+                                       {lo, (unsigned long long)w}, cluster_map(&sh_bar[gen & 1u], rank));
+                        }
+                    } else {
+                        unsigned char* out = P.sums_in + ((size_t)(gen & 1u) * gridDim.x + gfirst) * P.sums_stride +
+                                             (size_t)(blk - gfirst) * kResSlotBytes + 16 * (lane >> 3);
+                        for (int d = 8 * warp + (lane & 7); d < gsize; d += 8 * W)
+                            st_packet(out + (size_t)d * P.sums_stride,
+                                      {lo, (unsigned long long)w | ((unsigned long long)(epoch + gen) << 32)});
+                    }
+                }
+            }
+            if (CL && gsize > 1) {
+                if (!cluster_wait(&sh_bar[gen & 1u], ((gen - 1u) >> 1) & 1u)) s_fail = 1;
+                __syncthreads();
+                const unsigned char* in = sums_in + (size_t)(gen & 1u) * kResMaxCluster * kResSlotBytes +
+                                          16 * (lane >> 3);
+                double t = 0.0;
+                unsigned w = 0;
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const int i = (lane & 7) + 8 * j;
+                    if (i < gsize) {
+                        const Packet pk = *reinterpret_cast<const Packet*>(in + (size_t)i * kResSlotBytes);
+                        t += __longlong_as_double((long long)pk.lo);
+                        w |= (unsigned)pk.hi;
+                    }
+                }
+                if (gsize > 4) t += __shfl_xor_sync(0xffffffffu, t, 4);
+                if (gsize > 2) t += __shfl_xor_sync(0xffffffffu, t, 2);
+                t += __shfl_xor_sync(0xffffffffu, t, 1);
+#pragma unroll
+                for (int k = 0; k < kResSums; ++k) v[k] = __shfl_sync(0xffffffffu, t, 8 * k);
+                bits = __reduce_or_sync(0xffffffffu, w);
+                if (rows)
+#pragma unroll
+                    for (int u = 0; u < NH; ++u) {
+                        const int j = htid + u * T;
+                        if (j < h) {
+                            const Real* q =
+                                reinterpret_cast<const Real*>(rows_in + ((size_t)(it & 1) * P.max_halo + j) * RB);
+                            hq[u] = V3<Real>{q[0], q[1], q[2]};
+                        }
+                    }
+                timed_out = s_fail != 0;
+            } else if (gsize > 1) {
+                // This block's inbox: four warps each take one sum, lane i of them blocks i,
+                // i + 32, ...  With rows, the halo threads take their rows.  All reads of a
+                // poll are in flight together.
+                const int sum = W >= 8 ? warp - 4 : warp;
+                const bool polls = sum >= 0 && sum < kResSums;
+                const unsigned tag = epoch + gen;
+                const unsigned char* in = P.sums_in + ((size_t)(gen & 1u) * gridDim.x + blk) * P.sums_stride + 16 * sum;
+                const unsigned char* qin = P.rows_in + ((size_t)(it & 1) * P.halo_count + halo0) * RB;
+                Packet pk[kResSlotPoll];
+                unsigned todo = 0;
+#pragma unroll
+                for (int j = 0; j < kResSlotPoll; ++j) {
+                    pk[j] = Packet{0ull, 0ull};
+                    if (polls && lane + 32 * j < gsize) todo |= 1u << j;
+                }
+                if (rows)
+#pragma unroll
+                    for (int u = 0; u < NH; ++u)
+                        if (htid + u * T < h) todo |= 256u << u;
+                for (unsigned spins = 0; todo; ++spins) {
+#pragma unroll
+                    for (int j = 0; j < kResSlotPoll; ++j)
+                        if ((todo >> j) & 1u) pk[j] = ld_packet(in + (size_t)(lane + 32 * j) * kResSlotBytes);
+                    unsigned got = 0;
+#pragma unroll
+                    for (int u = 0; u < NH; ++u)
+                        if (((todo >> u) & 256u) && ld_row(qin + (size_t)(htid + u * T) * RB, tag, hq[u]))
+                            got |= 256u << u;
+#pragma unroll
+                    for (int j = 0; j < kResSlotPoll; ++j)
+                        if (((todo >> j) & 1u) && packet_tag(pk[j]) == tag) got |= 1u << j;
+                    todo &= ~got;
+                    if (spins > kResSpinLimit) {
+                        atomicOr(P.flags, kFlagBarrierTimeout);
+                        s_fail = 1;
+                        break;
+                    }
+                    if ((spins & 1023u) == 1023u && (*(volatile unsigned*)P.flags & kFlagBarrierTimeout)) {
+                        s_fail = 1;
+                        break;
+                    }
+                }
+                __syncwarp();
+                if (polls) {
+                    double t = 0.0;
+                    unsigned w = 0;
+#pragma unroll
+                    for (int j = 0; j < kResSlotPoll; ++j)
+                        if (lane + 32 * j < gsize) {
+                            t += __longlong_as_double((long long)pk[j].lo);
+                            w |= (unsigned)pk[j].hi;
+                        }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+                    if (lane == 0) sh_sum[gen & 1u][sum] = t;
+                    if (w) atomicOr(&sh_gbits[gen % 3u], w);
+                }
+                __syncthreads();
+#pragma unroll
+                for (int k = 0; k < kResSums; ++k) v[k] = sh_sum[gen & 1u][k];
+                bits = sh_gbits[gen % 3u];
+                if (tid == 0) sh_gbits[(gen + 2u) % 3u] = 0u;
+                timed_out = s_fail != 0;
+            }
+        }
+        if (timed_out) break;
+
+        double beta;
+        if (turn == kEnd) {
+            if (ran) residual = (isfinite(v[0]) && v[0] >= 0.0) ? sqrt(v[0]) : (double)INFINITY;
+            const bool solved = have_x && !(bits & 1u);
+            if (!have_x && !(fl & kFlagBreakdown)) fl |= kFlagInvalidRhs;
+            if (have_x && (bits & 1u)) fl |= kFlagNonFiniteDv;
+            if (solved) fl |= kFlagSolved;
+            if (solved && P.integrate) {
+                if (bits & 2u) {
+                    fl |= kFlagIntegrateAbort;
+                } else {
+                    if (has && cidx >= 0) {
+                        st3(P.node_v, node, nv);
+                        st3(P.node_x, node, nx);
+                    }
+                    fl |= kFlagIntegrated;
+                }
+            }
+            if (converged) fl |= kFlagConverged;
+            break;
+        } else if (turn == kFirst) {
+            delta = v[3];
+            turn = kEnd;
+            if (bits & 4u) {  // a malformed layout: report, do not solve
+                have_x = false;
+                fl |= kFlagBreakdown;
+            } else if ((bits & 1u) || P.max_iterations <= 0 || !isfinite(P.tolerance) || P.tolerance <= 0.0) {
+                // non-finite rhs or invalid settings: the reference clears x (the solve fails)
+                have_x = false;
+                fl |= kFlagInvalidRhs;
+            } else if (!(bits & 2u) && isfinite(delta) && delta >= 0.0) {
+                // (else the preconditioner's output is not finite: x stays 0)
+                target = P.tolerance * P.tolerance * delta;
+                if (isfinite(target)) {
+                    ran = true;
+                    if (delta <= target)
+                        converged = true;
+                    else
+                        turn = kProducts;
+                }
+            }
+            continue;  // (the exchange's barrier ordered the window's first d)
+        } else if (turn == kProducts) {
+            turn = kEnd;
+            if (pending) {
+                if (!close(v[3], bits & 2u, it)) {
+                    converged = delta <= target;
+                    continue;
+                }
+                if (delta <= target) {
+                    converged = true;
+                    continue;
+                }
+            }
+            // One reciprocal for both scalars: alpha = delta / dq (corrected to the quotient),
+            // and beta = (r'.s') / delta with r'.s' predicted, which is 1 + (alpha q.z - (q.s
+            // + r.z)) / dq.
+            const double dq = v[0], inv = 1.0 / dq;
+            double alpha = delta * inv;
+            alpha = fma(fma(-alpha, dq, delta), inv, alpha);
+            if ((bits & 1u) || !isfinite(dq) || dq <= 0.0 || !isfinite(alpha)) {
+                fl |= kFlagBreakdown;
+                converged = delta <= target;
+                continue;
+            }
+            // r'.s' before r' exists; not where it cancels, near the target or at the cap.
+            const double slope = fma(alpha, v[2], -v[1]);
+            beta = fma(slope, inv, 1.0);
+            const double next = fma(alpha, slope, delta);
+            pending = next > 0.0625 * delta && next > 1.05 * target && isfinite(next) && isfinite(beta) &&
+                      it + 1 < P.max_iterations;
+            const Scale<Real> pa(alpha), na = pa.negated();
+            sbad = 0;
+            rs_next = 0.0;
+            if (has) {
+                xv = pa.axpy(dv, xv);
+                rv = na.axpy(qv, rv);
+                sv = apply_minv(mi, rv);
+                if (!finite3(sv)) sbad = 2u;
+                rs_next = dot_acc<double>(rv, sv);
+            }
+#pragma unroll
+            for (int u = 0; u < NH; ++u) {
+                const int j = htid + u * T;
+                if (j < h) {
+                    V3<Real> r{hr[j], hr[h + j], hr[2 * h + j]};
+                    r = na.axpy(hq[u], r);
+                    hr[j] = r.x;
+                    hr[h + j] = r.y;
+                    hr[2 * h + j] = r.z;
+                    Real hmi[9];
+#pragma unroll
+                    for (int e = 0; e < 9; ++e) hmi[e] = hm[(size_t)e * h + j];
+                    hs[u] = apply_minv(hmi, r);
+                }
+            }
+            if (!pending) {
+                turn = kConfirm;
+                continue;
+            }
+        } else {
+            turn = kEnd;
+            const double old = delta;
+            if (!close(v[3], bits & 2u, it + 1) || it + 1 >= P.max_iterations || delta <= target) {
+                converged = delta <= target;
+                continue;
+            }
+            beta = delta / old;
+        }
+        // d = s + beta d: the owned row, then the halo copies.
+        const Real bt = Real(beta);
+        if (has) {
+            dv = fma3(bt, dv, sv);
+            Real* d = win + 3 * tid;
+            d[0] = dv.x;
+            d[1] = dv.y;
+            d[2] = dv.z;
+        }
+#pragma unroll
+        for (int u = 0; u < NH; ++u) {
+            const int j = htid + u * T;
+            if (j < h) {
+                Real* d = win + 3 * (m + j);
+                const V3<Real> nd = fma3(bt, V3<Real>{d[0], d[1], d[2]}, hs[u]);
+                d[0] = nd.x;
+                d[1] = nd.y;
+                d[2] = nd.z;
+            }
+        }
+        ++it;
+        turn = kProducts;
+        __syncthreads();
+    }
+
+    if (timed_out) fl |= kFlagBarrierTimeout;
+    if (leader && tid == 0) {
+        // The next solve's tags start after every tag a block of this group may have used
+        // (after a timeout a block may be an exchange ahead).
+        if (!CL && gsize > 1) P.epoch[gfirst] = epoch + gen + 16u;
+        if (P.grouped) {
+            // Per body; world-wide: the largest iteration count and residual, the OR of the
+            // failure flags and the AND of the success flags (missing: what some body lacks).
+            bs->iterations = iterations;
+            bs->converged = converged ? 1 : 0;
+            bs->residual_norm = residual;
+            bs->flags = fl;
+            atomicMax(&P.stats->iterations, iterations);
+            if (residual >= 0.0)  // non-negative doubles order like their bit patterns
+                atomicMax(reinterpret_cast<unsigned long long*>(&P.stats->residual_norm),
+                          (unsigned long long)__double_as_longlong(residual));
+            atomicOr(P.flags, fl & ~(kFlagSolved | kFlagIntegrated | kFlagConverged));
+            if (!(fl & kFlagSolved)) atomicOr(P.missing, kFlagSolved);
+            if (!(fl & kFlagIntegrated)) atomicOr(P.missing, kFlagIntegrated);
+            if (!(fl & kFlagConverged)) atomicOr(P.missing, kFlagConverged);
+        } else {
+            P.stats->iterations = iterations;
+            P.stats->converged = converged ? 1 : 0;
+            P.stats->residual_norm = residual;
+            atomicOr(P.flags, fl);
+        }
+    } else if (timed_out && tid == 0) {
+        atomicOr(P.flags, kFlagBarrierTimeout);
+    }
+    if (CL) cluster_barrier();  // nobody's shared memory goes while a peer may still write to it
+}
+
+template <class Real>
+const void* res_kernel(int threads, bool cluster)
+{
+    if (cluster)
+        return threads <= 256 ? (const void*)pcg_res_kernel<Real, 256, true>
+                              : (const void*)pcg_res_kernel<Real, 512, true>;
+    return threads <= 256 ? (const void*)pcg_res_kernel<Real, 256, false>
+                          : (const void*)pcg_res_kernel<Real, 512, false>;
+}
+
+template <class Real>
+ResLimits query_limits(int dev)
+{
+    ResLimits lim;
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return lim;
+    int per_sm = 1 << 20;
+    for (const int threads : {256, 512})
+        for (const bool cl : {false, true}) {
+            const void* k = res_kernel<Real>(threads, cl);
+            int b = 0;
+            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmemLimit) !=
+                    cudaSuccess ||
+                (cl && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, threads, kResSmemLimit) != cudaSuccess)
+                return lim;
+            per_sm = b < per_sm ? b : per_sm;
+        }
+    lim.blocks = sms * per_sm;
+    for (int q = 0; q < 5; ++q) {
+        lim.clusters[q] = 1 << 20;
+        for (const int threads : {256, 512}) {
+            cudaLaunchConfig_t c{};
+            c.gridDim = dim3(1u << q);
+            c.blockDim = dim3((unsigned)threads);
+            c.dynamicSmemBytes = kResSmemLimit;
+            cudaLaunchAttribute a;
+            a.id = cudaLaunchAttributeClusterDimension;
+            a.val.clusterDim.x = 1u << q;
+            a.val.clusterDim.y = a.val.clusterDim.z = 1;
+            c.attrs = &a;
+            c.numAttrs = 1;
+            int k = 0;
+            if (cudaOccupancyMaxActiveClusters(&k, res_kernel<Real>(threads, true), &c) != cudaSuccess) {
+                cudaGetLastError();
+                k = 0;
+            }
+            lim.clusters[q] = k < lim.clusters[q] ? k : lim.clusters[q];
+        }
+    }
+    return lim;
+}
+
+}  // namespace
+
+// A device's limits do not change: asked once per device (the queries take milliseconds),
+// which also raises the kernels' shared-memory limits on it.
+template <class Real>
+ResLimits pcg_res_limits()
+{
+    constexpr int kDevices = 64;
+    static std::once_flag asked[kDevices];
+    static ResLimits limits[kDevices];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return ResLimits{};
+    std::call_once(asked[dev], [dev] { limits[dev] = query_limits<Real>(dev); });
+    return limits[dev];
+}
+
+template <class Real>
+cudaError_t launch_pcg_res_kernel(const ResPcgArgs<Real>& args, int threads, int cluster, int grid, cudaStream_t stream)
+{
+    ResPcgArgs<Real> a = args;
+    void* kargs[] = {&a};
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3((unsigned)threads);
+    c.dynamicSmemBytes = args.smem_bytes;
+    c.stream = stream;
+    cudaLaunchAttribute at;
+    if (cluster > 0) {
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)cluster;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    } else {
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+    }
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelExC(&c, res_kernel<Real>(threads, cluster > 0), kargs);
+}
+
+template cudaError_t launch_pcg_res_kernel<float>(const ResPcgArgs<float>&, int, int, int, cudaStream_t);
+template cudaError_t launch_pcg_res_kernel<double>(const ResPcgArgs<double>&, int, int, int, cudaStream_t);
+template ResLimits pcg_res_limits<float>();
+template ResLimits pcg_res_limits<double>();
+
+}  // namespace pk

@@ -724,6 +724,9 @@ std::string build_layout_sym(int n, const int* row_start, const int* col, const 
 
 }  // namespace
 
+int plan_thread_count() { return plan_threads(); }
+void for_items(int count, const std::function<void(int, int)>& f) { parallel_items(count, f); }
+
 // The symmetric form where the caller allows it and it applies, else the full rows.
 std::string build_layout_form(int n, const int* row_start, const int* col, const int* lt_start, const int* lt_row,
                               const int* lt_block, const double* coords, const std::vector<int>& part_of,

@@ -26,6 +26,7 @@
 #pragma once
 
 #include <cstddef>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -118,6 +119,11 @@ enum SlabForm { kSlabFull = 0, kSlabSym = 1, kSlabAuto = 2 };
 std::string build_slab_plan(int n, const int* row_start, const int* col, const int* lt_start, const int* lt_row,
                             const int* lt_block, const double* coords, int parts, SlabPlan& out,
                             int form = kSlabAuto);
+
+// f(i, thread) for i in [0, count) on the layout builds' host threads (thread <
+// plan_thread_count()); each i must write only its own outputs.
+int plan_thread_count();
+void for_items(int count, const std::function<void(int, int)>& f);
 
 // The layout for per-body solves: the rows split into bodies (segments
 // [seg[b], seg[b + 1]), no block coupling two bodies), every body cut by coordinate

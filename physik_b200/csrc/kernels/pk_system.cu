@@ -251,6 +251,13 @@ struct pk_system {
     DevBuf slab_export;  // per slab row: held by another part's window
     int slab_fill_entries = 0;
     DevBuf slab_qs, slab_ss;
+    // resident PCG (pk_pcg_res.cu): the layout where the whole matrix fits on chip
+    bool res_tried = false;
+    int res_parts = 0;            // blocks of the launch (0: does not apply)
+    int res_halo_count = 0;
+    pk::ResPlan res_plan;         // its sizes; the arrays are on the device
+    pk::ResLimits res_limits;
+    DevBuf res_info, res_perm, res_halo, res_send, res_src, res_col, res_rows, res_sums, res_epoch;
     // FP64 outer true-residual refinement (FP32 storage, unbatched): passes, buffers
     int refine_passes = 0;
     DevBuf ref_x64, ref_rhs, ref_part, ref_bad;
@@ -274,6 +281,10 @@ struct pk_system {
     int graph_kernels = 0;
     // nodes; snap_x: positions at the start of the last substep (pk_system_snapshot_positions)
     DevBuf x, v, mass, node_to_dyn, snap_x;
+    // The positions first set after the nodes: what layouts are cut by, so that a layout (and
+    // the order of a solve's sums) does not depend on when it is built.
+    DevBuf layout_x;
+    bool have_layout_x = false;
     DevBuf contact_count, contact_tet, contact_point;  // pk_system_sphere_contacts
     bool have_snapshot = false;
     // tets
@@ -527,6 +538,8 @@ void reset_slab(pk_system* s)
     s->slab_filled = false;
     s->slab_parts = 0;
     s->slab_reason.clear();
+    s->res_tried = false;
+    s->res_parts = 0;
 }
 
 // Copies the assembled upper blocks (and their transposes) into the slab stream.
@@ -569,6 +582,111 @@ bool batched_solve(const pk_system* s)
     return s->batched && s->seg_start.size() >= 2 && s->conn_count == 0 && s->ext_count == 0;
 }
 
+// What a layout is cut from: the rows' node positions as first set, and the pattern.
+struct LayoutInputs {
+    std::vector<double> coords;
+    std::vector<int> col, ltr, ltb;
+};
+template <class Real>
+int layout_inputs(pk_system* s, LayoutInputs& in)
+{
+    const int n = s->dyn_count;
+    std::vector<double> nodes(3 * static_cast<size_t>(std::max(1, s->node_count)), 0.0);
+    if (s->node_count > 0) {
+        int rc = download_real<Real>(s->have_layout_x ? s->layout_x : s->x, nodes.data(), 3 * static_cast<size_t>(s->node_count), s->stream);
+        if (rc) return rc;
+    }
+    in.coords.resize(3 * static_cast<size_t>(n));
+    for (int r = 0; r < n; ++r)
+        for (int a = 0; a < 3; ++a) in.coords[3 * (size_t)r + a] = nodes[3 * (size_t)s->h_dyn_to_node[r] + a];
+    in.col.resize(static_cast<size_t>(s->nnz));
+    in.ltr.resize(static_cast<size_t>(s->lt_count));
+    in.ltb.resize(static_cast<size_t>(s->lt_count));
+    PK_CHECK(cudaMemcpy(in.col.data(), s->col.p, in.col.size() * sizeof(int), cudaMemcpyDeviceToHost));
+    if (s->lt_count > 0) {
+        PK_CHECK(cudaMemcpy(in.ltr.data(), s->lt_row.p, in.ltr.size() * sizeof(int), cudaMemcpyDeviceToHost));
+        PK_CHECK(cudaMemcpy(in.ltb.data(), s->lt_block.p, in.ltb.size() * sizeof(int), cudaMemcpyDeviceToHost));
+    }
+    return PK_OK;
+}
+
+// PK_PCG_RESIDENT=0 keeps every solve on the streaming kernels, for comparisons.
+bool resident_allowed(const pk_system* s)
+{
+    const char* e = std::getenv("PK_PCG_RESIDENT");
+    if (e && e[0] == '0') return false;
+    const int rk = requested_kernel();
+    if (s->dyn_count <= 0 || !s->have_pattern) return false;
+    return s->precision == PK_PREC_FP64 ? rk == -1 : (rk == -1 || rk == 3) && requested_slab_form() == pk::kSlabFull;
+}
+
+// Builds and uploads the resident kernel's layout (one group per body when `bodies`) if it
+// has not been tried yet; where it does not apply res_parts stays 0.  Synchronous.
+template <class Real>
+int ensure_resident(pk_system* s, bool bodies)
+{
+    if (s->res_tried || !resident_allowed(s)) return PK_OK;
+    s->res_tried = true;
+    s->res_parts = 0;
+    if (s->res_limits.blocks == 0) s->res_limits = pk::pcg_res_limits<Real>();
+    pk::ResLimits limits = s->res_limits;
+    if (s->pcg_grid_override > 0) {
+        limits.blocks = std::min(limits.blocks, s->pcg_grid_override);
+        for (int q = 0; q < 5; ++q) limits.clusters[q] = std::min(limits.clusters[q], s->pcg_grid_override >> q);
+    }
+    const int grid = limits.blocks;
+    const int n = s->dyn_count;
+    // Blocks of a row before padding: a matrix that cannot fit is refused without a layout.
+    const size_t entries = 2 * static_cast<size_t>(s->nnz);
+    if (grid <= 0 || entries > static_cast<size_t>(n) &&
+                         (entries - n) * (9 * sizeof(Real) + 2) > static_cast<size_t>(grid) * 2 * pk::kResSmemLimit)
+        return PK_OK;
+    LayoutInputs in;
+    int rc = layout_inputs<Real>(s, in);
+    if (rc) return rc;
+    const int whole[2] = {0, n};
+    pk::ResPlan plan;
+    const std::string why = pk::build_res_plan(
+        n, s->h_row_start.data(), in.col.data(), s->h_lts.data(), in.ltr.data(), in.ltb.data(), in.coords.data(),
+        bodies ? s->seg_start.data() : whole, bodies ? static_cast<int>(s->seg_start.size()) - 1 : 1, limits,
+        static_cast<int>(sizeof(Real)), plan);
+    if (!why.empty()) return PK_OK;
+    rc = upload_raw<int>(s->res_info, plan.part_info.data(), plan.part_info.size(), s->stream);
+    if (!rc) rc = upload_raw<int>(s->res_perm, plan.perm.data(), plan.perm.size(), s->stream);
+    if (!rc) rc = upload_raw<int>(s->res_halo, plan.halo_src.data(), plan.halo_src.size(), s->stream);
+    if (!rc) rc = upload_raw<int>(s->res_send, plan.send.data(), plan.send.size(), s->stream);
+    if (!rc) rc = upload_raw<unsigned>(s->res_src, plan.src.data(), plan.src.size(), s->stream);
+    if (!rc) rc = upload_raw<unsigned short>(s->res_col, plan.col.data(), plan.col.size(), s->stream);
+    if (rc) return rc;
+    if (plan.cluster == 0) {
+        const size_t rows = 2 * plan.halo_src.size() * pk::res_row_packet(sizeof(Real));
+        const size_t sums = 2 * static_cast<size_t>(plan.parts) * plan.max_group * pk::kResSlotBytes;
+        PK_CHECK(s->res_rows.ensure(rows));
+        PK_CHECK(s->res_sums.ensure(sums));
+        PK_CHECK(s->res_epoch.ensure(sizeof(unsigned) * static_cast<size_t>(plan.parts)));
+        PK_CHECK(cudaMemsetAsync(s->res_rows.p, 0, rows, s->stream));  // no packet carries a tag yet
+        PK_CHECK(cudaMemsetAsync(s->res_sums.p, 0, sums, s->stream));
+        PK_CHECK(cudaMemsetAsync(s->res_epoch.p, 0, sizeof(unsigned) * static_cast<size_t>(plan.parts), s->stream));
+    }
+    if (bodies) {  // a body without rows keeps zero statistics
+        const size_t bytes = sizeof(pk::BatchBodyStats) * s->seg_start.size();
+        PK_CHECK(s->body_stats.ensure(bytes));
+        PK_CHECK(cudaMemsetAsync(s->body_stats.p, 0, bytes, s->stream));
+    }
+    PK_CHECK(cudaStreamSynchronize(s->stream));
+    s->res_halo_count = static_cast<int>(plan.halo_src.size());
+    s->res_parts = plan.parts;
+    s->res_plan = pk::ResPlan{};
+    s->res_plan.lpr = plan.lpr;
+    s->res_plan.threads = plan.threads;
+    s->res_plan.slots = plan.slots;
+    s->res_plan.cluster = plan.cluster;
+    s->res_plan.max_group = plan.max_group;
+    s->res_plan.max_halo = plan.max_halo;
+    s->res_plan.smem_bytes = plan.smem_bytes;
+    return PK_OK;
+}
+
 // Builds and uploads the part-resident kernel's layout if it has not been tried yet for
 // this pattern and grid (synchronous: never called while a stream capture is open).
 // Parts are cut by the rows' node positions at this moment.  Not applicable (too large
@@ -582,6 +700,11 @@ int ensure_slab(pk_system* s)
     s->slab_tried = true;
     s->slab_for_bodies = bodies;
     s->slab_parts = 0;
+    if (const int rc = ensure_resident<float>(s, bodies)) return rc;
+    if (s->res_parts > 0) {  // the matrix stays on chip: no stream
+        s->slab_sym = false;
+        return PK_OK;
+    }
     if (!s->slab_max_grid) s->slab_max_grid = pk::pcg_slab_max_grid<Acc>();
     int grid = s->slab_max_grid;
     if (s->pcg_grid_override > 0) grid = std::min(grid, s->pcg_grid_override);
@@ -591,22 +714,10 @@ int ensure_slab(pk_system* s)
         return PK_OK;
     }
     const int n = s->dyn_count;
-    // node positions -> per-row coordinates
-    std::vector<double> nodes(3 * static_cast<size_t>(std::max(1, s->node_count)), 0.0);
-    if (s->node_count > 0) {
-        int rc = download_real<float>(s->x, nodes.data(), 3 * static_cast<size_t>(s->node_count), s->stream);
-        if (rc) return rc;
-    }
-    std::vector<double> coords(3 * static_cast<size_t>(n));
-    for (int r = 0; r < n; ++r)
-        for (int a = 0; a < 3; ++a) coords[3 * (size_t)r + a] = nodes[3 * (size_t)s->h_dyn_to_node[r] + a];
-    std::vector<int> col(static_cast<size_t>(s->nnz)), ltr(static_cast<size_t>(s->lt_count)),
-        ltb(static_cast<size_t>(s->lt_count));
-    PK_CHECK(cudaMemcpy(col.data(), s->col.p, col.size() * sizeof(int), cudaMemcpyDeviceToHost));
-    if (s->lt_count > 0) {
-        PK_CHECK(cudaMemcpy(ltr.data(), s->lt_row.p, ltr.size() * sizeof(int), cudaMemcpyDeviceToHost));
-        PK_CHECK(cudaMemcpy(ltb.data(), s->lt_block.p, ltb.size() * sizeof(int), cudaMemcpyDeviceToHost));
-    }
+    LayoutInputs in;
+    if (const int rc = layout_inputs<float>(s, in)) return rc;
+    const std::vector<double>& coords = in.coords;
+    const std::vector<int>&col = in.col, &ltr = in.ltr, &ltb = in.ltb;
     pk::SlabPlan plan;
     const std::string why =
         bodies ? pk::build_slab_plan_batched(n, s->h_row_start.data(), col.data(), s->h_lts.data(), ltr.data(),
@@ -716,7 +827,7 @@ int ensure_slab_any(pk_system* s)
 {
     if (s->precision == PK_PREC_FP32) return ensure_slab<float>(s);
     if (s->precision == PK_PREC_MIXED) return ensure_slab<double>(s);
-    return PK_OK;
+    return batched_solve(s) ? PK_OK : ensure_resident<double>(s, false);
 }
 
 // The per-body round table for the next solve (slab_schedule_kernel) on `stream`.
@@ -823,6 +934,56 @@ int run_pcg_slab(pk_system* s, const pk_step_params& p, int skip_on_flags)
         s->last_blocks = s->slab_parts;
         return PK_OK;
     }
+}
+
+template <class Real>
+int run_pcg_resident(pk_system* s, const pk_step_params& p, int skip_on_flags)
+{
+    int rc = ensure_solver_buffers(s, 1);
+    if (rc) return rc;
+    const bool bodies = batched_solve(s);
+    pk::DevStats* st = s->stats.as<pk::DevStats>();
+    pk::ResPcgArgs<Real> a{};
+    a.n = s->dyn_count;
+    a.part_info = s->res_info.as<int>();
+    a.perm = s->res_perm.as<int>();
+    a.halo_src = s->res_halo.as<int>();
+    a.halo_count = s->res_halo_count;
+    a.send = s->res_send.as<int2>();
+    a.src = s->res_src.as<unsigned>();
+    a.col = s->res_col.as<unsigned short>();
+    a.lpr = s->res_plan.lpr;
+    a.nslots = s->res_plan.slots;
+    a.max_halo = s->res_plan.max_halo;
+    a.slot_count = s->res_plan.slots * s->res_parts;
+    a.nnz = s->nnz;
+    a.smem_bytes = static_cast<unsigned>(s->res_plan.smem_bytes);
+    a.values = s->values.as<Real>();
+    a.b = s->rhs.as<Real>();
+    a.minv = s->minv.as<Real>();
+    a.x = s->px.as<Real>();
+    a.rows_in = s->res_rows.as<unsigned char>();
+    a.sums_in = s->res_sums.as<unsigned char>();
+    a.sums_stride = static_cast<size_t>(s->res_plan.max_group) * pk::kResSlotBytes;
+    a.epoch = s->res_epoch.as<unsigned>();
+    a.max_iterations = p.max_iterations;
+    a.tolerance = static_cast<double>(static_cast<Real>(p.tolerance));
+    a.skip_on_flags = skip_on_flags;
+    a.integrate = p.integrate;
+    a.dt = static_cast<Real>(p.dt);
+    a.dyn_to_node = s->dyn_to_node.as<int>();
+    a.node_x = s->x.as<Real>();
+    a.node_v = s->v.as<Real>();
+    a.flags = &st->flags;
+    a.stats = st;
+    a.grouped = bodies ? 1 : 0;
+    a.nbodies = bodies ? static_cast<int>(s->seg_start.size()) - 1 : 1;
+    a.body_stats = bodies ? s->body_stats.as<pk::BatchBodyStats>() : nullptr;
+    a.missing = &st->batch_missing;
+    PK_CHECK(pk::launch_pcg_res_kernel<Real>(a, s->res_plan.threads, s->res_plan.cluster, s->res_parts, s->stream));
+    s->launches += 1;
+    s->last_blocks = s->res_parts;
+    return PK_OK;
 }
 
 // Cuts every body (segment) into parts of about equal row count, one block each, so that
@@ -937,12 +1098,19 @@ int run_pcg_batch(pk_system* s, const pk_step_params& p, int skip_on_flags)
     return PK_OK;
 }
 
-// The PCG kernel the next unbatched solve uses (0 ring, 1 staged, 2 plain, 3 slab).
+// The part-resident kernel family has a layout: resident rows, or the stream.
+bool slab_ready(const pk_system* s)
+{
+    return s->slab_parts > 0 || (s->precision != PK_PREC_FP64 && s->res_parts > 0);
+}
+
+// The PCG kernel the next unbatched solve uses (0 ring, 1 staged, 2 plain, 3 slab).  Where
+// the resident layout applies it takes the place of 3, and of 0 for FP64 storage.
 int solve_kernel(const pk_system* s)
 {
-    if (s->kernel_choice == 3 && s->slab_parts <= 0) return s->ring_tiles > 0 ? 0 : (s->ntiles > 0 ? 1 : 2);
+    if (s->kernel_choice == 3 && !slab_ready(s)) return s->ring_tiles > 0 ? 0 : (s->ntiles > 0 ? 1 : 2);
     if (s->kernel_choice >= 0) return s->kernel_choice;
-    return s->slab_parts > 0 ? 3 : (s->ring_tiles > 0 ? 0 : (s->ntiles > 0 ? 1 : 2));
+    return slab_ready(s) ? 3 : (s->ring_tiles > 0 ? 0 : (s->ntiles > 0 ? 1 : 2));
 }
 
 template <class Real, class Acc>
@@ -955,6 +1123,10 @@ int run_pcg(pk_system* s, const pk_step_params& p, int skip_on_flags)
             if (s->batch_slab) {
                 int rc = ensure_slab<Acc>(s);
                 if (rc) return rc;
+                if (s->res_parts > 0 && s->slab_for_bodies) {
+                    s->last_kernel = 5;
+                    return run_pcg_resident<Real>(s, p, skip_on_flags);
+                }
                 if (s->slab_parts > 0 && s->slab_for_bodies) return run_pcg_slab<Real, Acc>(s, p, skip_on_flags);
             }
         }
@@ -964,9 +1136,14 @@ int run_pcg(pk_system* s, const pk_step_params& p, int skip_on_flags)
     if constexpr (std::is_same<Real, float>::value) {
         int rc = ensure_slab<Acc>(s);
         if (rc) return rc;
+    } else {
+        int rc = ensure_resident<double>(s, false);
+        if (rc) return rc;
     }
     const int kernel = solve_kernel(s);
     s->last_kernel = kernel;
+    if (s->res_parts > 0 && kernel == (std::is_same<Real, float>::value ? 3 : 0))
+        return run_pcg_resident<Real>(s, p, skip_on_flags);
     if (kernel == 3) return run_pcg_slab<Real, Acc>(s, p, skip_on_flags);
     if (kernel == 0 && s->ring_tiles > 0) {
         int rc = ensure_solver_buffers(s, 1);
@@ -1233,8 +1410,8 @@ int run_step(pk_system* s, const pk_step_params& p)
             if (!p.explicit_mode && (!batched_solve(s) || s->batch_slab)) {
                 int rc = s->precision == PK_PREC_MIXED ? ensure_slab<double>(s) : ensure_slab<float>(s);
                 if (rc) return rc;
-                const bool uses = batched_solve(s) ? (s->slab_parts > 0 && s->slab_for_bodies) : solve_kernel(s) == 3;
-                if (uses) {
+                const bool uses = batched_solve(s) ? s->slab_for_bodies : solve_kernel(s) == 3;
+                if (uses && s->slab_parts > 0) {
                     rc = slab_fill(s);
                     if (rc) return rc;
                 }
@@ -1453,6 +1630,7 @@ PKCUDA_API int pk_system_set_nodes(pk_system* s, int node_count, const int* node
     if (!s || node_count < 0 || (node_count > 0 && (!node_to_dyn || !mass))) return fail(PK_ERR_ARG, "set_nodes");
     PK_CHECK(cudaSetDevice(s->device));
     s->node_count = node_count;
+    s->have_layout_x = false;
     s->have_snapshot = false;
     s->h_node_to_dyn.assign(node_to_dyn, node_to_dyn + node_count);
     s->slots_ok = false;
@@ -1471,6 +1649,16 @@ PKCUDA_API int pk_system_set_nodes(pk_system* s, int node_count, const int* node
     return PK_OK;
 }
 
+static int keep_layout_positions(pk_system* s)
+{
+    if (s->have_layout_x) return PK_OK;
+    const size_t bytes = 3 * s->rsize() * static_cast<size_t>(s->node_count);
+    PK_CHECK(s->layout_x.ensure(bytes));
+    if (bytes) PK_CHECK(cudaMemcpyAsync(s->layout_x.p, s->x.p, bytes, cudaMemcpyDeviceToDevice, s->stream));
+    s->have_layout_x = true;
+    return PK_OK;
+}
+
 PKCUDA_API int pk_system_set_state_f64(pk_system* s, const double* x, const double* v)
 {
     if (!s || !s->have_nodes) return fail(PK_ERR_STATE, "set_state before set_nodes");
@@ -1479,7 +1667,7 @@ PKCUDA_API int pk_system_set_state_f64(pk_system* s, const double* x, const doub
     int rc = PK_OK;
     if (x) rc = upload_real_any(s, s->x, x, n);
     if (!rc && v) rc = upload_real_any(s, s->v, v, n);
-    return rc;
+    return !rc && x ? keep_layout_positions(s) : rc;
 }
 
 PKCUDA_API int pk_system_set_state_f32(pk_system* s, const float* x, const float* v)
@@ -1496,7 +1684,7 @@ PKCUDA_API int pk_system_set_state_f32(pk_system* s, const float* x, const float
     // float storage: copy straight from the caller's buffer (pinned buffers stay asynchronous)
     if (x) PK_CHECK(cudaMemcpyAsync(s->x.p, x, n * sizeof(float), cudaMemcpyHostToDevice, s->stream));
     if (v) PK_CHECK(cudaMemcpyAsync(s->v.p, v, n * sizeof(float), cudaMemcpyHostToDevice, s->stream));
-    return PK_OK;
+    return x ? keep_layout_positions(s) : PK_OK;
 }
 
 PKCUDA_API int pk_system_get_state_f64(pk_system* s, double* x, double* v)
@@ -2250,7 +2438,7 @@ PKCUDA_API int pk_system_autotune(pk_system* s, const pk_step_params* p, int rep
             s->batch_slab = true;
             int rc = ensure_slab_any(s);
             if (rc) return rc;
-            if (s->slab_parts > 0 && s->slab_for_bodies) {
+            if (slab_ready(s) && s->slab_for_bodies) {
                 slab_t = time_solves(s, *p, repeats);
                 if (slab_t < 0) return static_cast<int>(slab_t);
             }
@@ -2294,7 +2482,7 @@ PKCUDA_API int pk_system_autotune(pk_system* s, const pk_step_params* p, int rep
         int i = 0;
         for (const Cand& c : cand) {
             if (c.kernel == 0 && s->ring_tiles <= 0) { ++i; continue; }
-            if (c.kernel == 3 && s->slab_parts <= 0) { ++i; continue; }
+            if (c.kernel == 3 && !slab_ready(s)) { ++i; continue; }
             if (c.kernel == 1) {
                 int rc = retile(c.rows);
                 if (rc) return rc;
@@ -2633,6 +2821,41 @@ PKCUDA_API int pk_slab_plan_batched_selfcheck(int n, const int* row_start, const
         info[3] = static_cast<int>(plan.stream.size() / 1024);
         info[4] = launches;
         info[5] = plan.sym ? 1 : 0;
+    }
+    return PK_OK;
+}
+
+PKCUDA_API int pk_res_plan_selfcheck(int n, const int* row_start, const int* col_index, const double* values,
+                                     const double* x, const double* coords, const int* segment_row_start,
+                                     int segment_count, int max_blocks, int precision, double* y, int* info)
+{
+    if (n <= 0 || segment_count <= 0 || max_blocks == 0 || !row_start || !col_index || !values || !x || !y ||
+        !coords || !segment_row_start)
+        return fail(PK_ERR_ARG, "resident selfcheck");
+    for (int r = 0; r < n; ++r)
+        for (int k = row_start[r]; k < row_start[r + 1]; ++k)
+            if (col_index[k] < r || col_index[k] >= n) return fail(PK_ERR_ARG, "column outside [row, n)");
+    std::vector<int> lts, ltr, ltb;
+    build_transpose(n, row_start, col_index, lts, ltr, ltb);
+    const int real = precision == PK_PREC_FP64 ? 8 : 4;
+    // max_blocks > 0: that many blocks, and the clusters that fit them; < 0: no clusters
+    pk::ResLimits limits;
+    limits.blocks = std::abs(max_blocks);
+    for (int q = 0; q < 5 && max_blocks > 0; ++q) limits.clusters[q] = max_blocks >> q;
+    pk::ResPlan plan;
+    std::string why = pk::build_res_plan(n, row_start, col_index, lts.data(), ltr.data(), ltb.data(), coords,
+                                         segment_row_start, segment_count, limits, real, plan);
+    if (!why.empty()) return fail(PK_ERR_UNSUPPORTED, "resident layout: " + why);
+    why = pk::res_check(plan, row_start[n], limits, real);
+    if (!why.empty()) return fail(PK_ERR_STATE, "resident layout: " + why);
+    pk::res_spmv_host(plan, values, x, y);
+    if (info) {
+        info[0] = plan.parts;
+        info[1] = plan.max_rows;
+        info[2] = plan.lpr;
+        info[3] = static_cast<int>(plan.smem_bytes);
+        info[4] = plan.cluster;
+        info[5] = plan.threads;
     }
     return PK_OK;
 }
