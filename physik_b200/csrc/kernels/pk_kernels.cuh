@@ -66,18 +66,25 @@ struct TetView {
     const unsigned char* enabled;    // bit 0: active, rest volume > 0, body simulated; bit 1: linear FEM
     const Real* dm_inv;              // 9 per tet, column-major
     const Real* params;              // 4 per tet: rest volume, lambda, mu, damping
-    // kTetRec per tet, read by the row kernel (one aligned record per tet): R (9), a 3x3
-    // matrix M (9) and a form value (index 31), written by the tet kernel each step
-    // (rec[kTetRec t] = NaN when the tet is skipped this step); DmInv (9), rest volume,
-    // lambda, mu, damping (18..30), written once when the tets are set (launch_tet_pack).
-    // Form 0: M = S = R * V * sigma, node a's elastic force is -S g_a.  Form 1 (the
-    // implicit step with a slot table): M = T = -(dt S + dt^2 Q), where Q g_a is the tet's
-    // sum_b K_ab v_b, so the tet adds T g_a - dt c v_a to row a's right-hand side.
+    // tet_rec() values per tet, written by the tet kernel each step and read by the row
+    // kernels (one aligned record per tet): four corners of four values P_k = R g_k and V
+    // lambda, then four of B_k and V mu, with B_k = T g_k - dt c v_k the tet's right-hand side
+    // at corner k (T = -(dt S + dt^2 Q), S = R V sigma, Q g_a the tet's sum_b K_ab v_b); in
+    // FP64 then g_a.g_b (10) and R R^T (6).  A tet that is not folded so has NaN in place of
+    // P_k's V lambda, and its form in place of B_0's V mu: kFormForces, B_k = -S g_k (V lambda
+    // and V mu in B_1 and B_3); kFormPlain (FP32, a rotation whose iteration ran out), R in
+    // the first three corners and S in the next three; kFormSkip, no part in this step.
+    // Explicit step: kTetForces values per tet, four corners of the force -S g_k and the damping.
     Real* rec;
+    const Real* rest;                // 12 per tet: DmInv, rest volume, lambda, mu (launch_tet_pack)
 };
-constexpr int kTetRec = 32;
-constexpr unsigned kSlotNone = 255u, kSlotMissing = 254u;
-constexpr int kSlotMaxRow = 16;  // the row kernel's register-slot paths (MAXU 8 and 16)
+template <class Real>
+constexpr int tet_rec()
+{
+    return sizeof(Real) == 4 ? 32 : 48;
+}
+constexpr int kTetForces = 16;
+constexpr int kFormForces = 1, kFormPlain = 2, kFormSkip = 3;
 
 template <class Real>
 struct AssemblyArgs {
@@ -92,12 +99,12 @@ struct AssemblyArgs {
     Real* x_out;                     // explicit mode position update target
     const int* inc_start;            // per dyn row
     const int* inc_list;             // t*4 + a
-    // Per incidence, the row slots of the tet's 4 nodes (8 bits each, node b in bits
-    // 8b..8b+7): the block's index in the row's upper blocks, kSlotNone when the column is
-    // not in the upper row (a lower or non-dynamic node), kSlotMissing when the pattern
-    // lacks it.  NULL: no table (rows longer than kSlotMaxRow, or not built).
-    const unsigned* inc_slot;
-    int row_lanes;                   // with a slot table: four lanes per row (1) or one thread (0)
+    // The blocks' tets (block_list_kernel); NULL: one thread per row over its incidences.
+    int nnz;
+    const int2* blk_range;           // per stored block
+    const unsigned* blk_list;
+    const int* blk_missing;          // rows whose tets couple a block the pattern lacks
+    int fold;                        // fold the tets' K v into their right-hand sides
     Real* values;                    // out: A blocks
     Real* rhs;                       // out: b
     Real* minv;                      // out: block-Jacobi inverse
@@ -549,9 +556,9 @@ struct AdjointArgs {
 // Launchers (pk_kernels.cu).  All asynchronous on `stream`.
 template <class Real>
 cudaError_t launch_tet_kernel(const AssemblyArgs<Real>& args, bool fp64_polar_fallback, cudaStream_t stream);
-// The static part of the tet records (DmInv and the material of every tet).
+// TetView::rest, when the tets are set.
 template <class Real>
-cudaError_t launch_tet_pack(const Real* dm_inv, const Real* params, Real* rec, int tet_count, cudaStream_t stream);
+cudaError_t launch_tet_pack(const Real* dm_inv, const Real* params, Real* rest, int tet_count, cudaStream_t stream);
 template <class Real>
 cudaError_t launch_visual_kernel(int kind, const int* nodes, const float* weights, const unsigned char* live, int count,
                                  const Real* x, float* verts, float* normals, cudaStream_t stream);
@@ -565,10 +572,11 @@ template <class Real>
 cudaError_t launch_conn_kernel(const AssemblyArgs<Real>& args, cudaStream_t stream);
 template <class Real>
 cudaError_t launch_row_kernel(const AssemblyArgs<Real>& args, int max_row_blocks, cudaStream_t stream);
-// Builds AssemblyArgs::inc_slot for the pattern, the incidences and the tets' nodes.
-cudaError_t launch_inc_slot_kernel(int n, const int* row_start, const int* col, const int* inc_start,
-                                   const int* inc_list, const int4* tet_nodes, const int* node_to_dyn, unsigned* out,
-                                   cudaStream_t stream);
+// Builds AssemblyArgs::blk_range and blk_list (4 entries per incidence) for the pattern, the
+// incidences and the tets' nodes; counts into *missing (zeroed).
+cudaError_t launch_block_list_kernel(int n, const int* row_start, const int* col, const int* inc_start,
+                                     const int* inc_list, const int4* tet_nodes, const int* node_to_dyn, int2* range,
+                                     unsigned* list, int* missing, cudaStream_t stream);
 template <class Real, class Acc>
 cudaError_t launch_pcg_kernel(const PcgArgs<Real, Acc>& args, int grid, int threads, cudaStream_t stream);
 // Largest cooperative grid (one wave) for the staged (args.ntiles > 0) or unstaged kernel.

@@ -126,12 +126,13 @@ __host__ __device__ __forceinline__ bool finite9(const M3<T>& m)
 }
 // Adjugate inverse; identity when |det| <= 1e-6.
 template <class T>
-__host__ __device__ __forceinline__ M3<T> inverse(const M3<T>& m)
+__host__ __device__ __forceinline__ M3<T> inverse(const M3<T>& m, T* determinant = nullptr)
 {
     const V3<T> r0 = cross(m.c[1], m.c[2]);
     const V3<T> r1 = cross(m.c[2], m.c[0]);
     const V3<T> r2 = cross(m.c[0], m.c[1]);
     const T d = dot(m.c[0], r0);
+    if (determinant) *determinant = d;
     if (fabs(d) <= T(0.000001)) return mident<T>();
     const T inv = T(1) / d;
     return transpose(mcols(r0 * inv, r1 * inv, r2 * inv));
@@ -151,13 +152,16 @@ __host__ __device__ __forceinline__ V3<T> cast(const V3<U>& a)
 // Polar rotation of F by Newton averaging R <- (R + R^-T)/2: at most 12 iterations,
 // stop when ||R_next - R||_F^2 <= 1e-10, identity when F or an iterate is singular
 // (|det| <= 1e-8) or non-finite, and negate column 2 if det(R) < 0.
-// Returns the iteration count through *iterations; *fallback is set on the identity exits.
+// Returns the iteration count through *iterations; *fallback is set on the identity exits;
+// *converged (may be NULL) is cleared when the iterations ran out before the stopping test.
 template <class T>
-__host__ __device__ inline M3<T> polar_rotation(const M3<T>& f, int* iterations, bool* fallback)
+__host__ __device__ inline M3<T> polar_rotation(const M3<T>& f, int* iterations, bool* fallback,
+                                                bool* converged = nullptr)
 {
     const T min_det = T(1.0e-8);
     *iterations = 0;
     *fallback = false;
+    bool done = false;
     if (!finite9(f) || fabs(det(f)) <= min_det) {
         *fallback = true;
         return mident<T>();
@@ -165,24 +169,30 @@ __host__ __device__ inline M3<T> polar_rotation(const M3<T>& f, int* iterations,
     M3<T> r = f;
     for (int it = 0; it < 12; ++it) {
         *iterations = it + 1;
-        const M3<T> ti = inverse(transpose(r));
-        if (!finite9(ti) || fabs(det(ti)) <= min_det) {
-            *fallback = true;
-            return mident<T>();
-        }
+        T dr;
+        const M3<T> ti = inverse(transpose(r), &dr);
         const M3<T> next = scale(add(r, ti), T(0.5));
-        if (!finite9(next)) {
-            *fallback = true;
-            return mident<T>();
-        }
         T diff = T(0);
         for (int col = 0; col < 3; ++col) {
             const V3<T> d = next.c[col] - r.c[col];
             diff += dot(d, d);
         }
+        // The identity exits, off the common path: with 1e-6 < |det r| < 1e6 the inverse's
+        // determinant, 1 / det r to rounding, is far above the limit; and r is finite, so a
+        // non-finite inverse or iterate shows in diff.
+        if (!(fabs(dr) > T(1.0e-6) && fabs(dr) < T(1.0e6)) || !isfinite(diff)) {
+            if (!finite9(ti) || fabs(det(ti)) <= min_det || !finite9(next)) {
+                *fallback = true;
+                return mident<T>();
+            }
+        }
         r = next;
-        if (diff <= T(1.0e-10)) break;
+        if (diff <= T(1.0e-10)) {
+            done = true;
+            break;
+        }
     }
+    if (converged) *converged = done;
     if (!finite9(r)) {
         *fallback = true;
         return mident<T>();

@@ -288,15 +288,15 @@ struct pk_system {
     DevBuf contact_count, contact_tet, contact_point;  // pk_system_sphere_contacts
     bool have_snapshot = false;
     // tets
-    DevBuf tet_nodes, tet_enabled, dm_inv, tet_params, tet_rec;
+    DevBuf tet_nodes, tet_enabled, dm_inv, tet_params, tet_rec, tet_rest;
     // rows
     DevBuf dyn_to_node, row_start, col, lt_start, lt_row, lt_block, inc_start, inc_list, values, rhs, minv;
-    DevBuf inc_slot;        // per incidence: the row slots of the tet's nodes (built on first use)
+    DevBuf blk_range, blk_list, blk_missing;  // the blocks' tets (built on first use)
     // FP64 rest data and masses of an FP32-stored system, for the refinement's element-
     // wise FP64 residual (FP64 systems use their own arrays), and its scratch.
     DevBuf dm_inv64, params64, mass64, elem_u, elem_vx;
     bool rest64_ok = false;  // pk_system_set_rest64 matches the current tets and nodes
-    bool slots_ok = false;  // inc_slot matches the pattern, incidences, tets and node rows
+    bool lists_ok = false;  // the blocks' tets match the pattern, incidences, tets and node rows
     // solver
     DevBuf px, pr, psd0, psd1, pq, part_a, part_b, part_bad, sync, stats;
     pk::DevStats* host_stats = nullptr;  // pinned
@@ -314,7 +314,8 @@ struct pk_system {
 
 namespace {
 
-bool row_lanes_enabled();
+bool block_rows_enabled();
+bool assembly_fold_enabled();
 
 template <class Real>
 pk::AssemblyArgs<Real> assembly_args(pk_system* s, const pk_step_params& p)
@@ -326,6 +327,7 @@ pk::AssemblyArgs<Real> assembly_args(pk_system* s, const pk_step_params& p)
     a.tets.dm_inv = s->dm_inv.as<Real>();
     a.tets.params = s->tet_params.as<Real>();
     a.tets.rec = s->tet_rec.as<Real>();
+    a.tets.rest = s->tet_rest.as<Real>();
     a.a.n = s->dyn_count;
     a.a.row_start = s->row_start.as<int>();
     a.a.col = s->col.as<int>();
@@ -342,8 +344,13 @@ pk::AssemblyArgs<Real> assembly_args(pk_system* s, const pk_step_params& p)
     a.x_out = s->x.as<Real>();
     a.inc_start = s->inc_start.as<int>();
     a.inc_list = s->inc_list.as<int>();
-    a.inc_slot = s->slots_ok ? s->inc_slot.as<unsigned>() : nullptr;
-    a.row_lanes = row_lanes_enabled() ? 1 : 0;
+    a.nnz = s->nnz;
+    a.fold = assembly_fold_enabled() ? 1 : 0;
+    if (s->lists_ok && block_rows_enabled()) {
+        a.blk_range = s->blk_range.as<int2>();
+        a.blk_list = s->blk_list.as<unsigned>();
+        a.blk_missing = s->blk_missing.as<int>();
+    }
     a.values = s->values.as<Real>();
     a.rhs = s->rhs.as<Real>();
     a.minv = s->minv.as<Real>();
@@ -1332,42 +1339,46 @@ int run_pcg_refined(pk_system* s, const pk_step_params& p, int skip_on_flags)
     return PK_OK;
 }
 
-// PK_ROW_KERNEL=thread assembles the rows one thread each (the four-lane kernel's blocks
-// and right-hand side are the same bits; kept for comparisons).
-bool row_lanes_enabled()
+// PK_ROW_KERNEL=thread assembles the rows one thread each (the same bits as the kernel over
+// block lists, for rows of up to 16 blocks; kept for comparisons).
+bool block_rows_enabled()
 {
     const char* e = std::getenv("PK_ROW_KERNEL");
     return !(e && std::strcmp(e, "thread") == 0);
 }
 
-// PK_ASSEMBLY_FOLD=0 keeps every tet on the long assembly path (all 16 blocks per tet
-// and K v in the row kernel), for comparisons; the default folds K v into the tet kernel.
+// PK_ASSEMBLY_FOLD=0 keeps every tet on the long assembly path (K v in the row kernel), for
+// comparisons; the default folds K v into the tet kernel.
 bool assembly_fold_enabled()
 {
     const char* e = std::getenv("PK_ASSEMBLY_FOLD");
     return !(e && e[0] == '0');
 }
 
-// The slot table of the folded assembly (rows of at most kSlotMaxRow upper blocks), built
-// on the device after the pattern, the incidences, the tets or the node rows changed.
-int ensure_inc_slots(pk_system* s)
+// The blocks' tets, built on the device after the pattern, the incidences, the tets or the
+// node rows changed.
+int ensure_block_lists(pk_system* s)
 {
-    if (s->slots_ok || s->dyn_count <= 0 || s->inc_count <= 0 || !s->have_tets || s->max_row > pk::kSlotMaxRow ||
-        !assembly_fold_enabled())
+    if (s->lists_ok || s->dyn_count <= 0 || s->inc_count <= 0 || !s->have_tets || !block_rows_enabled())
         return PK_OK;
-    PK_CHECK(s->inc_slot.ensure(sizeof(unsigned) * static_cast<size_t>(s->inc_count)));
-    PK_CHECK(pk::launch_inc_slot_kernel(s->dyn_count, s->row_start.as<int>(), s->col.as<int>(),
-                                        s->inc_start.as<int>(), s->inc_list.as<int>(), s->tet_nodes.as<int4>(),
-                                        s->node_to_dyn.as<int>(), s->inc_slot.as<unsigned>(), s->stream));
+    if (s->tet_count >= (1 << 28) || s->inc_count >= (1 << 29)) return PK_OK;  // a list entry is 32 bits
+    PK_CHECK(s->blk_range.ensure(sizeof(int2) * static_cast<size_t>(s->nnz)));
+    PK_CHECK(s->blk_list.ensure(4 * sizeof(unsigned) * static_cast<size_t>(s->inc_count)));
+    PK_CHECK(s->blk_missing.ensure(sizeof(int)));
+    PK_CHECK(cudaMemsetAsync(s->blk_missing.p, 0, sizeof(int), s->stream));
+    PK_CHECK(pk::launch_block_list_kernel(s->dyn_count, s->row_start.as<int>(), s->col.as<int>(),
+                                          s->inc_start.as<int>(), s->inc_list.as<int>(), s->tet_nodes.as<int4>(),
+                                          s->node_to_dyn.as<int>(), s->blk_range.as<int2>(),
+                                          s->blk_list.as<unsigned>(), s->blk_missing.as<int>(), s->stream));
     s->launches += 1;
-    s->slots_ok = true;
+    s->lists_ok = true;
     return PK_OK;
 }
 
 template <class Real>
 int run_step(pk_system* s, const pk_step_params& p)
 {
-    if (const int rc = ensure_inc_slots(s)) return rc;
+    if (const int rc = ensure_block_lists(s)) return rc;
     PK_CHECK(cudaMemsetAsync(s->stats.p, 0, sizeof(pk::DevStats), s->stream));
     // A per-body part-resident layout from an earlier step: its round table for this solve
     // is built on the side stream while the step assembles.
@@ -1438,9 +1449,18 @@ int run_step(pk_system* s, const pk_step_params& p)
         PK_CHECK(cudaEventRecord(s->ev_pool[evi[2]], s->stream));
         s->ev_pending.push_back({evi[0], evi[1], evi[2]});
     }
-    PK_CHECK(cudaMemcpyAsync(s->host_stats, s->stats.p, sizeof(pk::DevStats), cudaMemcpyDeviceToHost, s->stream));
-    s->stats_pending = true;
+    s->stats_pending = true;  // fetched when somebody asks (pk_system_stats)
     if (!p.explicit_mode) s->assembled = true;
+    return PK_OK;
+}
+
+// The last step's statistics, if they are still on the device only (waits).
+int fetch_stats(pk_system* s)
+{
+    if (!s->stats_pending) return PK_OK;
+    PK_CHECK(cudaMemcpyAsync(s->host_stats, s->stats.p, sizeof(pk::DevStats), cudaMemcpyDeviceToHost, s->stream));
+    PK_CHECK(cudaStreamSynchronize(s->stream));
+    s->stats_pending = false;
     return PK_OK;
 }
 
@@ -1473,7 +1493,7 @@ int run_step_graph(pk_system* s, const pk_step_params& p)
         // Everything built lazily (allocations, uploads) must exist before the capture.
         int prc = ensure_batch_parts_any(s);
         if (!prc) prc = ensure_slab_any(s);
-        if (!prc) prc = ensure_inc_slots(s);
+        if (!prc) prc = ensure_block_lists(s);
         if (prc) return prc;
         const bool timing = s->timing;
         const long long launches = s->launches;
@@ -1633,7 +1653,7 @@ PKCUDA_API int pk_system_set_nodes(pk_system* s, int node_count, const int* node
     s->have_layout_x = false;
     s->have_snapshot = false;
     s->h_node_to_dyn.assign(node_to_dyn, node_to_dyn + node_count);
-    s->slots_ok = false;
+    s->lists_ok = false;
     s->h_mass.assign(mass, mass + node_count);
     int rc = upload_raw<int>(s->node_to_dyn, node_to_dyn, node_count, s->stream);
     if (!rc) rc = upload_real_any(s, s->mass, mass, node_count);
@@ -1922,7 +1942,7 @@ PKCUDA_API int pk_system_set_tets(pk_system* s, int tet_count, const int* tet_no
     for (long long i = 0; i < 4ll * tet_count; ++i)
         if (tet_nodes[i] < 0 || tet_nodes[i] >= s->node_count) return fail(PK_ERR_ARG, "tet node out of range");
     s->tet_count = tet_count;
-    s->slots_ok = false;
+    s->lists_ok = false;
     s->h_tet_nodes.assign(tet_nodes, tet_nodes + 4 * static_cast<size_t>(tet_count));
     s->h_enabled.assign(enabled, enabled + tet_count);
     s->h_damping.assign(damping, damping + tet_count);
@@ -1939,13 +1959,15 @@ PKCUDA_API int pk_system_set_tets(pk_system* s, int tet_count, const int* tet_no
     if (!rc) rc = upload_real_any(s, s->tet_params, params.data(), params.size());
     s->rest64_ok = false;
     if (rc) return rc;
-    PK_CHECK(s->tet_rec.ensure(pk::kTetRec * s->rsize() * std::max<size_t>(1, tet_count)));
+    const size_t rec = s->precision == PK_PREC_FP64 ? pk::tet_rec<double>() : pk::tet_rec<float>();
+    PK_CHECK(s->tet_rec.ensure(rec * s->rsize() * std::max<size_t>(1, tet_count)));
+    PK_CHECK(s->tet_rest.ensure(12 * s->rsize() * std::max<size_t>(1, tet_count)));
     if (s->precision == PK_PREC_FP64)
         PK_CHECK(pk::launch_tet_pack<double>(s->dm_inv.as<double>(), s->tet_params.as<double>(),
-                                             s->tet_rec.as<double>(), tet_count, s->stream));
+                                             s->tet_rest.as<double>(), tet_count, s->stream));
     else
-        PK_CHECK(pk::launch_tet_pack<float>(s->dm_inv.as<float>(), s->tet_params.as<float>(),
-                                            s->tet_rec.as<float>(), tet_count, s->stream));
+        PK_CHECK(pk::launch_tet_pack<float>(s->dm_inv.as<float>(), s->tet_params.as<float>(), s->tet_rest.as<float>(),
+                                            tet_count, s->stream));
     s->have_tets = true;
     return PK_OK;
 }
@@ -2107,7 +2129,7 @@ PKCUDA_API int pk_system_set_pattern(pk_system* s, int dyn_count, const int* dyn
     s->nnz = nnz;
     s->lt_count = static_cast<int>(ltr.size());
     s->inc_count = inc;
-    s->slots_ok = false;
+    s->lists_ok = false;
     s->max_row = max_row;
     s->diag_first = diag_first;
     int rc = upload_raw<int>(s->dyn_to_node, dyn_to_node, dyn_count, s->stream);
@@ -2188,6 +2210,7 @@ PKCUDA_API int pk_system_stats(pk_system* s, pk_step_stats* out)
 {
     if (!s || !out) return fail(PK_ERR_ARG, "stats");
     PK_CHECK(cudaSetDevice(s->device));
+    if (const int rc = fetch_stats(s)) return rc;
     PK_CHECK(cudaStreamSynchronize(s->stream));
     std::memset(out, 0, sizeof(*out));
     const pk::DevStats& d = *s->host_stats;
@@ -2237,7 +2260,7 @@ PKCUDA_API int pk_system_solve_given_f64(pk_system* s, const double* values, con
         else rc = run_pcg<double, double>(s, *p, 0);
         if (rc) return rc;
     }
-    PK_CHECK(cudaMemcpyAsync(s->host_stats, s->stats.p, sizeof(pk::DevStats), cudaMemcpyDeviceToHost, s->stream));
+    s->stats_pending = true;
     return PK_OK;
 }
 
@@ -2423,6 +2446,7 @@ PKCUDA_API int pk_system_autotune(pk_system* s, const pk_step_params* p, int rep
     if (!s->have_pattern || !s->assembled || s->dyn_count <= 0)
         return fail(PK_ERR_STATE, "autotune needs an assembled system (step once first)");
     PK_CHECK(cudaSetDevice(s->device));
+    if (const int rc = fetch_stats(s)) return rc;  // the timed solves overwrite them
     PK_CHECK(cudaStreamSynchronize(s->stream));
     drop_graph(s);
     repeats = std::max(1, repeats);
@@ -2542,8 +2566,8 @@ int adjoint_step(pk_system* s, const pk_step_params& p, const double* xbar_next,
     else if (s->precision == PK_PREC_MIXED) rc = run_pcg<float, double>(s, q, 0);
     else rc = run_pcg<double, double>(s, q, 0);
     if (rc) return rc;
-    PK_CHECK(cudaMemcpyAsync(s->host_stats, s->stats.p, sizeof(pk::DevStats), cudaMemcpyDeviceToHost, s->stream));
-    PK_CHECK(cudaStreamSynchronize(s->stream));
+    s->stats_pending = true;
+    if ((rc = fetch_stats(s))) return rc;
     if (!(s->host_stats->flags & PK_FLAG_SOLVED)) return fail(PK_ERR_STATE, "adjoint: the adjoint solve failed");
     std::vector<double> w(3 * static_cast<size_t>(n)), aw(3 * static_cast<size_t>(n));
     rc = download_real<Real>(s->px, w.data(), w.size(), s->stream);
