@@ -183,6 +183,75 @@ __global__ void __launch_bounds__(128) adjoint_tet_kernel(AdjointArgs<Real> A)
     }
 }
 
+template <class Real>
+__global__ void __launch_bounds__(128) adjoint_rhs_kernel(AdjointArgs<Real> A)
+{
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= A.rows) return;
+    const size_t node = 3 * (size_t)__ldg(A.dyn_to_node + r), o = 3 * (size_t)r;
+    for (int c = 0; c < 3; ++c) {
+        const double g = A.vbar[node + c] + A.dt_exact * A.xbar[node + c];
+        A.g[o + c] = g;
+        A.rhs[o + c] = Real(g);
+        A.du[o + c] = double(A.solution[o + c]);
+    }
+}
+
+template <class Real>
+__global__ void __launch_bounds__(256) adjoint_widen_kernel(AdjointArgs<Real> A)
+{
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 3 * (size_t)A.rows) A.w[i] = double(A.solution[i]);
+}
+
+// Node sensitivities before the step, a thread per dynamic row.  Positions: x' = x + dt v'
+// carries the adjoint of x' back unchanged, plus dJ/dx on dynamic nodes (fixed nodes never
+// move), the row's tets in tet order.  Velocities: v' = v + du carries g back on dynamic
+// rows, plus d(w.b)/dv = -dt^2 K w - dt c w with dt^2 K w = A w - m w (c: the damping of the
+// node's active tets); fixed nodes keep their adjoint (their velocity only enters through b's
+// coupling blocks, which the dynamic-row matrix does not hold: not propagated).
+template <class Real>
+__global__ void __launch_bounds__(64) adjoint_node_kernel(AdjointArgs<Real> A)
+{
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= A.rows) return;
+    const int node = __ldg(A.dyn_to_node + r);
+    const int i0 = __ldg(A.inc_start + r), i1 = __ldg(A.inc_start + r + 1);
+    double* xb = A.xbar + 3 * (size_t)node;
+    double x[3] = {xb[0], xb[1], xb[2]}, csum = 0.0;
+    constexpr int kBatch = 8;  // loads in flight
+    for (int i = i0; i < i1; i += kBatch) {
+        double f[kBatch][3], d[kBatch];
+        bool on[kBatch];
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q) {
+            const int code = i + q < i1 ? __ldg(A.inc_list + i + q) : -1;
+            on[q] = code >= 0 && (__ldg(A.enabled + (code >> 2)) & 1u);
+            if (!on[q]) continue;
+            const double* g = A.tet_grad + 12 * (size_t)(code >> 2) + 3 * (code & 3);
+            f[q][0] = g[0];
+            f[q][1] = g[1];
+            f[q][2] = g[2];
+            d[q] = __ldg(A.damping + (code >> 2));
+        }
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q)
+            if (on[q]) {
+                x[0] += f[q][0];
+                x[1] += f[q][1];
+                x[2] += f[q][2];
+                csum += d[q];
+            }
+    }
+    const double m = A.mass[node];
+    for (int c = 0; c < 3; ++c) {
+        xb[c] = x[c];
+        const double w = A.w[3 * (size_t)r + c];
+        A.vbar[3 * (size_t)node + c] = A.g[3 * (size_t)r + c] - double(A.product[3 * (size_t)r + c]) + m * w -
+                                       A.dt_exact * csum * w;
+    }
+}
+
 }  // namespace
 
 template <class Real>
@@ -194,6 +263,34 @@ cudaError_t launch_adjoint_tet_kernel(const AdjointArgs<Real>& args, cudaStream_
     return cudaGetLastError();
 }
 
+template <class Real>
+cudaError_t launch_adjoint_rhs_kernel(const AdjointArgs<Real>& args, cudaStream_t stream)
+{
+    if (args.rows <= 0) return cudaSuccess;
+    adjoint_rhs_kernel<Real><<<(args.rows + 127) / 128, 128, 0, stream>>>(args);
+    return cudaGetLastError();
+}
+template <class Real>
+cudaError_t launch_adjoint_widen_kernel(const AdjointArgs<Real>& args, cudaStream_t stream)
+{
+    if (args.rows <= 0) return cudaSuccess;
+    adjoint_widen_kernel<Real><<<(unsigned)((3 * (size_t)args.rows + 255) / 256), 256, 0, stream>>>(args);
+    return cudaGetLastError();
+}
+template <class Real>
+cudaError_t launch_adjoint_node_kernel(const AdjointArgs<Real>& args, cudaStream_t stream)
+{
+    if (args.rows <= 0) return cudaSuccess;
+    adjoint_node_kernel<Real><<<(args.rows + 63) / 64, 64, 0, stream>>>(args);
+    return cudaGetLastError();
+}
+
+template cudaError_t launch_adjoint_rhs_kernel<float>(const AdjointArgs<float>&, cudaStream_t);
+template cudaError_t launch_adjoint_rhs_kernel<double>(const AdjointArgs<double>&, cudaStream_t);
+template cudaError_t launch_adjoint_widen_kernel<float>(const AdjointArgs<float>&, cudaStream_t);
+template cudaError_t launch_adjoint_widen_kernel<double>(const AdjointArgs<double>&, cudaStream_t);
+template cudaError_t launch_adjoint_node_kernel<float>(const AdjointArgs<float>&, cudaStream_t);
+template cudaError_t launch_adjoint_node_kernel<double>(const AdjointArgs<double>&, cudaStream_t);
 template cudaError_t launch_adjoint_tet_kernel<float>(const AdjointArgs<float>&, cudaStream_t);
 template cudaError_t launch_adjoint_tet_kernel<double>(const AdjointArgs<double>&, cudaStream_t);
 

@@ -536,6 +536,7 @@ cudaError_t launch_elem_residual(const ElemResidualArgs<Real>& args, cudaStream_
 // log Young's modulus.
 template <class Real>
 struct AdjointArgs {
+    int rows;                // dynamic rows
     int tet_count;
     const int4* nodes;
     const unsigned char* enabled;
@@ -544,9 +545,20 @@ struct AdjointArgs {
     const Real* x;           // per world node
     const Real* v;
     const int* node_to_dyn;
-    const double* w;         // adjoint solution, per dynamic row
-    const double* du;        // the step's delta-v, per dynamic row
-    double dt;
+    const int* dyn_to_node;
+    const int* inc_start;    // incidence of the dynamic rows, as in AssemblyArgs
+    const int* inc_list;
+    const double* mass;      // per node
+    const double* damping;   // per tet
+    double* w;               // adjoint solution, per dynamic row
+    double* du;              // the step's delta-v, per dynamic row
+    double* g;               // adjoint right-hand side, per dynamic row
+    double* xbar;            // per node: the adjoints after the step, then before it
+    double* vbar;
+    Real* rhs;               // out: g in the storage type
+    const Real* solution;    // per dynamic row: of the last solve
+    const Real* product;     // A w
+    double dt, dt_exact;     // the step's dt in the storage type, and as given
     int linear;
     unsigned* flags;
     double* tet_grad;        // out: 12 per tet
@@ -584,6 +596,15 @@ template <class Real, class Acc>
 int pcg_max_grid(int threads, bool staged);
 template <class Real>
 cudaError_t launch_spmv_kernel(const BsrView<Real>& a, const Real* x, Real* y, cudaStream_t stream);
+// g = vbar + dt xbar on the dynamic rows (into g and rhs); du = the last solution.
+template <class Real>
+cudaError_t launch_adjoint_rhs_kernel(const AdjointArgs<Real>& args, cudaStream_t stream);
+// w = the last solution, in double.
+template <class Real>
+cudaError_t launch_adjoint_widen_kernel(const AdjointArgs<Real>& args, cudaStream_t stream);
+// The nodes' adjoints before the step, from the tets' gradients, in place.
+template <class Real>
+cudaError_t launch_adjoint_node_kernel(const AdjointArgs<Real>& args, cudaStream_t stream);
 template <class Real>
 cudaError_t launch_adjoint_tet_kernel(const AdjointArgs<Real>& args, cudaStream_t stream);
 // Batched per-body PCG (pk_pcg_batch.cu): cooperative, one block per body part.
