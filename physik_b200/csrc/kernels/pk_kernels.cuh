@@ -422,6 +422,7 @@ struct ResPcgArgs {
     int n;
     int lpr;                         // lanes per row: 1, 2, 4 or 8
     int nslots;                      // slots per thread
+    int tmem_slots;                  // of them in tensor memory
     int max_halo;                    // most halo rows of a part (clusters: the inbox's rows)
     const int* part_info;            // [grid] x kResPartInts
     const int* perm;                 // part order -> dynamic row
@@ -633,7 +634,7 @@ cudaError_t launch_slab_fill_kernel(const float* values, int nnz, const int* til
 // Resident PCG (pk_pcg_res.cu): `grid` blocks of `threads`, in clusters of `cluster` blocks
 // or, with 0, as a cooperative launch.
 template <class Real>
-cudaError_t launch_pcg_res_kernel(const ResPcgArgs<Real>& args, int threads, int cluster, int grid,
+cudaError_t launch_pcg_res_kernel(const ResPcgArgs<Real>& args, int threads, int rpt, int cluster, int grid,
                                   cudaStream_t stream);
 template <class Real>
 ResLimits pcg_res_limits();

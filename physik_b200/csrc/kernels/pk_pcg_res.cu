@@ -9,8 +9,13 @@
 // in two grid exchanges and the loads around them.  Here
 //
 // * every block loads its part's rows once, straight from the assembled blocks, into
-//   shared memory and registers; x, r, s, d and M^-1 of a row stay in the registers of the
-//   lane that owns it.
+//   registers, tensor memory and shared memory; x, r, s, d and M^-1 of a row stay in the
+//   registers of the lane that owns it.
+// * parts of more than 256 rows (FP32) give a thread two rows and keep most of the blocks in
+//   tensor memory: a warp's tcgen05.ld of 36 words a thread brings four blocks without using
+//   the shared memory's bandwidth, and its 256 KB beside the 224 KB of shared memory hold a
+//   part of 640 rows of 15 blocks (94,000 rows on the GPU).  FP64 uses it where registers and
+//   shared memory are too small.
 // * an iteration has one exchange.  The blocks publish, with the partial sums of d.q, the
 //   rows of q = A d that other parts' windows hold; every block then knows alpha and beta
 //   and updates r, s = M^-1 r and d of its halo rows itself, with the same operations as
@@ -31,7 +36,8 @@
 //
 // Measured per CG iteration against the streaming kernels (part-resident stream for FP32
 // storage, ring for FP64): 8x8x8 box FP32 1.8 us (7.2), 32x8x8 beam FP64 3.0 us (13.3),
-// 64x16x16 beam 3.3 us mixed (10.9) and 4.2 us FP64 (18.5).  What is left is a chain of
+// 64x16x16 beam 3.3 us mixed (10.9) and 4.2 us FP64 (18.5), 61x47x29 block mixed (594 rows a
+// part) 6.7 us (19.3).  What is left is a chain of
 // latencies: about 3,000 cycles of a block's own work (product, two sets of FP64 sums by
 // shuffles, the scalars, the updates; 8.6 cycles an FP64 add, 24 a shuffle, 45 a barrier of
 // 512 threads) and the exchange.
@@ -202,12 +208,58 @@ __device__ __forceinline__ void cluster_barrier()
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// 36 words of a thread's tensor memory (the warp's lanes, 36 columns), each waiting for its
+// own completion.
+struct Words {
+    unsigned w[kResTmemWords];
+};
+#define PK_W(i) "=r"(t.w[i]), "=r"(t.w[i + 1]), "=r"(t.w[i + 2]), "=r"(t.w[i + 3])
+__device__ __forceinline__ void tmem_ld36(unsigned addr, Words& t)
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
+        "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%36];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%32,%33,%34,%35}, [%37];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : PK_W(0), PK_W(4), PK_W(8), PK_W(12), PK_W(16), PK_W(20), PK_W(24), PK_W(28), PK_W(32)
+        : "r"(addr), "r"(addr + 32u)
+        : "memory");
+}
+#undef PK_W
+#define PK_W(i) "r"(t.w[i]), "r"(t.w[i + 1]), "r"(t.w[i + 2]), "r"(t.w[i + 3])
+__device__ __forceinline__ void tmem_st36(unsigned addr, const Words& t)
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%36], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,"
+        "%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};\n\t"
+        "tcgen05.st.sync.aligned.32x32b.x4.b32 [%37], {%32,%33,%34,%35};\n\t"
+        "tcgen05.wait::st.sync.aligned;" ::PK_W(0),
+        PK_W(4), PK_W(8), PK_W(12), PK_W(16), PK_W(20), PK_W(24), PK_W(28), PK_W(32), "r"(addr), "r"(addr + 32u)
+        : "memory");
+}
+#undef PK_W
+__device__ __forceinline__ float words_at(const Words& t, int i, float) { return __uint_as_float(t.w[i]); }
+__device__ __forceinline__ double words_at(const Words& t, int i, double)
+{
+    return __hiloint2double((int)t.w[2 * i + 1], (int)t.w[2 * i]);
+}
+__device__ __forceinline__ void words_set(Words& t, int i, float v) { t.w[i] = __float_as_uint(v); }
+__device__ __forceinline__ void words_set(Words& t, int i, double v)
+{
+    t.w[2 * i] = (unsigned)__double2loint(v);
+    t.w[2 * i + 1] = (unsigned)__double2hiint(v);
+}
+
 // MAXT: threads per block at most (256 leaves a thread twice the registers of 512).
 // CL: exchange inside a cluster (else through global memory).
-template <class Real, int MAXT, bool CL>
+// R: rows per thread (2: one lane a row, rows tid and tid + T, whose entries alternate in the
+// slots).  TM: slots in tensor memory.
+template <class Real, int MAXT, bool CL, int R, bool TM>
 __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
 {
-    constexpr int KR = res_reg_slots(sizeof(Real), MAXT);
+    constexpr int KR = res_reg_slots(sizeof(Real), MAXT, R);
+    constexpr int KB = res_tmem_batch(sizeof(Real));
+    static_assert(KR % R == 0 && KB % R == 0, "a slot's row is known at compile time");
     constexpr int NH = kResHaloPerThread;
     constexpr int RB = (int)res_row_packet(sizeof(Real));
     extern __shared__ __align__(128) unsigned char dyn[];
@@ -217,6 +269,7 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
     __shared__ unsigned sh_bits[3], sh_gbits[3];  // flags by exchange number
     __shared__ __align__(8) unsigned long long sh_bar[2];
     __shared__ int s_fail;
+    __shared__ unsigned s_tmem;
 
     const int T = blockDim.x, W = T >> 5, lpr = P.lpr;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, blk = blockIdx.x;
@@ -243,9 +296,16 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
         bad0 = 4u;
     }
     int nslots = P.nslots;
-    if (m < 0 || m * lpr > T || h < 0 || h > NH * T || h > P.max_halo || row0 < 0 || row0 + m > P.n || halo0 < 0 ||
-        halo0 + h > P.halo_count || sends_n < 0 || send0 < 0 || send0 + sends_n > P.halo_count || nslots < 0 || slot0 < 0 || slot0 + nslots > P.slot_count ||
-        res_smem_bytes(sizeof(Real), T, m, h, nslots, CL ? 1 : 0, P.max_halo) > P.smem_bytes) {
+    // (the launch's tensor memory: the host's rule, else none)
+    const int tslots = TM && P.tmem_slots > 0 && P.tmem_slots <= res_tmem_slots(sizeof(Real), T) &&
+                               P.tmem_slots % KB == 0 && P.smem_bytes >= kResAloneBytes
+                           ? P.tmem_slots
+                           : 0;
+    const int s0 = KR + tslots;  // first slot in shared memory
+    if (m < 0 || m * lpr > T * R || (R > 1 && lpr != 1) || nslots % R != 0 || h < 0 || h > NH * T || h > P.max_halo ||
+        row0 < 0 || row0 + m > P.n || halo0 < 0 || halo0 + h > P.halo_count || sends_n < 0 || send0 < 0 ||
+        send0 + sends_n > P.halo_count || nslots < 0 || slot0 < 0 || slot0 + nslots > P.slot_count ||
+        res_smem_bytes(sizeof(Real), T, m, h, max(0, nslots - s0), tslots, CL ? 1 : 0, P.max_halo) > P.smem_bytes) {
         m = h = nslots = sends_n = 0;
         bad0 = 4u;
     }
@@ -281,7 +341,7 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
     off += res_align(3 * (size_t)m * sizeof(Real));
     // [slot][thread][element]: nine words apart, so a warp's reads hit different banks
     Real* const vals = reinterpret_cast<Real*>(dyn + off);
-    off += res_align((size_t)max(0, nslots - KR) * T * 9 * sizeof(Real));
+    off += res_align((size_t)max(0, nslots - s0) * T * 9 * sizeof(Real));
     unsigned short* const cols = reinterpret_cast<unsigned short*>(dyn + off);
     if (tid == 0) {
         for (int i = 0; i < 3; ++i) sh_bits[i] = sh_gbits[i] = 0u;
@@ -292,44 +352,64 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
             mbar_fence_init();
         }
     }
+    if (TM && tslots > 0 && warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)),
+                     "r"(512u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (TM) asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     unsigned epoch = 0u;
     if (!CL && gsize > 1) epoch = *(volatile unsigned*)(P.epoch + gfirst);
     if (CL)
         cluster_barrier();  // every block's barriers exist before anybody writes to them
     else
         __syncthreads();
+    if (TM) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const unsigned tmem0 = TM && tslots > 0 ? s_tmem + ((32u * (unsigned)(warp & 3)) << 16) +
+                                                   (unsigned)(warp >> 2) * (unsigned)res_tmem_columns(T)
+                                             : 0u;
     if (idle) {
         cluster_barrier();
         return;
     }
 
-    // Thread i < m owns row i: its vectors and M^-1 stay in its registers.  Packing the rows
-    // into the first warps keeps the FP64 work of the sums off the others.  The last threads
-    // hold the halo rows.
-    const bool has = tid < m;
-    const int owner_warps = (m + 31) / 32;
+    // Thread i owns row i < m (R = 2: and row i + T): its vectors and M^-1 stay in its
+    // registers.  Packing the rows into the first warps keeps the FP64 work of the sums off the
+    // others.  The last threads hold the halo rows.
+    bool has[R];
+#pragma unroll
+    for (int p = 0; p < R; ++p) has[p] = tid + p * T < m;
+    const int owner_warps = ((R == 1 ? m : min(m, T)) + 31) / 32;
+    // the row that this thread's lane group completes (R = 1; m: none)
+    const int qrow = tid % lpr == 0 ? tid / lpr : m;
     const int htid = T - 1 - tid;
     const V3<Real> zero{Real(0), Real(0), Real(0)};
-    int cidx = -1;
+    int cidx[R];
     // the rows this thread sends {row, place}: the first few in registers
     int2 send[kResSendRegs];
 #pragma unroll
     for (int u = 0; u < kResSendRegs; ++u)
         send[u] = tid + u * T < sends_n ? __ldg(P.send + send0 + tid + u * T) : make_int2(-1, -1);
-    V3<Real> xv = zero, rv = zero, sv = zero, dv = zero, qv = zero;
-    Real mi[9];
-#pragma unroll
-    for (int e = 0; e < 9; ++e) mi[e] = Real(0);
+    V3<Real> xv[R], rv[R], sv[R], dv[R], qv[R];
+    Real mi[R][9];
     unsigned bad = bad0;
-    if (has) {
-        cidx = __ldg(P.perm + row0 + tid);
-        if ((unsigned)cidx >= (unsigned)P.n) {
-            cidx = -1;
-            bad |= 4u;
-        } else {
-            rv = ld3(P.b, cidx);
 #pragma unroll
-            for (int e = 0; e < 9; ++e) mi[e] = __ldg(P.minv + 9 * (size_t)cidx + e);
+    for (int p = 0; p < R; ++p) {
+        xv[p] = rv[p] = sv[p] = dv[p] = qv[p] = zero;
+        cidx[p] = -1;
+#pragma unroll
+        for (int e = 0; e < 9; ++e) mi[p][e] = Real(0);
+        if (has[p]) {
+            const int c = __ldg(P.perm + row0 + tid + p * T);
+            if ((unsigned)c >= (unsigned)P.n) {
+                bad |= 4u;
+            } else {
+                cidx[p] = c;
+                rv[p] = ld3(P.b, c);
+#pragma unroll
+                for (int e = 0; e < 9; ++e) mi[p][e] = __ldg(P.minv + 9 * (size_t)c + e);
+            }
         }
     }
     // Halo rows: r = b and M^-1 in shared memory, d = s in the window.
@@ -361,7 +441,8 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
             d[2] = s.z;
         }
     }
-    // The part's blocks: the first KR slots in registers, the others in shared memory.
+    // The part's blocks: the first KR slots in registers, then those in tensor memory, the
+    // others in shared memory.
     Real rval[KR > 0 ? KR : 1][9];
     int rcol[KR > 0 ? KR : 1];
     auto load_entry = [&](int slot, Real (&v)[9]) -> int {
@@ -386,40 +467,59 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
         for (int e = 0; e < 9; ++e) rval[k][e] = Real(0);
         if (k < nslots) rcol[k] = load_entry(k, rval[k]);
     }
+    // (columns of all but the register slots go to shared memory)
+    for (int k0 = KR; TM && k0 < s0; k0 += KB) {
+        Words t;
+#pragma unroll
+        for (int u = 0; u < KB; ++u) {
+            Real v[9] = {};
+            const int c = k0 + u < nslots ? load_entry(k0 + u, v) : 0;
+#pragma unroll
+            for (int e = 0; e < 9; ++e) words_set(t, 9 * u + e, v[e]);
+            cols[(size_t)(k0 + u - KR) * T + tid] = (unsigned short)c;
+        }
+        __syncwarp();
+        tmem_st36(tmem0 + (unsigned)((k0 - KR) / KB * kResTmemWords), t);
+    }
 #pragma unroll 2
-    for (int k = KR; k < nslots; ++k) {
+    for (int k = s0; k < nslots; ++k) {
         Real v[9];
-        const size_t at = (size_t)(k - KR) * T + tid;
-        cols[at] = (unsigned short)load_entry(k, v);
+        const size_t at = (size_t)(k - s0) * T + tid;
+        cols[(size_t)(k - KR) * T + tid] = (unsigned short)load_entry(k, v);
 #pragma unroll
         for (int e = 0; e < 9; ++e) vals[9 * at + e] = v[e];
     }
 
     unsigned fl = 0;
-    int iterations = 0, it = 0, node = 0;
+    int iterations = 0, it = 0, node[R];
     bool converged = false, have_x = true, timed_out = false;
     bool ran = false;      // the iteration was entered: the residual norm is reported
     bool pending = false;  // the last iteration's r.s comes with the next exchange
     double residual = 0.0, delta = 0.0, target = 0.0, rs_next = 0.0;
     unsigned sbad = 0, gen = 0;
-    V3<Real> hq[NH], hs[NH], nx = zero, nv = zero;
+    V3<Real> hq[NH], hs[NH], nx[R], nv[R];
 #pragma unroll
     for (int u = 0; u < NH; ++u) hq[u] = hs[u] = zero;
-    if (has && cidx >= 0) {
-        if (!finite3(rv)) bad |= 1u;
-        sv = apply_minv(mi, rv);
-        bool fin = finite3(sv);
 #pragma unroll
-        for (int e = 0; e < 9; ++e) fin = fin && isfinite(mi[e]);
-        if (!fin) bad |= 2u;
-        dv = sv;
-        rs_next = dot_acc<double>(rv, sv);
-    }
-    if (has) {
-        Real* d = win + 3 * tid;
-        d[0] = dv.x;
-        d[1] = dv.y;
-        d[2] = dv.z;
+    for (int p = 0; p < R; ++p) {
+        node[p] = 0;
+        nx[p] = nv[p] = zero;
+        if (has[p] && cidx[p] >= 0) {
+            if (!finite3(rv[p])) bad |= 1u;
+            sv[p] = apply_minv(mi[p], rv[p]);
+            bool fin = finite3(sv[p]);
+#pragma unroll
+            for (int e = 0; e < 9; ++e) fin = fin && isfinite(mi[p][e]);
+            if (!fin) bad |= 2u;
+            dv[p] = sv[p];
+            rs_next += dot_acc<double>(rv[p], sv[p]);
+        }
+        if (has[p]) {
+            Real* d = win + 3 * (tid + p * T);
+            d[0] = dv[p].x;
+            d[1] = dv[p].y;
+            d[2] = dv[p].z;
+        }
     }
 
     // The end of an iteration whose r.s is known: false ends the solve.
@@ -448,15 +548,24 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
         unsigned bits = 0;
         if (turn == kProducts) {
             // q = A d for the part's rows.
-            V3<Real> acc = zero;
+            V3<Real> acc[R];
+#pragma unroll
+            for (int p = 0; p < R; ++p) acc[p] = zero;
+            auto mul = [&](V3<Real>& y, const auto& e, const Real* d) {
+                const Real dx = d[0], dy = d[1], dz = d[2];
+                y.x += e(0) * dx + e(3) * dy + e(6) * dz;
+                y.y += e(1) * dx + e(4) * dy + e(7) * dz;
+                y.z += e(2) * dx + e(5) * dy + e(8) * dz;
+            };
             auto mul_regs = [&](auto count) {
 #pragma unroll
                 for (int k = 0; k < decltype(count)::value; ++k) {
                     const Real* d = win + rcol[k];
                     const Real dx = d[0], dy = d[1], dz = d[2];
-                    acc.x += rval[k][0] * dx + rval[k][3] * dy + rval[k][6] * dz;
-                    acc.y += rval[k][1] * dx + rval[k][4] * dy + rval[k][7] * dz;
-                    acc.z += rval[k][2] * dx + rval[k][5] * dy + rval[k][8] * dz;
+                    V3<Real>& y = acc[k % R];
+                    y.x += rval[k][0] * dx + rval[k][3] * dy + rval[k][6] * dz;
+                    y.y += rval[k][1] * dx + rval[k][4] * dy + rval[k][7] * dz;
+                    y.z += rval[k][2] * dx + rval[k][5] * dy + rval[k][8] * dz;
                 }
             };
             if (KR > 0) {  // (a slot the plan does not have is a zero block)
@@ -467,31 +576,55 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
                 else
                     mul_regs(std::integral_constant<int, (KR + 3) / 4>{});
             }
-            {
-                const unsigned short* cp = cols + tid;
-                const Real* e = vals + 9 * tid;
-#pragma unroll 4
-                for (int k = KR; k < nslots; ++k, cp += T, e += 9 * T) {
-                    const Real* d = win + *cp;
-                    const Real dx = d[0], dy = d[1], dz = d[2];
-                    acc.x += e[0] * dx + e[3] * dy + e[6] * dz;
-                    acc.y += e[1] * dx + e[4] * dy + e[7] * dz;
-                    acc.z += e[2] * dx + e[5] * dy + e[8] * dz;
+            const unsigned short* cp = cols + tid;
+            if (TM) {
+                for (int k0 = KR; k0 < s0; k0 += KB, cp += KB * T) {
+                    const Real* d[KB];
+#pragma unroll
+                    for (int u = 0; u < KB; ++u) d[u] = win + cp[u * T];
+                    Words t;
+                    tmem_ld36(tmem0 + (unsigned)((k0 - KR) / KB * kResTmemWords), t);
+#pragma unroll
+                    for (int u = 0; u < KB; ++u)
+                        mul(acc[u % R], [&](int e) { return words_at(t, 9 * u + e, Real()); }, d[u]);
                 }
             }
-#pragma unroll
-            for (int o = 4; o > 0; o >>= 1)
-                if (lpr > o) {
-                    acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
-                    acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
-                    acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o);
+            if constexpr (R == 1) {
+                const Real* e = vals + 9 * tid;
+#pragma unroll 4
+                for (int k = s0; k < nslots; ++k, cp += T, e += 9 * T) {
+                    const Real* d = win + *cp;
+                    const Real dx = d[0], dy = d[1], dz = d[2];
+                    acc[0].x += e[0] * dx + e[3] * dy + e[6] * dz;
+                    acc[0].y += e[1] * dx + e[4] * dy + e[7] * dz;
+                    acc[0].z += e[2] * dx + e[5] * dy + e[8] * dz;
                 }
-            const int row = tid / lpr;
-            if (tid % lpr == 0 && row < m) {
-                Real* q = qbuf + 3 * row;
-                q[0] = acc.x;
-                q[1] = acc.y;
-                q[2] = acc.z;
+            } else {
+                const Real* e = vals + 9 * tid;
+#pragma unroll 2
+                for (int k = s0; k < nslots; k += R)
+#pragma unroll
+                    for (int p = 0; p < R; ++p, cp += T, e += 9 * T)
+                        mul(acc[p], [&](int i) { return e[i]; }, win + *cp);
+            }
+            if (R == 1) {
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1)
+                    if (lpr > o) {
+                        acc[0].x += __shfl_xor_sync(0xffffffffu, acc[0].x, o);
+                        acc[0].y += __shfl_xor_sync(0xffffffffu, acc[0].y, o);
+                        acc[0].z += __shfl_xor_sync(0xffffffffu, acc[0].z, o);
+                    }
+            }
+#pragma unroll
+            for (int p = 0; p < R; ++p) {
+                const int row = R == 1 ? qrow : tid + p * T;
+                if (row < m) {
+                    Real* q = qbuf + 3 * row;
+                    q[0] = acc[p].x;
+                    q[1] = acc[p].y;
+                    q[2] = acc[p].z;
+                }
             }
             __syncthreads();
             bits = sbad;
@@ -512,29 +645,37 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
 #pragma unroll
             for (int u = 0; u < kResSendRegs; ++u) send_row(send[u]);
             for (int e = tid + kResSendRegs * T; e < sends_n; e += T) send_row(__ldg(P.send + send0 + e));
-            if (has) {
-                qv = V3<Real>{qbuf[3 * tid], qbuf[3 * tid + 1], qbuf[3 * tid + 2]};
-                if (!finite3(qv)) bits |= 1u;
-                const V3<Real> z = apply_minv(mi, qv);
-                v[0] = dot_acc<double>(dv, qv);
-                v[1] = dot_acc<double>(qv, sv) + dot_acc<double>(rv, z);
-                v[2] = dot_acc<double>(qv, z);
-                v[3] = rs_next;
-            }
+#pragma unroll
+            for (int p = 0; p < R; ++p)
+                if (has[p]) {
+                    const Real* q = qbuf + 3 * (tid + p * T);
+                    qv[p] = V3<Real>{q[0], q[1], q[2]};
+                    if (!finite3(qv[p])) bits |= 1u;
+                    const V3<Real> z = apply_minv(mi[p], qv[p]);
+                    const double dq = dot_acc<double>(dv[p], qv[p]), qz = dot_acc<double>(qv[p], z),
+                                 slope = dot_acc<double>(qv[p], sv[p]) + dot_acc<double>(rv[p], z);
+                    v[0] = p == 0 ? dq : v[0] + dq;
+                    v[1] = p == 0 ? slope : v[1] + slope;
+                    v[2] = p == 0 ? qz : v[2] + qz;
+                }
+            v[3] = rs_next;
         } else if (turn == kEnd) {
             // delta-v back in dynamic-row order; the solve succeeds when it is present and
             // finite; integration is all-or-nothing.
-            if (has) v[0] = dot_acc<double>(rv, rv);
-            if (has && cidx >= 0) {
-                if (!have_x) xv = zero;
-                st3(P.x, cidx, xv);
-                if (!finite3(xv)) bits |= 1u;
-                if (P.integrate) {
-                    node = __ldg(P.dyn_to_node + cidx);
-                    const V3<Real> xo = ldplain3(P.node_x, node), vo = ldplain3(P.node_v, node);
-                    nv = vo + xv;
-                    nx = xo + nv * P.dt;
-                    if (!finite3(xo) || !finite3(vo) || !finite3(nv) || !finite3(nx)) bits |= 2u;
+#pragma unroll
+            for (int p = 0; p < R; ++p) {
+                if (has[p]) v[0] += dot_acc<double>(rv[p], rv[p]);
+                if (has[p] && cidx[p] >= 0) {
+                    if (!have_x) xv[p] = zero;
+                    st3(P.x, cidx[p], xv[p]);
+                    if (!finite3(xv[p])) bits |= 1u;
+                    if (P.integrate) {
+                        node[p] = __ldg(P.dyn_to_node + cidx[p]);
+                        const V3<Real> xo = ldplain3(P.node_x, node[p]), vo = ldplain3(P.node_v, node[p]);
+                        nv[p] = vo + xv[p];
+                        nx[p] = xo + nv[p] * P.dt;
+                        if (!finite3(xo) || !finite3(vo) || !finite3(nv[p]) || !finite3(nx[p])) bits |= 2u;
+                    }
                 }
             }
         } else {
@@ -717,10 +858,12 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
                 if (bits & 2u) {
                     fl |= kFlagIntegrateAbort;
                 } else {
-                    if (has && cidx >= 0) {
-                        st3(P.node_v, node, nv);
-                        st3(P.node_x, node, nx);
-                    }
+#pragma unroll
+                    for (int p = 0; p < R; ++p)
+                        if (has[p] && cidx[p] >= 0) {
+                            st3(P.node_v, node[p], nv[p]);
+                            st3(P.node_x, node[p], nx[p]);
+                        }
                     fl |= kFlagIntegrated;
                 }
             }
@@ -780,13 +923,16 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
             const Scale<Real> pa(alpha), na = pa.negated();
             sbad = 0;
             rs_next = 0.0;
-            if (has) {
-                xv = pa.axpy(dv, xv);
-                rv = na.axpy(qv, rv);
-                sv = apply_minv(mi, rv);
-                if (!finite3(sv)) sbad = 2u;
-                rs_next = dot_acc<double>(rv, sv);
-            }
+#pragma unroll
+            for (int p = 0; p < R; ++p)
+                if (has[p]) {
+                    xv[p] = pa.axpy(dv[p], xv[p]);
+                    rv[p] = na.axpy(qv[p], rv[p]);
+                    sv[p] = apply_minv(mi[p], rv[p]);
+                    if (!finite3(sv[p])) sbad = 2u;
+                    const double rs = dot_acc<double>(rv[p], sv[p]);
+                    rs_next = p == 0 ? rs : rs_next + rs;
+                }
 #pragma unroll
             for (int u = 0; u < NH; ++u) {
                 const int j = htid + u * T;
@@ -817,13 +963,15 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
         }
         // d = s + beta d: the owned row, then the halo copies.
         const Real bt = Real(beta);
-        if (has) {
-            dv = fma3(bt, dv, sv);
-            Real* d = win + 3 * tid;
-            d[0] = dv.x;
-            d[1] = dv.y;
-            d[2] = dv.z;
-        }
+#pragma unroll
+        for (int p = 0; p < R; ++p)
+            if (has[p]) {
+                dv[p] = fma3(bt, dv[p], sv[p]);
+                Real* d = win + 3 * (tid + p * T);
+                d[0] = dv[p].x;
+                d[1] = dv[p].y;
+                d[2] = dv[p].z;
+            }
 #pragma unroll
         for (int u = 0; u < NH; ++u) {
             const int j = htid + u * T;
@@ -869,17 +1017,32 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
     } else if (timed_out && tid == 0) {
         atomicOr(P.flags, kFlagBarrierTimeout);
     }
+    if (TM && tslots > 0) {
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        if (warp == 0) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s_tmem), "r"(512u) : "memory");
+        }
+    }
     if (CL) cluster_barrier();  // nobody's shared memory goes while a peer may still write to it
 }
 
 template <class Real>
-const void* res_kernel(int threads, bool cluster)
+const void* res_kernel(int threads, bool cluster, int rpt, bool tmem)
 {
     if (cluster)
-        return threads <= 256 ? (const void*)pcg_res_kernel<Real, 256, true>
-                              : (const void*)pcg_res_kernel<Real, 512, true>;
-    return threads <= 256 ? (const void*)pcg_res_kernel<Real, 256, false>
-                          : (const void*)pcg_res_kernel<Real, 512, false>;
+        return threads <= 256 ? (const void*)pcg_res_kernel<Real, 256, true, 1, false>
+                              : (const void*)pcg_res_kernel<Real, 512, true, 1, false>;
+    if (rpt == 1 && threads <= 256) {
+        if constexpr (sizeof(Real) == 8)
+            if (tmem) return (const void*)pcg_res_kernel<Real, 256, false, 1, true>;
+        return (const void*)pcg_res_kernel<Real, 256, false, 1, false>;
+    }
+    if constexpr (sizeof(Real) == 4)
+        return (const void*)pcg_res_kernel<Real, kResPairThreads, false, 2, true>;  // (never asked for 512 threads)
+    else
+        return (const void*)pcg_res_kernel<Real, 512, false, 1, false>;
 }
 
 template <class Real>
@@ -889,17 +1052,20 @@ ResLimits query_limits(int dev)
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return lim;
     int per_sm = 1 << 20;
-    for (const int threads : {256, 512})
-        for (const bool cl : {false, true}) {
-            const void* k = res_kernel<Real>(threads, cl);
-            int b = 0;
-            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmemLimit) !=
-                    cudaSuccess ||
-                (cl && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, threads, kResSmemLimit) != cudaSuccess)
-                return lim;
-            per_sm = b < per_sm ? b : per_sm;
-        }
+    struct {
+        int threads, rpt;
+        bool cluster, tmem;
+    } const kinds[] = {{256, 1, false, false}, {256, 1, false, true}, {256, 1, true, false}, {512, 1, true, false},
+                       {sizeof(Real) == 4 ? kResPairThreads : 512, sizeof(Real) == 4 ? 2 : 1, false, false}};
+    for (const auto& kind : kinds) {
+        const void* k = res_kernel<Real>(kind.threads, kind.cluster, kind.rpt, kind.tmem);
+        int b = 0;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmemLimit) != cudaSuccess ||
+            (kind.cluster && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, kind.threads, kResSmemLimit) != cudaSuccess)
+            return lim;
+        per_sm = b < per_sm ? b : per_sm;
+    }
     lim.blocks = sms * per_sm;
     for (int q = 0; q < 5; ++q) {
         lim.clusters[q] = 1 << 20;
@@ -915,7 +1081,7 @@ ResLimits query_limits(int dev)
             c.attrs = &a;
             c.numAttrs = 1;
             int k = 0;
-            if (cudaOccupancyMaxActiveClusters(&k, res_kernel<Real>(threads, true), &c) != cudaSuccess) {
+            if (cudaOccupancyMaxActiveClusters(&k, res_kernel<Real>(threads, true, 1, false), &c) != cudaSuccess) {
                 cudaGetLastError();
                 k = 0;
             }
@@ -942,7 +1108,8 @@ ResLimits pcg_res_limits()
 }
 
 template <class Real>
-cudaError_t launch_pcg_res_kernel(const ResPcgArgs<Real>& args, int threads, int cluster, int grid, cudaStream_t stream)
+cudaError_t launch_pcg_res_kernel(const ResPcgArgs<Real>& args, int threads, int rpt, int cluster, int grid,
+                                  cudaStream_t stream)
 {
     ResPcgArgs<Real> a = args;
     void* kargs[] = {&a};
@@ -962,11 +1129,11 @@ cudaError_t launch_pcg_res_kernel(const ResPcgArgs<Real>& args, int threads, int
     }
     c.attrs = &at;
     c.numAttrs = 1;
-    return cudaLaunchKernelExC(&c, res_kernel<Real>(threads, cluster > 0), kargs);
+    return cudaLaunchKernelExC(&c, res_kernel<Real>(threads, cluster > 0, rpt, args.tmem_slots > 0), kargs);
 }
 
-template cudaError_t launch_pcg_res_kernel<float>(const ResPcgArgs<float>&, int, int, int, cudaStream_t);
-template cudaError_t launch_pcg_res_kernel<double>(const ResPcgArgs<double>&, int, int, int, cudaStream_t);
+template cudaError_t launch_pcg_res_kernel<float>(const ResPcgArgs<float>&, int, int, int, int, cudaStream_t);
+template cudaError_t launch_pcg_res_kernel<double>(const ResPcgArgs<double>&, int, int, int, int, cudaStream_t);
 template ResLimits pcg_res_limits<float>();
 template ResLimits pcg_res_limits<double>();
 

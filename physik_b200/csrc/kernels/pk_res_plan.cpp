@@ -28,6 +28,7 @@ double exchange_cycles(int group, bool cluster)
 struct Cut {
     int per, cluster, cap;
     double cycles;
+    bool pairs = false;  // two rows a thread
 };
 
 // Lanes per row, the most that keep the block under its threads, and the threads.
@@ -134,15 +135,19 @@ std::string build_cut(int n, const int* row_start, const int* col, const int* lt
         }
     }
     // 2. lanes
-    const Lanes lanes = lanes_for(out.max_rows, cut.cap);
-    if (lanes.threads > kResMaxThreads) return "a part has more rows than threads";
+    const Lanes lanes = cut.pairs ? Lanes{1, std::max(kResMinThreads, (out.max_rows + 63) / 64 * 32)}
+                                  : lanes_for(out.max_rows, cut.cap);
+    if (lanes.threads > (cut.pairs ? kResPairThreads : kResMaxThreads)) return "a part has more rows than threads";
     out.lpr = lanes.lpr;
     out.threads = lanes.threads;
+    out.rpt = cut.pairs ? 2 : 1;
+    out.real = real;
     out.n = n;
     out.parts = parts;
     out.cluster = cut.cluster;
     const int T = out.threads;
     for (int r = 0; r < n; ++r) out.slots = std::max(out.slots, (len[r] + out.lpr - 1) / out.lpr);
+    out.slots *= out.rpt;
     // 3. part order: parts in order, rows ascending
     std::vector<int> start(parts + 1, 0), inv(n);
     for (int p = 0; p < parts; ++p) start[p + 1] = start[p] + rows_of[p];
@@ -194,10 +199,25 @@ std::string build_cut(int n, const int* row_start, const int* col, const int* lt
         out.max_halo = std::max(out.max_halo, h);
         out.halo_src.insert(out.halo_src.end(), halo.begin(), halo.end());
     }
-    for (int p = 0; p < parts; ++p)
-        out.smem_bytes =
-            std::max(out.smem_bytes, res_smem_bytes(real, T, rows_of[p], out.part_info[(size_t)kResPartInts * p + 3],
-                                                    out.slots, out.cluster, out.max_halo));
+    // Tensor memory takes as many slots as it holds where a thread has two rows, and in FP64
+    // where shared memory is too small (the path costs 2 % where it is not): blocks that may share an SM (half its
+    // shared memory each) must not ask for it.
+    const auto most_bytes = [&] {
+        size_t most = 0;
+        for (int p = 0; p < parts; ++p)
+            most = std::max(most, res_smem_bytes(real, T, rows_of[p], out.part_info[(size_t)kResPartInts * p + 3],
+                                                 out.smem_slots(), out.tmem, out.cluster, out.max_halo));
+        return most;
+    };
+    const int batch = res_tmem_batch(real), in_regs = res_reg_slots(real, T, out.rpt);
+    const int fit = std::min(res_tmem_slots(real, T), (std::max(0, out.slots - in_regs) + batch - 1) / batch * batch);
+    if (cut.pairs) out.tmem = fit;
+    out.smem_bytes = most_bytes();
+    if (out.smem_bytes > kResSmemLimit && real == 8 && cut.cluster == 0 && T <= 256) {
+        out.tmem = fit;
+        out.smem_bytes = most_bytes();
+    }
+    if (out.tmem > 0) out.smem_bytes = std::max(out.smem_bytes, kResAloneBytes);
     if (out.smem_bytes > kResSmemLimit) return "a part's rows exceed on-chip memory";
     if ((size_t)out.slots * parts * T > 0x7fffffffull) return "too many slots";
     // 5. slots
@@ -225,7 +245,9 @@ std::string build_cut(int n, const int* row_start, const int* col, const int* lt
                 row.push_back({win[lt_row[e]], static_cast<unsigned>(lt_block[e]) | kSlabLowerBit});
             std::sort(row.begin(), row.end(), [](const Entry& a, const Entry& b) { return a.win < b.win; });
             for (size_t j = 0; j < row.size(); ++j) {
-                const size_t at = ((size_t)pi[4] + j / out.lpr) * T + (size_t)i * out.lpr + j % out.lpr;
+                const size_t at = out.rpt == 1
+                                      ? ((size_t)pi[4] + j / out.lpr) * T + (size_t)i * out.lpr + j % out.lpr
+                                      : ((size_t)pi[4] + 2 * j + i / T) * T + i % T;
                 out.src[at] = row[j].src;
                 out.col[at] = static_cast<unsigned short>(3 * row[j].win);
             }
@@ -274,12 +296,12 @@ std::string build_res_plan(int n, const int* row_start, const int* col, const in
     const int max_blocks = std::min(limits.blocks, kResMaxParts);
     std::vector<int> group(nseg), place;
     std::vector<int> pers;
-    for (int per = 16; per <= kResMaxThreads; per += per < 64 ? 4 : 8) pers.push_back(per);
+    for (int per = 16; per <= 2 * kResPairThreads; per += per < 64 ? 4 : 8) pers.push_back(per);
     for (int q = 0; q < 5; ++q) {
         const int c = 1 << q;
         if (limits.clusters[q] <= 0) continue;
         for (const int per : pers) {
-            if (parts_of(largest, per) > c) continue;
+            if (parts_of(largest, per) > c || per > kResMaxThreads) continue;
             if (c > 1 && parts_of(largest, per) <= c / 2) break;  // a smaller cluster does it
             for (int b = 0; b < nseg; ++b) group[b] = parts_of(seg[b + 1] - seg[b], per);
             const int waves = (pack(group, c, place) + limits.clusters[q] - 1) / limits.clusters[q];
@@ -288,7 +310,7 @@ std::string build_res_plan(int n, const int* row_start, const int* col, const in
             cuts.push_back(
                 {per, c, cap, waves * (block_cycles(rows, real, lanes_for(rows, cap).lpr) + exchange_cycles(c, true))});
             const Lanes l = lanes_for(rows, 128);
-            const int slots = std::max(0, (longest + l.lpr - 1) / l.lpr - res_reg_slots(real, l.threads));
+            const int slots = std::max(0, (longest + l.lpr - 1) / l.lpr - res_reg_slots(real, l.threads, 1));
             if (waves > 1 && l.threads == 128 && slots * 128 * (9 * real + 2) < 80 * 1024)
                 cuts.push_back({per, c, 128,
                                 (waves + 1) / 2 * 1.4 * (block_cycles(rows, real, l.lpr) + exchange_cycles(c, true))});
@@ -300,18 +322,26 @@ std::string build_res_plan(int n, const int* row_start, const int* col, const in
         if (total > max_blocks) continue;
         const int k = parts_of(largest, per);
         const int rows = std::min(largest, per);
+        // More rows than 256 threads: two a thread in FP32 (16 warps pay the exchange and the
+        // sums more than 10 pay a second row).
+        const bool pairs = real == 4 && rows > 256;
+        if (!pairs && rows > kResMaxThreads) continue;
         const int cap = rows > 256 ? 512 : 256;
-        cuts.push_back(
-            {per, 0, cap, block_cycles(rows, real, lanes_for(rows, cap).lpr) + exchange_cycles(k, false)});
+        cuts.push_back({per, 0, cap,
+                        block_cycles(rows, real, pairs ? 1 : lanes_for(rows, cap).lpr) + exchange_cycles(k, false),
+                        pairs});
     }
     if (cuts.empty()) return "more rows than the blocks hold";
     std::stable_sort(cuts.begin(), cuts.end(), [](const Cut& a, const Cut& b) { return a.cycles < b.cycles; });
     std::string why;
     for (const Cut& c : cuts) {
-        // shared memory of the values alone, before a layout is built
+        // memory of the values alone, before a layout is built
         const double rows = std::min<double>(c.per, largest);
-        if (rows * longest * (9 * real + 2) - 512.0 * res_reg_slots(real, 512) * 9 * real > 1.0 * kResSmemLimit)
-            continue;
+        const int T = c.pairs ? std::max(kResMinThreads, ((int)rows + 63) / 64 * 32) : lanes_for((int)rows, c.cap).threads;
+        const double off_smem = 9.0 * real * T *
+                                (res_reg_slots(real, T, c.pairs ? 2 : 1) +
+                                 (c.pairs || (real == 8 && c.cluster == 0 && T <= 256) ? res_tmem_slots(real, T) : 0));
+        if (rows * longest * (9 * real + 2) - off_smem > 1.0 * kResSmemLimit) continue;
         why = build_cut(n, row_start, col, lt_start, lt_row, lt_block, coords, seg, nseg, len, c, max_blocks, real, out);
         if (why.empty()) return why;
     }
@@ -326,7 +356,13 @@ std::string res_check(const ResPlan& plan, int nnz, const ResLimits& limits, int
         return "bad part count";
     if (plan.lpr != 1 && plan.lpr != 2 && plan.lpr != 4 && plan.lpr != 8) return "bad lanes per row";
     const int T = plan.threads;
-    if (T < kResMinThreads || T > kResMaxThreads || T % 32 != 0) return "bad threads";
+    if (T < kResMinThreads || T > (plan.rpt == 2 ? kResPairThreads : kResMaxThreads) || T % 32 != 0)
+        return "bad threads";
+    if (plan.rpt != 1 && (plan.rpt != 2 || plan.lpr != 1 || plan.cluster != 0 || real != 4)) return "bad rows per thread";
+    if (plan.slots % plan.rpt != 0) return "bad slots";
+    if (plan.tmem < 0 || plan.tmem % res_tmem_batch(real) != 0 || plan.tmem > res_tmem_slots(real, T) ||
+        (plan.tmem > 0 && (plan.smem_bytes < kResAloneBytes || plan.cluster != 0)))
+        return "bad tensor memory";
     if (plan.smem_bytes > kResSmemLimit) return "too much shared memory";
     const size_t slot_count = plan.src.size() / T;
     if (plan.send.size() != 2 * plan.halo_src.size()) return "bad send lists";
@@ -334,7 +370,7 @@ std::string res_check(const ResPlan& plan, int nnz, const ResLimits& limits, int
     std::vector<unsigned char> owned(plan.n, 0), seen(nnz, 0);
     for (int p = 0; p < plan.parts; ++p) {
         const int* pi = plan.part_info.data() + (size_t)kResPartInts * p;
-        if (pi[1] < (pi[7] > 0 ? 1 : 0) || pi[0] < 0 || pi[0] + pi[1] > plan.n || pi[1] * plan.lpr > T)
+        if (pi[1] < (pi[7] > 0 ? 1 : 0) || pi[0] < 0 || pi[0] + pi[1] > plan.n || pi[1] * plan.lpr > T * plan.rpt)
             return "bad rows";
         if (pi[7] == 0 && pi[1] != 0) return "rows without a group";
         for (int g = pi[0]; g < pi[0] + pi[1]; ++g) {
@@ -351,7 +387,7 @@ std::string res_check(const ResPlan& plan, int nnz, const ResLimits& limits, int
             return "bad halo";
         if (pi[4] < 0 || (size_t)pi[4] + plan.slots > slot_count) return "bad slots";
         if (pi[9] < 0 || pi[10] < 0 || (size_t)pi[9] + pi[10] > plan.halo_src.size()) return "bad sends";
-        if (res_smem_bytes(real, T, m, h, plan.slots, plan.cluster, plan.max_halo) > plan.smem_bytes) return "bad size";
+        if (res_smem_bytes(real, T, m, h, plan.smem_slots(), plan.tmem, plan.cluster, plan.max_halo) > plan.smem_bytes) return "bad size";
         if (pi[7] > plan.max_group || pi[6] < 0 || p < pi[6] || p >= pi[6] + pi[7] || pi[6] + pi[7] > plan.parts)
             return "bad group";
         if (plan.cluster > 0 && pi[6] / plan.cluster != (pi[6] + pi[7] - 1) / plan.cluster)
@@ -400,13 +436,15 @@ void res_spmv_host(const ResPlan& plan, const double* values, const double* x, d
         for (int i = 0; i < m; ++i)
             for (int a = 0; a < 3; ++a) y[3 * (size_t)plan.perm[pi[0] + i] + a] = 0.0;
         for (int k = 0; k < plan.slots; ++k)
-            for (int t = 0; t < m * plan.lpr; ++t) {
+            for (int t = 0; t < plan.threads; ++t) {
+                const int row = plan.rpt == 1 ? t / plan.lpr : t + k % 2 * plan.threads;
+                if (row >= m) continue;
                 const size_t at = ((size_t)pi[4] + k) * plan.threads + t;
                 const unsigned s = plan.src[at];
                 if (s == kSlabNoPos) continue;
                 const double* v = values + 9 * (size_t)(s & ~kSlabLowerBit);
                 const double* d = win.data() + plan.col[at];
-                double* out = y + 3 * (size_t)plan.perm[pi[0] + t / plan.lpr];
+                double* out = y + 3 * (size_t)plan.perm[pi[0] + row];
                 for (int a = 0; a < 3; ++a)
                     for (int c = 0; c < 3; ++c) out[a] += v[(s & kSlabLowerBit) ? 3 * a + c : 3 * c + a] * d[c];
             }

@@ -9,7 +9,10 @@
 // solves; a body's parts are consecutive blocks: a group).  `lpr` lanes share a row, one
 // pass of the block covers the part.  The full symmetric row (upper blocks and transposes
 // of the lower ones, by ascending window column) is dealt round-robin to the row's lanes:
-// lane l holds entries l, l + lpr, ...  A slot is one entry per thread: src[slot][thread]
+// lane l holds entries l, l + lpr, ...  A part of more rows than a block has threads to
+// spare gives a thread two rows, t and t + threads, whose entries alternate in its slots.
+// Slots live in registers first, then in tensor memory where the launch uses it, then in
+// shared memory.  A slot is one entry per thread: src[slot][thread]
 // the canonical upper block (kSlabLowerBit: its transpose; kSlabNoPos: none, a zero block)
 // and col[slot][thread] three times the window index of its column.
 //
@@ -31,6 +34,7 @@
 namespace pk {
 
 constexpr int kResMaxThreads = 512, kResMinThreads = 128;
+constexpr int kResPairThreads = 320;  // threads of a block with two rows a thread
 constexpr int kResHaloPerThread = 2;
 constexpr int kResMaxParts = 160;   // blocks of a group exchanging through global memory
 constexpr int kResSlotPoll = kResMaxParts / 32;
@@ -38,31 +42,51 @@ constexpr int kResMaxCluster = 16;
 // Per part: row0, rows, halo0, halo rows, slot0, (unused), first block and size of its group
 // (size 0: the block has no part), body, first and number of its sends.
 constexpr int kResPartInts = 12;
+constexpr size_t kResAloneBytes = 116 * 1024;  // more than half an SM's: no second block beside this one
 constexpr size_t kResSmemLimit = 224 * 1024;  // dynamic shared memory of one block per SM
 
-// Slots that stay in registers: what the register file leaves beside a row's vectors at
-// 128 registers a thread (512 threads) or 255 (up to 256 threads).
-constexpr int res_reg_slots(int real, int threads)
+// Slots that stay in registers: what the register file leaves beside the rows' vectors at
+// 128 registers a thread (512 threads), 204 (two rows a thread) or 255 (up to 256 threads).
+constexpr int res_reg_slots(int real, int threads, int rpt)
 {
+    if (rpt > 1) return 2;
     return threads <= 256 ? (real == 4 ? 8 : 4) : (real == 4 ? 4 : 0);
+}
+// Tensor memory: 512 columns of one word for the warps of a quarter of the lanes (every
+// fourth warp), read in batches of 36 words a thread: four FP32 slots or two FP64 slots.
+constexpr int kResTmemWords = 36;
+constexpr int res_tmem_batch(int real) { return kResTmemWords / (9 * real / 4); }
+constexpr int res_tmem_columns(int threads) { return 512 / ((threads / 32 + 3) / 4); }
+constexpr int res_tmem_slots(int real, int threads)
+{
+    return res_tmem_columns(threads) / kResTmemWords * res_tmem_batch(real);
 }
 constexpr size_t res_align(size_t v) { return (v + 15) & ~(size_t)15; }
 constexpr size_t res_row_packet(int real) { return real == 4 ? 16 : 32; }
 
 // Bytes of dynamic shared memory of a part: inbox (clusters: two buffers of sums and of the
-// launch's most halo rows), window, halo r and M^-1, q, values, columns.
-constexpr size_t res_smem_bytes(int real, int threads, int m, int h, int slots, int cluster, int max_halo)
+// launch's most halo rows), window, halo r and M^-1, q, values of in_smem slots, columns of those
+// and of the tensor memory's.
+constexpr size_t res_smem_bytes(int real, int threads, int m, int h, int in_smem, int tmem, int cluster,
+                                int max_halo)
 {
-    const int in_smem = slots > res_reg_slots(real, threads) ? slots - res_reg_slots(real, threads) : 0;
     const size_t inbox = cluster > 0 ? 2 * (size_t)kResMaxCluster * 64 + 2 * (size_t)max_halo * res_row_packet(real) : 0;
     return inbox + res_align(3 * (size_t)(m + h) * real) + res_align(12 * (size_t)h * real) +
            res_align(3 * (size_t)m * real) + res_align((size_t)in_smem * threads * 9 * real) +
-           res_align((size_t)in_smem * threads * 2);
+           res_align((size_t)(in_smem + tmem) * threads * 2);
 }
 
 struct ResPlan {
     int n = 0, parts = 0;         // parts: blocks of the launch, those without rows included
     int lpr = 4, threads = 128, slots = 0, cluster = 0;
+    int rpt = 1;                  // rows per thread: 1 (lpr lanes a row) or 2 (one lane a row)
+    int tmem = 0;                 // slots in tensor memory, after those in registers
+    int smem_slots() const
+    {
+        const int rest = slots - tmem - res_reg_slots(real, threads, rpt);
+        return rest > 0 ? rest : 0;
+    }
+    int real = 4;
     std::vector<int> perm;        // part order -> dynamic row
     std::vector<int> part_info;   // kResPartInts per part
     std::vector<int> halo_src;    // part-order index of every halo row, part by part

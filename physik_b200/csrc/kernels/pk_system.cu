@@ -688,6 +688,8 @@ int ensure_resident(pk_system* s, bool bodies)
     s->res_plan.lpr = plan.lpr;
     s->res_plan.threads = plan.threads;
     s->res_plan.slots = plan.slots;
+    s->res_plan.rpt = plan.rpt;
+    s->res_plan.tmem = plan.tmem;
     s->res_plan.cluster = plan.cluster;
     s->res_plan.max_group = plan.max_group;
     s->res_plan.max_halo = plan.max_halo;
@@ -962,6 +964,7 @@ int run_pcg_resident(pk_system* s, const pk_step_params& p, int skip_on_flags)
     a.col = s->res_col.as<unsigned short>();
     a.lpr = s->res_plan.lpr;
     a.nslots = s->res_plan.slots;
+    a.tmem_slots = s->res_plan.tmem;
     a.max_halo = s->res_plan.max_halo;
     a.slot_count = s->res_plan.slots * s->res_parts;
     a.nnz = s->nnz;
@@ -988,7 +991,7 @@ int run_pcg_resident(pk_system* s, const pk_step_params& p, int skip_on_flags)
     a.nbodies = bodies ? static_cast<int>(s->seg_start.size()) - 1 : 1;
     a.body_stats = bodies ? s->body_stats.as<pk::BatchBodyStats>() : nullptr;
     a.missing = &st->batch_missing;
-    PK_CHECK(pk::launch_pcg_res_kernel<Real>(a, s->res_plan.threads, s->res_plan.cluster, s->res_parts, s->stream));
+    PK_CHECK(pk::launch_pcg_res_kernel<Real>(a, s->res_plan.threads, s->res_plan.rpt, s->res_plan.cluster, s->res_parts, s->stream));
     s->launches += 1;
     s->last_blocks = s->res_parts;
     return PK_OK;
@@ -2911,7 +2914,7 @@ PKCUDA_API int pk_res_plan_selfcheck(int n, const int* row_start, const int* col
         info[2] = plan.lpr;
         info[3] = static_cast<int>(plan.smem_bytes);
         info[4] = plan.cluster;
-        info[5] = plan.threads;
+        info[5] = plan.threads * plan.rpt;
     }
     return PK_OK;
 }
