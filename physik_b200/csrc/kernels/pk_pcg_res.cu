@@ -37,7 +37,7 @@
 // Measured per CG iteration against the streaming kernels (part-resident stream for FP32
 // storage, ring for FP64): 8x8x8 box FP32 1.8 us (7.2), 32x8x8 beam FP64 3.0 us (13.3),
 // 64x16x16 beam 3.3 us mixed (10.9) and 4.2 us FP64 (18.5), 61x47x29 block mixed (594 rows a
-// part) 6.7 us (19.3).  What is left is a chain of
+// part) 7.0 us (19.3).  What is left is a chain of
 // latencies: about 3,000 cycles of a block's own work (product, two sets of FP64 sums by
 // shuffles, the scalars, the updates; 8.6 cycles an FP64 add, 24 a shuffle, 45 a barrier of
 // 512 threads) and the exchange.
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
     constexpr int KR = res_reg_slots(sizeof(Real), MAXT, R);
     constexpr int KB = res_tmem_batch(sizeof(Real));
     static_assert(KR % R == 0 && KB % R == 0, "a slot's row is known at compile time");
-    constexpr int NH = kResHaloPerThread;
+    constexpr int NH = res_halo_per_thread(R);
     constexpr int RB = (int)res_row_packet(sizeof(Real));
     extern __shared__ __align__(128) unsigned char dyn[];
     // the owner warps' partials and the group's sums, by exchange parity

@@ -186,7 +186,7 @@ std::string build_cut(int n, const int* row_start, const int* col, const int* lt
         for (const int g : halo)
             if (gsize[p] <= 1 || gfirst[part_of[out.perm[g]]] != gfirst[p]) return "a block couples two bodies";
         const int m = rows_of[p], h = static_cast<int>(halo.size());
-        if (h > kResHaloPerThread * T) return "a part's halo exceeds its threads";
+        if (h > res_halo_per_thread(out.rpt) * T) return "a part's halo exceeds its threads";
         if (3 * (m + h) > 65535) return "a part's window exceeds its column index";
         pi[0] = start[p];
         pi[1] = m;
@@ -382,7 +382,7 @@ std::string res_check(const ResPlan& plan, int nnz, const ResLimits& limits, int
         const int* pi = plan.part_info.data() + (size_t)kResPartInts * p;
         const int m = pi[1], h = pi[3];
         if (pi[7] == 0) continue;
-        if (h < 0 || h > kResHaloPerThread * T || h > plan.max_halo || pi[2] < 0 ||
+        if (h < 0 || h > res_halo_per_thread(plan.rpt) * T || h > plan.max_halo || pi[2] < 0 ||
             (size_t)pi[2] + h > plan.halo_src.size())
             return "bad halo";
         if (pi[4] < 0 || (size_t)pi[4] + plan.slots > slot_count) return "bad slots";
