@@ -65,9 +65,6 @@ __device__ __forceinline__ V3<Real> row_spmv(const BsrView<Real>& A, int r, int 
     return acc;
 }
 
-// ------------------------------------------------------------------ tet records
-// A record of kTetRec values moved with 16-byte accesses (it starts on a 16-byte boundary);
-// the tet kernel stores its first 18 values (R, S) each step.
 // ------------------------------------------------------------------ element stiffness block
 // K_ab = V (lambda P_a P_b^T + mu P_b P_a^T + mu (g_a.g_b) R R^T), P = R g, written with
 // explicit roundings (products and fused multiply-adds in one fixed order) so that every

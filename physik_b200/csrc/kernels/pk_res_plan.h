@@ -47,7 +47,7 @@ constexpr size_t kResAloneBytes = 116 * 1024;  // more than half an SM's: no sec
 constexpr size_t kResSmemLimit = 224 * 1024;  // dynamic shared memory of one block per SM
 
 // Slots that stay in registers: what the register file leaves beside the rows' vectors at
-// 128 registers a thread (512 threads), 204 (two rows a thread) or 255 (up to 256 threads).
+// 128 registers a thread (512 threads), 168 (two rows a thread) or 255 (up to 256 threads).
 constexpr int res_reg_slots(int real, int threads, int rpt)
 {
     if (rpt > 1) return 2;

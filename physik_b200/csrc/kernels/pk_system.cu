@@ -991,7 +991,8 @@ int run_pcg_resident(pk_system* s, const pk_step_params& p, int skip_on_flags)
     a.nbodies = bodies ? static_cast<int>(s->seg_start.size()) - 1 : 1;
     a.body_stats = bodies ? s->body_stats.as<pk::BatchBodyStats>() : nullptr;
     a.missing = &st->batch_missing;
-    PK_CHECK(pk::launch_pcg_res_kernel<Real>(a, s->res_plan.threads, s->res_plan.rpt, s->res_plan.cluster, s->res_parts, s->stream));
+    PK_CHECK(pk::launch_pcg_res_kernel<Real>(a, s->res_plan.threads, s->res_plan.rpt, s->res_plan.cluster, s->res_parts,
+                                             s->stream));
     s->launches += 1;
     s->last_blocks = s->res_parts;
     return PK_OK;
