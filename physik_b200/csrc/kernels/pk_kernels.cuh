@@ -414,6 +414,59 @@ struct SlabPcgArgs {
     int sym;
 };
 
+// ------------------------------------------------------------------ part-resident PCG, FP64
+// pk_pcg_slab64.cu: the window (24 bytes a row), a ring of as many stages as fit, the table.
+constexpr size_t kSlab64SmemLimit = 224 * 1024;
+constexpr int kSlab64MaxStages = 9;
+constexpr size_t slab64_ring_offset(int window) { return (24 * size_t(window) + 127) / 128 * 128; }
+constexpr int slab64_stages(int window)
+{
+    const size_t fixed = slab64_ring_offset(window) + 16 * size_t(kSlab64MaxTiles);
+    const size_t fit = fixed < kSlab64SmemLimit ? (kSlab64SmemLimit - fixed) / kSlab64StageBytes : 0;
+    return fit < size_t(kSlab64MaxStages) ? int(fit) : kSlab64MaxStages;
+}
+static_assert(slab64_stages(kSlabWinCap) >= 4, "the largest window must leave a ring");
+struct Slab64PcgArgs {
+    int n;                       // dynamic rows
+    const int* part_info;        // [grid] x kSlabPartInts
+    const int* send_start;       // [grid + 1]
+    const int2* send;            // {row of the part, halo row}
+    const int4* tile_desc;
+    int tile_count, halo_count;
+    const unsigned char* stream;
+    unsigned long long stream_bytes;
+    int stages, win_cap;
+    unsigned ring_offset;
+    unsigned char* rows_in;      // two packets per halo row; zero at launch
+    unsigned char* sums_in;      // the blocks' inboxes; zero at launch
+    const int* perm;             // slab index -> dynamic row
+    const double* b;             // per dynamic row
+    const double* minv;
+    double* x;                   // per dynamic row: delta-v out
+    double* qs;                  // 4 per slab row
+    double* mrow;                // M^-1 in slab order, [9][n]
+    int max_iterations;
+    double tolerance;
+    int skip_on_flags, integrate;
+    double dt;
+    const int* dyn_to_node;
+    double* node_x;
+    double* node_v;
+    unsigned* flags;
+    DevStats* stats;
+};
+struct Slab64FillArgs {
+    const double* values;        // the assembled blocks
+    int nnz;
+    const int4* tile_desc;
+    const int* tile_entry0;
+    int tile_count, entries;
+    const unsigned* fill_src;
+    const unsigned char* layout; // headers and columns (SlabPlan::stream): written instead of the blocks
+    unsigned char* stream;
+    unsigned long long stream_bytes;
+};
+
 // ------------------------------------------------------------------ resident PCG
 // The resident PCG kernel (pk_pcg_res.cu; layout in pk_res_plan.h): one block per part,
 // the part's rows on chip for the whole solve, one exchange per iteration.
@@ -569,6 +622,10 @@ struct AdjointArgs {
 // Launchers (pk_kernels.cu).  All asynchronous on `stream`.
 template <class Real>
 cudaError_t launch_tet_kernel(const AssemblyArgs<Real>& args, bool fp64_polar_fallback, cudaStream_t stream);
+// Part-resident PCG in FP64 (pk_pcg_slab64.cu), cooperative, a block per part.
+int pcg_slab64_max_grid();
+cudaError_t launch_pcg_slab64_kernel(const Slab64PcgArgs& args, int grid, cudaStream_t stream);
+cudaError_t launch_slab64_fill_kernel(const Slab64FillArgs& args, cudaStream_t stream);
 // TetView::rest, when the tets are set.
 template <class Real>
 cudaError_t launch_tet_pack(const Real* dm_inv, const Real* params, Real* rest, int tet_count, cudaStream_t stream);

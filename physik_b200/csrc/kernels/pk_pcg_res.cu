@@ -55,6 +55,7 @@
 #include <type_traits>
 
 #include "pk_device.cuh"
+#include "pk_exchange.cuh"
 
 namespace pk {
 namespace {
@@ -63,94 +64,6 @@ constexpr int kResMaxWarps = kResMaxThreads / 32;
 constexpr int kResSums = 4;  // d.q, q.s + r.z, q.z, r.s; at the end r.r in the first
 constexpr int kResSendRegs = 2;
 constexpr unsigned kResSpinLimit = 1u << 22;  // polls of one wait: seconds
-
-struct Packet {
-    unsigned long long lo, hi;
-};
-__device__ __forceinline__ void st_packet(void* p, Packet v)
-{
-    asm volatile(
-        "{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p), "l"(v.lo),
-        "l"(v.hi)
-        : "memory");
-}
-__device__ __forceinline__ Packet ld_packet(const void* p)
-{
-    Packet v;
-    asm volatile(
-        "{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
-        : "=l"(v.lo), "=l"(v.hi)
-        : "l"(p)
-        : "memory");
-    return v;
-}
-__device__ __forceinline__ unsigned packet_tag(Packet v) { return (unsigned)(v.hi >> 32); }
-
-// A row of q with its tag: one packet in FP32; two in FP64 (96 bits of data and a tag each).
-__device__ __forceinline__ void st_row(unsigned char* p, V3<float> q, unsigned tag)
-{
-    st_packet(p, {(unsigned long long)__float_as_uint(q.x) | ((unsigned long long)__float_as_uint(q.y) << 32),
-                  (unsigned long long)__float_as_uint(q.z) | ((unsigned long long)tag << 32)});
-}
-__device__ __forceinline__ void st_row(unsigned char* p, V3<double> q, unsigned tag)
-{
-    const unsigned long long x = __double_as_longlong(q.x), y = __double_as_longlong(q.y),
-                             z = __double_as_longlong(q.z), t = (unsigned long long)tag << 32;
-    st_packet(p, {x, (y & 0xffffffffull) | t});
-    st_packet(p + 16, {(y >> 32) | (z << 32), (z >> 32) | t});
-}
-__device__ __forceinline__ bool ld_row(const unsigned char* p, unsigned tag, V3<float>& q)
-{
-    const Packet a = ld_packet(p);
-    q = V3<float>{__uint_as_float((unsigned)a.lo), __uint_as_float((unsigned)(a.lo >> 32)),
-                  __uint_as_float((unsigned)a.hi)};
-    return packet_tag(a) == tag;
-}
-__device__ __forceinline__ bool ld_row(const unsigned char* p, unsigned tag, V3<double>& q)
-{
-    const Packet a = ld_packet(p), b = ld_packet(p + 16);
-    q = V3<double>{__longlong_as_double((long long)a.lo),
-                   __longlong_as_double((long long)((a.hi & 0xffffffffull) | (b.lo << 32))),
-                   __longlong_as_double((long long)((b.lo >> 32) | (b.hi << 32)))};
-    return packet_tag(a) == tag && packet_tag(b) == tag;
-}
-
-// The row updates, with every rounding spelled out: owners and halo copies must agree.
-template <class Real>
-__device__ __forceinline__ V3<Real> fma3(Real a, V3<Real> b, V3<Real> c)
-{
-    return V3<Real>{fma(a, b.x, c.x), fma(a, b.y, c.y), fma(a, b.z, c.z)};
-}
-__device__ __forceinline__ V3<float> fma3(float a, V3<float> b, V3<float> c)
-{
-    return V3<float>{__fmaf_rn(a, b.x, c.x), __fmaf_rn(a, b.y, c.y), __fmaf_rn(a, b.z, c.z)};
-}
-template <class Real>
-__device__ __forceinline__ V3<Real> apply_minv(const Real (&m)[9], V3<Real> v)
-{
-    V3<Real> r{m[0] * v.x, m[1] * v.x, m[2] * v.x};
-    r = V3<Real>{fma(m[3], v.y, r.x), fma(m[4], v.y, r.y), fma(m[5], v.y, r.z)};
-    return V3<Real>{fma(m[6], v.z, r.x), fma(m[7], v.z, r.y), fma(m[8], v.z, r.z)};
-}
-// c + a b with the FP64 scalar a: in FP32 a is split into two floats (see SplitAlpha in
-// pk_pcg_slab.cu: within an ulp of the FP64 update, without conversions).
-template <class Real>
-struct Scale;
-template <>
-struct Scale<float> {
-    float hi, lo;
-    __device__ __forceinline__ explicit Scale(double a) : hi(float(a)), lo(float(a - double(float(a)))) {}
-    __device__ __forceinline__ Scale(float h, float l) : hi(h), lo(l) {}
-    __device__ __forceinline__ Scale negated() const { return Scale(-hi, -lo); }
-    __device__ __forceinline__ V3<float> axpy(V3<float> b, V3<float> c) const { return fma3(lo, b, fma3(hi, b, c)); }
-};
-template <>
-struct Scale<double> {
-    double a;
-    __device__ __forceinline__ explicit Scale(double v) : a(v) {}
-    __device__ __forceinline__ Scale negated() const { return Scale(-a); }
-    __device__ __forceinline__ V3<double> axpy(V3<double> b, V3<double> c) const { return fma3(a, b, c); }
-};
 
 // ------------------------------------------------------------------ cluster exchange
 __device__ __forceinline__ unsigned cluster_map(const void* p, unsigned rank)

@@ -142,7 +142,7 @@ namespace {
 // once (and its transpose once, off the diagonal).
 std::string build_layout(int n, const int* row_start, const int* col, const int* lt_start, const int* lt_row,
                          const int* lt_block, const std::vector<int>& part_of, const std::vector<int>& len, int parts,
-                         SlabPlan& out)
+                         SlabPlan& out, bool wide)
 {
     const int nnz = row_start[n];
     // slab order: parts in order; inside a part the interior rows (every block's column in
@@ -181,6 +181,8 @@ std::string build_layout(int n, const int* row_start, const int* col, const int*
 
     // Pass 1: tiles of consecutive owned rows, at most kSlabRows rows and kSlabCapE
     // entries (padded to a multiple of 8 so the arrays stay 16-byte aligned).
+    const int tile_rows = wide ? kSlab64Rows : kSlabRows, cap = wide ? kSlab64CapE : kSlabCapE;
+    const int entry_bytes = wide ? kSlab64EntryBytes : kSlabEntryBytes;
     std::vector<int> part_tile0(parts + 1, 0);
     size_t stream_bytes = 0, entries = 0;
     for (int p = 0; p < parts; ++p) {
@@ -190,15 +192,15 @@ std::string build_layout(int n, const int* row_start, const int* col, const int*
         int a = 0;
         while (a < m) {
             int b = a, e = 0;
-            while (b < m && b - a < kSlabRows) {
+            while (b < m && b - a < tile_rows) {
                 const int e2 = e + len[out.perm[g0 + b]];
-                if (((e2 + 7) & ~7) > kSlabCapE) break;
+                if (((e2 + 7) & ~7) > cap) break;
                 e = e2;
                 ++b;
             }
             if (b == a) return "a row has more blocks than a tile holds";
             const int ne = (e + 7) & ~7;
-            const size_t bytes = (size_t)kSlabHeaderBytes + (size_t)kSlabEntryBytes * ne;
+            const size_t bytes = (size_t)kSlabHeaderBytes + (size_t)entry_bytes * ne;
             if (stream_bytes / 16 > 0x7fffffffULL || (stream_bytes + bytes) / 4 >= 0xffffffffULL)
                 return "stream too large";
             out.tile_desc.insert(out.tile_desc.end(),
@@ -209,12 +211,14 @@ std::string build_layout(int n, const int* row_start, const int* col, const int*
             if (entries > 0x7fffffffu) return "stream too large";
             a = b;
         }
-        if (static_cast<int>(out.tile_desc.size() / 4) - part_tile0[p] > kSlabMaxTiles)
+        if (static_cast<int>(out.tile_desc.size() / 4) - part_tile0[p] > (wide ? kSlab64MaxTiles : kSlabMaxTiles))
             return "a part has more tiles than the table holds";
     }
     part_tile0[parts] = static_cast<int>(out.tile_desc.size() / 4);
     out.tile_entry0.push_back(static_cast<int>(entries));
-    out.stream.assign(stream_bytes, 0);
+    out.wide = wide;
+    out.stream_bytes = stream_bytes;
+    out.stream.assign(wide ? (size_t)kSlabHeaderBytes * part_tile0[parts] + 2 * entries : stream_bytes, 0);
     out.fill_src.assign(entries, kSlabNoPos);
 
     // Pass 2: per part, its halo (rows of other parts its rows couple to, ascending slab
@@ -254,11 +258,11 @@ std::string build_layout(int n, const int* row_start, const int* col, const int*
         std::vector<Entry> row_entries;
         for (int ti = part_tile0[p]; ti < part_tile0[p + 1]; ++ti) {
             const int* d = out.tile_desc.data() + 4 * (size_t)ti;
-            const size_t off = 16 * (size_t)d[0];
+            const size_t off = wide ? (size_t)kSlabHeaderBytes * ti + 2 * (size_t)out.tile_entry0[ti] : 16 * (size_t)d[0];
             const int a = d[2], b = d[2] + d[3];
             const int ne = out.tile_entry0[ti + 1] - out.tile_entry0[ti];
             const size_t vals_off = off + kSlabHeaderBytes;
-            const size_t col_off = vals_off + 36 * (size_t)ne;
+            const size_t col_off = wide ? vals_off : vals_off + 36 * (size_t)ne;
             unsigned* src = out.fill_src.data() + out.tile_entry0[ti];
             int j = 0;
             for (int i = a; i < b; ++i) {
@@ -727,23 +731,43 @@ std::string build_layout_sym(int n, const int* row_start, const int* col, const 
 int plan_thread_count() { return plan_threads(); }
 void for_items(int count, const std::function<void(int, int)>& f) { parallel_items(count, f); }
 
+// Who sends which row where.
+void add_sends(SlabPlan& plan)
+{
+    std::vector<int> part_of(plan.n);
+    for (int p = 0; p < plan.parts; ++p) {
+        const int* pi = plan.part_info.data() + (size_t)kSlabPartInts * p;
+        std::fill(part_of.begin() + pi[0], part_of.begin() + pi[0] + pi[1], p);
+    }
+    plan.send_start.assign(plan.parts + 1, 0);
+    for (const int g : plan.halo_src) ++plan.send_start[part_of[g] + 1];
+    for (int p = 0; p < plan.parts; ++p) plan.send_start[p + 1] += plan.send_start[p];
+    plan.send.assign(2 * plan.halo_src.size(), 0);
+    std::vector<int> at(plan.send_start.begin(), plan.send_start.end() - 1);
+    for (size_t i = 0; i < plan.halo_src.size(); ++i) {
+        const int g = plan.halo_src[i], q = part_of[g], e = at[q]++;
+        plan.send[2 * (size_t)e] = g - plan.part_info[(size_t)kSlabPartInts * q];
+        plan.send[2 * (size_t)e + 1] = static_cast<int>(i);
+    }
+}
+
 // The symmetric form where the caller allows it and it applies, else the full rows.
 std::string build_layout_form(int n, const int* row_start, const int* col, const int* lt_start, const int* lt_row,
                               const int* lt_block, const double* coords, const std::vector<int>& part_of,
                               const std::vector<int>& len, const std::vector<double>& w, int parts, int form,
-                              SlabPlan& out)
+                              SlabPlan& out, bool wide = false)
 {
-    if (form != kSlabFull) {
+    if (form != kSlabFull && !wide) {
         const std::string why =
             build_layout_sym(n, row_start, col, lt_start, lt_row, lt_block, coords, part_of, w, parts, out);
         if (why.empty() || form == kSlabSym) return why;
         out = SlabPlan{};
     }
-    return build_layout(n, row_start, col, lt_start, lt_row, lt_block, part_of, len, parts, out);
+    return build_layout(n, row_start, col, lt_start, lt_row, lt_block, part_of, len, parts, out, wide);
 }
 
 std::string build_slab_plan(int n, const int* row_start, const int* col, const int* lt_start, const int* lt_row,
-                            const int* lt_block, const double* coords, int parts, SlabPlan& out, int form)
+                            const int* lt_block, const double* coords, int parts, SlabPlan& out, int form, bool wide)
 {
     out = SlabPlan{};
     if (n <= 0 || parts <= 0) return "empty system";
@@ -751,7 +775,7 @@ std::string build_slab_plan(int n, const int* row_start, const int* col, const i
     std::vector<int> len(n);
     for (int r = 0; r < n; ++r) len[r] = (row_start[r + 1] - row_start[r]) + (lt_start[r + 1] - lt_start[r]);
     for (int r = 0; r < n; ++r)
-        if (len[r] > kSlabCapE) return "a row has more blocks than a tile holds";
+        if (len[r] > (wide ? kSlab64CapE : kSlabCapE)) return "a row has more blocks than a tile holds";
     std::vector<int> part_of(n, 0);
     std::vector<double> w(n);
     const double extra = row_weight_extra();
@@ -769,7 +793,7 @@ std::string build_slab_plan(int n, const int* row_start, const int* col, const i
         }
     }
     const std::string why =
-        build_layout_form(n, row_start, col, lt_start, lt_row, lt_block, coords, part_of, len, w, parts, form, out);
+        build_layout_form(n, row_start, col, lt_start, lt_row, lt_block, coords, part_of, len, w, parts, form, out, wide);
     if (!why.empty()) return why;
     for (int p = 0; p < parts; ++p) {
         out.part_info[(size_t)kSlabPartInts * p + 6] = 0;
@@ -777,6 +801,7 @@ std::string build_slab_plan(int n, const int* row_start, const int* col, const i
     }
     out.part_body.assign(parts, 0);
     out.launch_start = {0, parts};
+    if (wide) add_sends(out);
     return "";
 }
 

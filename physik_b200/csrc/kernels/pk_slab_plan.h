@@ -92,6 +92,15 @@ static_assert(2 * (kSlabRows + 1) <= kSlabHeaderBytes, "header too small");
 constexpr int kSlabHaloWord = kSlabHeaderBytes / 2 - 1;
 static_assert(kSlabHaloWord >= kSlabRows + 1, "the halo word must not overlap the row offsets");
 
+// The FP64 form of the stream (pk_pcg_slab64.cu): the full rows in tiles of half as many rows,
+// eight consumer lanes a row, 74 bytes an entry.
+constexpr int kSlab64Rows = 16, kSlab64Lanes = 8;
+constexpr int kSlab64EntryBytes = 74;   // 9 doubles + u16 column
+constexpr int kSlab64CapE = 256;
+constexpr int kSlab64StageBytes = 19072;
+constexpr int kSlab64MaxTiles = 256;
+static_assert(kSlabHeaderBytes + kSlab64CapE * kSlab64EntryBytes <= kSlab64StageBytes, "stage too small");
+
 struct SlabPlan {
     int n = 0;
     int parts = 0;
@@ -105,6 +114,12 @@ struct SlabPlan {
     std::vector<int> part_body;  // body (segment) of each part; 0 for the coupled solve
     std::vector<int> launch_start;  // parts [launch_start[l], launch_start[l + 1]) form launch l
     int max_window = 0, max_tiles = 0, max_rows = 0;
+    // FP64 form: `stream` holds only the tiles' headers and columns, one after another (a tile's
+    // at kSlabHeaderBytes x tile + 2 x its first entry); the whole stream has stream_bytes.
+    // send: what each part sends, part by part from send_start, {row of the part, halo_src index}.
+    bool wide = false;
+    size_t stream_bytes = 0;
+    std::vector<int> send, send_start;
     bool sym = false;  // the symmetric form (tiles and headers as described above)
 };
 
@@ -118,7 +133,7 @@ enum SlabForm { kSlabFull = 0, kSlabSym = 1, kSlabAuto = 2 };
 // layout does not apply (a window or a row too large); `out` is then unusable.
 std::string build_slab_plan(int n, const int* row_start, const int* col, const int* lt_start, const int* lt_row,
                             const int* lt_block, const double* coords, int parts, SlabPlan& out,
-                            int form = kSlabAuto);
+                            int form = kSlabAuto, bool wide = false);
 
 // f(i, thread) for i in [0, count) on the layout builds' host threads (thread <
 // plan_thread_count()); each i must write only its own outputs.
