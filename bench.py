@@ -72,8 +72,8 @@ def measured_peaks():
 
 
 KERNEL_NAMES = {
-    "slab": "pcg_slab_kernel (cooperative, one block per part: search directions resident in shared memory, "
-            "full symmetric rows streamed by TMA, block-Jacobi, dots, integrate)",
+    "slab": "pcg_part_kernel (cooperative, one block per part: search directions resident in shared memory, "
+            "full symmetric rows streamed by TMA, block-Jacobi, one exchange per iteration, integrate)",
     "ring": "pcg_ring_kernel (cooperative: TMA-staged upper BSR rows, L2 gathers of lower blocks and records, "
             "block-Jacobi, dots, integrate)",
     "staged": "pcg_kernel (cooperative, TMA-staged tiles)",

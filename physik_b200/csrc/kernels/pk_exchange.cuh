@@ -1,5 +1,5 @@
 // pk_exchange.cuh -- exchanges between blocks by tagged packets, and the row updates that
-// owners and copies of a row share (pk_pcg_res.cu, pk_pcg_slab64.cu).
+// owners and copies of a row share (pk_pcg_res.cu, pk_pcg_part.cu).
 //
 // Every value of an exchange travels in a 16-byte packet with a tag (the exchange's number),
 // written and read whole, so that no fence orders it.

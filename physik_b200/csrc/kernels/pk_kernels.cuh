@@ -414,19 +414,24 @@ struct SlabPcgArgs {
     int sym;
 };
 
-// ------------------------------------------------------------------ part-resident PCG, FP64
-// pk_pcg_slab64.cu: the window (24 bytes a row), a ring of as many stages as fit, the table.
-constexpr size_t kSlab64SmemLimit = 224 * 1024;
-constexpr int kSlab64MaxStages = 9;
-constexpr size_t slab64_ring_offset(int window) { return (24 * size_t(window) + 127) / 128 * 128; }
-constexpr int slab64_stages(int window)
+// ------------------------------------------------------------------ part-resident PCG, coupled
+// pk_pcg_part.cu: the window, a ring of as many stages as fit, the table.
+constexpr size_t kPartSmemLimit = 224 * 1024;
+// Six: with nine the exchange's packets wait behind a longer refill (17.9 against 17.6 us an
+// iteration with 122,400 FP32 rows).
+constexpr int kPartMaxStages = 6;
+constexpr size_t part_stage(size_t real) { return real == 8 ? kWideStageBytes : kSlabStageBytes; }
+constexpr size_t part_table(size_t real) { return 16 * size_t(real == 8 ? kWideMaxTiles : kSlabMaxTiles); }
+constexpr size_t part_ring_offset(size_t real, int window) { return (3 * real * window + 127) / 128 * 128; }
+constexpr int part_stages(size_t real, int window)
 {
-    const size_t fixed = slab64_ring_offset(window) + 16 * size_t(kSlab64MaxTiles);
-    const size_t fit = fixed < kSlab64SmemLimit ? (kSlab64SmemLimit - fixed) / kSlab64StageBytes : 0;
-    return fit < size_t(kSlab64MaxStages) ? int(fit) : kSlab64MaxStages;
+    const size_t fixed = part_ring_offset(real, window) + part_table(real);
+    const size_t fit = fixed < kPartSmemLimit ? (kPartSmemLimit - fixed) / part_stage(real) : 0;
+    return fit < size_t(kPartMaxStages) ? int(fit) : kPartMaxStages;
 }
-static_assert(slab64_stages(kSlabWinCap) >= 4, "the largest window must leave a ring");
-struct Slab64PcgArgs {
+static_assert(part_stages(8, kSlabWinCap) >= 4, "the largest window must leave a ring");
+template <class Real>
+struct PartPcgArgs {
     int n;                       // dynamic rows
     const int* part_info;        // [grid] x kSlabPartInts
     const int* send_start;       // [grid + 1]
@@ -437,25 +442,25 @@ struct Slab64PcgArgs {
     unsigned long long stream_bytes;
     int stages, win_cap;
     unsigned ring_offset;
-    unsigned char* rows_in;      // two packets per halo row; zero at launch
+    unsigned char* rows_in;      // a packet (FP64: two) per halo row; zero at launch
     unsigned char* sums_in;      // the blocks' inboxes; zero at launch
     const int* perm;             // slab index -> dynamic row
-    const double* b;             // per dynamic row
-    const double* minv;
-    double* x;                   // per dynamic row: delta-v out
-    double* qs;                  // 4 per slab row
-    double* mrow;                // M^-1 in slab order, [9][n]
+    const Real* b;             // per dynamic row
+    const Real* minv;
+    Real* x;                   // per dynamic row: delta-v out
+    Real* qs;                  // 4 per slab row
+    Real* mrow;                // FP64: M^-1 in slab order, [9][n]
     int max_iterations;
     double tolerance;
     int skip_on_flags, integrate;
-    double dt;
+    Real dt;
     const int* dyn_to_node;
-    double* node_x;
-    double* node_v;
+    Real* node_x;
+    Real* node_v;
     unsigned* flags;
     DevStats* stats;
 };
-struct Slab64FillArgs {
+struct WideFillArgs {
     const double* values;        // the assembled blocks
     int nnz;
     const int4* tile_desc;
@@ -622,10 +627,12 @@ struct AdjointArgs {
 // Launchers (pk_kernels.cu).  All asynchronous on `stream`.
 template <class Real>
 cudaError_t launch_tet_kernel(const AssemblyArgs<Real>& args, bool fp64_polar_fallback, cudaStream_t stream);
-// Part-resident PCG in FP64 (pk_pcg_slab64.cu), cooperative, a block per part.
-int pcg_slab64_max_grid();
-cudaError_t launch_pcg_slab64_kernel(const Slab64PcgArgs& args, int grid, cudaStream_t stream);
-cudaError_t launch_slab64_fill_kernel(const Slab64FillArgs& args, cudaStream_t stream);
+// Coupled part-resident PCG (pk_pcg_part.cu), cooperative, a block per part.
+template <class Real>
+int pcg_part_max_grid();
+template <class Real>
+cudaError_t launch_pcg_part_kernel(const PartPcgArgs<Real>& args, int grid, cudaStream_t stream);
+cudaError_t launch_wide_fill_kernel(const WideFillArgs& args, cudaStream_t stream);
 // TetView::rest, when the tets are set.
 template <class Real>
 cudaError_t launch_tet_pack(const Real* dm_inv, const Real* params, Real* rest, int tet_count, cudaStream_t stream);

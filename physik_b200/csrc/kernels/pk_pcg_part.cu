@@ -1,22 +1,31 @@
-// pk_pcg_slab64.cu -- the part-resident cooperative block-Jacobi PCG kernel in FP64, for
-// systems whose matrix exceeds the chip (pk_pcg_res.cu) and whose parts fit its windows.
+// pk_pcg_part.cu -- the part-resident cooperative block-Jacobi PCG kernel for coupled solves
+// of systems whose matrix exceeds the chip (pk_pcg_res.cu) and whose parts fit its windows.
 //
 // The solve of the other PCG kernels (SolvePreconditionedConjugateGradient,
 // src/Core/Solvers/Linear/ConjugateGradientSolver.cpp:114-241, with the SpMV of
 // SparseBlockMatrix::Multiply, src/Math/SparseBlockMatrix.cpp:209-268, and
 // World::IntegrateImplicitEuler, src/Core/World/World.cpp:644-695, fused at the end), laid
-// out as pk_pcg_slab.cu: one block per part, the search directions of its window (rows, then
-// halo) in shared memory, full symmetric rows streamed by TMA bulk copies into a ring, x and
-// r of a row in tensor memory.  What differs:
+// out as pk_pcg_slab.cu (which keeps the per-body solves and the symmetric stream): one block
+// per part, the search directions of its window (rows, then halo) in shared memory, full
+// symmetric rows streamed by TMA bulk copies into a ring, x and r (in FP32 M^-1 too) of a row
+// in tensor memory.  What differs:
 //
 // * one exchange per iteration with the predicted beta of pk_pcg_res.cu; the rows of d that
 //   other windows hold are pushed as tagged packets and collected by the halo warp while the
 //   consumers stream the interior tiles.
-// * a window of 5,300 rows leaves five stages of 19 KB (16 rows, 74 bytes an entry; smaller
-//   copies stream slower), of which the three consumer groups would hold three: a tile's
-//   values go to registers first (a row of up to 16 blocks is two entries on each of its
-//   eight lanes) and the stage is free again before they are multiplied.
-// * M^-1 is read from global memory (part order, nine arrays), two rows at a time.
+// * a tile's values go to registers first (a row of up to 16 blocks is one pass of its lanes)
+//   and the stage is free again before they are multiplied: the three consumer groups would
+//   otherwise hold three of the five FP64 stages that fit beside a window of 5,300 rows (138
+//   against 117 us an iteration).
+// * the producer warp runs on its own, outside the block's barriers.
+// * FP64: M^-1 is read from global memory (part order, nine arrays), two rows at a time.
+//
+// Per iteration, FP64 against the ring kernel: 51,450 rows 27.9 -> 15.8 us, 126 k rows 51.6 ->
+// 29.7, 537 k rows 177.5 -> 117.  FP32 against pcg_slab_kernel: 122,400 rows 22.4 -> 17.6,
+// 199,836 rows 29.3 -> 23.7, 537 k rows 55.6 -> 55.1.  Large FP32 systems are bound by the
+// stream (DRAM), the others by a tile's latency in its consumer warps and by the exchange,
+// whose packets queue behind the ring's refill; holding the refill back until the update is
+// done was slower (57.4 us at 537 k rows), a ring of nine stages too (17.9 at 122,400).
 //
 // All sums keep one fixed order; every wait is bounded and the kernel leaves through its
 // normal exit, after waiting for its own bulk copies.  No TMA multicast is used.
@@ -31,13 +40,11 @@
 namespace pk {
 namespace {
 
-using Real = double;
 constexpr int kConsumerWarps = 12, kGroups = 3, kGroupWarps = 4;
 constexpr int kTeamWarps = kConsumerWarps + 1;     // and the halo warp; the producer runs alone
-constexpr int kThreads64 = 32 * (kConsumerWarps + 2);
+constexpr int kPartThreads = 32 * (kConsumerWarps + 2);
 constexpr int kOwners = 32 * kConsumerWarps;       // record k of thread t: row t + 384 k
 constexpr unsigned kOwnBar = 1, kTeamBar = 2;      // named barriers
-constexpr int kRowBytes = 32;                      // packets of a pushed row
 
 __device__ __forceinline__ void mbar_arrive_one(unsigned long long* bar)
 {
@@ -54,7 +61,7 @@ __device__ __forceinline__ void bulk_g2s_first(void* dst, const void* src, unsig
         : "memory");
 }
 
-// A row record: x and r, twelve of sixteen 32-bit columns.
+// A row record of sixteen 32-bit columns: x and r, in FP32 then M^-1 (column-major).
 struct Rec {
     unsigned w[16];
 };
@@ -78,37 +85,62 @@ __device__ __forceinline__ void rec_st(unsigned addr, const Rec& t)
         : "memory");
 }
 #undef PK_IO
-__device__ __forceinline__ V3<Real> rec_get(const Rec& t, int o)
+__device__ __forceinline__ float rec_at(const Rec& t, int i, float) { return __uint_as_float(t.w[i]); }
+__device__ __forceinline__ double rec_at(const Rec& t, int i, double)
 {
-    return V3<Real>{__hiloint2double((int)t.w[o + 1], (int)t.w[o]), __hiloint2double((int)t.w[o + 3], (int)t.w[o + 2]),
-                    __hiloint2double((int)t.w[o + 5], (int)t.w[o + 4])};
+    return __hiloint2double((int)t.w[2 * i + 1], (int)t.w[2 * i]);
 }
+__device__ __forceinline__ void rec_set(Rec& t, int i, float v) { t.w[i] = __float_as_uint(v); }
+__device__ __forceinline__ void rec_set(Rec& t, int i, double v)
+{
+    t.w[2 * i] = (unsigned)__double2loint(v);
+    t.w[2 * i + 1] = (unsigned)__double2hiint(v);
+}
+template <class Real>
+__device__ __forceinline__ V3<Real> rec_get(const Rec& t, int o)  // 0: x, 3: r
+{
+    return V3<Real>{rec_at(t, o, Real()), rec_at(t, o + 1, Real()), rec_at(t, o + 2, Real())};
+}
+template <class Real>
 __device__ __forceinline__ void rec_put(Rec& t, int o, V3<Real> v)
 {
-    const double d[3] = {v.x, v.y, v.z};
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        t.w[o + 2 * i] = (unsigned)__double2loint(d[i]);
-        t.w[o + 2 * i + 1] = (unsigned)__double2hiint(d[i]);
-    }
+    rec_set(t, o, v.x);
+    rec_set(t, o + 1, v.y);
+    rec_set(t, o + 2, v.z);
 }
-__device__ __forceinline__ V3<Real> ld_q(const Real* p)
+__device__ __forceinline__ V3<float> ld_q(const float* p)
+{
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(p));
+    return V3<float>{a.x, a.y, a.z};
+}
+__device__ __forceinline__ void st_q(float* p, V3<float> v)
+{
+    __stcg(reinterpret_cast<float4*>(p), make_float4(v.x, v.y, v.z, 0.f));
+}
+__device__ __forceinline__ V3<double> ld_q(const double* p)
 {
     const double2 a = __ldcg(reinterpret_cast<const double2*>(p));
-    return V3<Real>{a.x, a.y, __ldcg(p + 2)};
+    return V3<double>{a.x, a.y, __ldcg(p + 2)};
 }
-__device__ __forceinline__ void st_q(Real* p, V3<Real> v)
+__device__ __forceinline__ void st_q(double* p, V3<double> v)
 {
     __stcg(reinterpret_cast<double2*>(p), make_double2(v.x, v.y));
     __stcg(p + 2, v.z);
 }
 
-__global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_constant__ Slab64PcgArgs P)
+template <class Real>
+__global__ void __launch_bounds__(kPartThreads, 1) pcg_part_kernel(const __grid_constant__ PartPcgArgs<Real> P)
 {
-    constexpr int LPR = kSlab64Lanes;
+    constexpr bool kWide = sizeof(Real) == 8;
+    constexpr int LPR = kWide ? kWideLanes : kSlabLanesPerRow, NE = 16 / LPR;  // entries of a lane and pass
+    constexpr int kEntryBytes = kWide ? kWideEntryBytes : kSlabEntryBytes, kValueBytes = 9 * (int)sizeof(Real);
+    constexpr int kCapE = kWide ? kWideCapE : kSlabCapE, kRows = kWide ? kWideRows : kSlabRows;
+    constexpr int kStageBytes = kWide ? kWideStageBytes : kSlabStageBytes;
+    constexpr int kMaxTiles = kWide ? kWideMaxTiles : kSlabMaxTiles;
+    constexpr int kRowBytes = kWide ? 32 : 16;  // packets of a pushed row
     extern __shared__ __align__(128) unsigned char dyn[];
-    __shared__ __align__(8) unsigned long long full_bar[kSlab64MaxStages];
-    __shared__ __align__(8) unsigned long long empty_bar[kSlab64MaxStages];
+    __shared__ __align__(8) unsigned long long full_bar[kPartMaxStages];
+    __shared__ __align__(8) unsigned long long empty_bar[kPartMaxStages];
     __shared__ TagShared sh;
     __shared__ int s_fail, s_bad, s_done, s_halo_gen;
     __shared__ unsigned s_tmem;
@@ -119,10 +151,10 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
     const TagTeam team{kTeamWarps, kTeamBar};
     const int group = warp / kGroupWarps;
     const int slot_row = ((warp % kGroupWarps) * 32 + lane) / LPR, sub = lane % LPR;
-    const int S = min(P.stages, kSlab64MaxStages);
+    const int S = min(P.stages, kPartMaxStages);
     Real* const win = reinterpret_cast<Real*>(dyn);  // 3 values per window row
     unsigned char* const ring = dyn + P.ring_offset;
-    int4* const table = reinterpret_cast<int4*>(ring + (size_t)S * kSlab64StageBytes);
+    int4* const table = reinterpret_cast<int4*>(ring + (size_t)S * kStageBytes);
 
     const unsigned in_flags = *(volatile unsigned*)P.flags;
     const bool skip = P.skip_on_flags && (in_flags & (kFlagPrecomputeFailed | kFlagSingularDiag));
@@ -159,7 +191,7 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (m < 0 || m > kSlabMaxRows || h < 0 || m + h > P.win_cap || row0 < 0 || row0 + m > P.n || ntiles < 0 ||
-        ntiles > kSlab64MaxTiles || halo0 < 0 || halo0 + h > P.halo_count || tile0 < 0 ||
+        ntiles > kMaxTiles || halo0 < 0 || halo0 + h > P.halo_count || tile0 < 0 ||
         tile0 + ntiles > P.tile_count || sends_n < 0 || send0 < 0 || send0 + sends_n > P.halo_count) {
         m = h = ntiles = sends_n = row0 = halo0 = 0;
         if (tid == 0) s_bad = 1;
@@ -168,10 +200,10 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
     // Tile descriptors, checked once: a bad one becomes an empty tile and reports a breakdown.
     for (int i = tid; i < ntiles; i += blockDim.x) {
         int4 d = __ldg(P.tile_desc + tile0 + i);
-        const int ne = (d.y - kSlabHeaderBytes) / kSlab64EntryBytes;
-        if (!(d.x >= 0 && d.y >= kSlabHeaderBytes && d.y <= kSlab64StageBytes && (d.y & 15) == 0 &&
-              d.y == kSlabHeaderBytes + kSlab64EntryBytes * ne && ne <= kSlab64CapE && d.w >= 1 &&
-              d.w <= kSlab64Rows && d.z >= 0 && d.z + d.w <= m &&
+        const int ne = (d.y - kSlabHeaderBytes) / kEntryBytes;
+        if (!(d.x >= 0 && d.y >= kSlabHeaderBytes && d.y <= kStageBytes && (d.y & 15) == 0 &&
+              d.y == kSlabHeaderBytes + kEntryBytes * ne && ne <= kCapE && d.w >= 1 &&
+              d.w <= kRows && d.z >= 0 && d.z + d.w <= m &&
               16ull * (unsigned long long)d.x + (unsigned long long)d.y <= P.stream_bytes)) {
             d = make_int4(0, 0, 0, 0);
             s_bad = 1;
@@ -186,7 +218,7 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
         s_tmem + ((32u * (unsigned)(warp % 4)) << 16) + (unsigned)((warp / 4) * kSlabRowsPerThread * 16);
     unsigned issued = 0;  // tiles issued so far (producer lane 0)
     unsigned xgen = 0;
-    const V3<Real> zero{0.0, 0.0, 0.0};
+    const V3<Real> zero{Real(0), Real(0), Real(0)};
     // Ring position p is stage p % S in its use p / S, counted along; the iteration's first:
     int bstage = 0;
     unsigned buse = 0;
@@ -210,7 +242,7 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
             if (*(volatile int*)&s_done) return;
             mbar_arrive_expect_tx(&full_bar[stage], (unsigned)d.y);
             if (d.y > 0)
-                bulk_g2s_first(ring + (size_t)stage * kSlab64StageBytes, P.stream + 16 * (size_t)d.x, (unsigned)d.y,
+                bulk_g2s_first(ring + (size_t)stage * kStageBytes, P.stream + 16 * (size_t)d.x, (unsigned)d.y,
                                &full_bar[stage], pol);
             ++issued;
             if (++tile == ntiles) tile = 0;
@@ -284,11 +316,11 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
                     break;
                 }
                 const int4 d = table[t];
-                const unsigned char* st = ring + (size_t)s * kSlab64StageBytes;
-                const int ne = d.y > 0 ? (d.y - kSlabHeaderBytes) / kSlab64EntryBytes : 0;
+                const unsigned char* st = ring + (size_t)s * kStageBytes;
+                const int ne = d.y > 0 ? (d.y - kSlabHeaderBytes) / kEntryBytes : 0;
                 const unsigned short* roff = reinterpret_cast<const unsigned short*>(st);
                 const Real* vals = reinterpret_cast<const Real*>(st + kSlabHeaderBytes);
-                const unsigned short* lcol = reinterpret_cast<const unsigned short*>(st + kSlabHeaderBytes + 72 * ne);
+                const unsigned short* lcol = reinterpret_cast<const unsigned short*>(st + kSlabHeaderBytes + kValueBytes * ne);
                 const bool valid = slot_row < d.w, flagged = d.y > 0 && roff[kSlabHaloWord] != 0;
                 int e0 = 0, e1 = 0;
                 if (valid) {
@@ -296,19 +328,19 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
                     e1 = min((int)roff[slot_row + 1], ne);
                 }
                 V3<Real> acc = zero;
-                // two entries a lane and pass, the stage released after the last pass's loads
-                const int passes = __reduce_max_sync(0xffffffffu, (e1 - e0 + 2 * LPR - 1) / (2 * LPR));
+                // sixteen entries of a row a pass, the stage released after the last pass's loads
+                const int passes = __reduce_max_sync(0xffffffffu, (e1 - e0 + 15) / 16);
                 for (int p = 0; p < passes || p == 0; ++p) {
-                    int c[2];
-                    Real b[2][9];
-                    bool live[2];
+                    int c[NE];
+                    Real b[NE][9];
+                    bool live[NE];
 #pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        const int j = e0 + sub + (2 * p + q) * LPR;
+                    for (int q = 0; q < NE; ++q) {
+                        const int j = e0 + sub + (NE * p + q) * LPR;
                         live[q] = j < e1;
                         c[q] = live[q] ? 3 * min((int)lcol[j], wmax) : 0;
 #pragma unroll
-                        for (int e = 0; e < 9; ++e) b[q][e] = live[q] ? vals[9 * j + e] : 0.0;
+                        for (int e = 0; e < 9; ++e) b[q][e] = live[q] ? vals[9 * j + e] : Real(0);
                     }
                     if (p + 1 >= passes) {
                         __syncwarp();
@@ -320,7 +352,7 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
                         halo_in = true;
                     }
 #pragma unroll
-                    for (int q = 0; q < 2; ++q)
+                    for (int q = 0; q < NE; ++q)
                         if (live[q]) {
                             const Real x = win[c[q]], y = win[c[q] + 1], z = win[c[q] + 2];
                             acc.x += b[q][0] * x + b[q][3] * y + b[q][6] * z;
@@ -342,7 +374,7 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
                 if (valid && sub == 0) {
                     const int li = d.z + slot_row;
                     st_q(P.qs + 4 * (size_t)(row0 + li), acc);
-                    dq += dot(V3<Real>{win[3 * li], win[3 * li + 1], win[3 * li + 2]}, acc);
+                    dq += dot_acc<double>(V3<Real>{win[3 * li], win[3 * li + 1], win[3 * li + 2]}, acc);
                     if (!finite3(acc)) bits |= 1u;
                 }
             }
@@ -355,7 +387,7 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
         }
     };
 
-    // f(k, local row or -1, its q, its M^-1) for the thread's rows, the loads of two in flight.
+    // f(k, local row or -1, its q, its M^-1, its record) for the thread's rows, the loads of two in flight.
     auto each_row = [&](bool want_q, auto&& f) {
         for (int k0 = 0; k0 < krows; k0 += 2) {
             V3<Real> q[2] = {zero, zero};
@@ -364,7 +396,8 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
             for (int u = 0; u < 2; ++u) {
                 const int i = rt + kOwners * (k0 + u);
 #pragma unroll
-                for (int e = 0; e < 9; ++e) mi[u][e] = i < m ? __ldcg(P.mrow + (size_t)e * P.n + row0 + i) : 0.0;
+                for (int e = 0; e < 9; ++e)
+                    mi[u][e] = kWide && i < m ? __ldcg(P.mrow + (size_t)e * P.n + row0 + i) : Real(0);
                 if (want_q && i < m) q[u] = ld_q(P.qs + 4 * (size_t)(row0 + i));
             }
 #pragma unroll
@@ -372,7 +405,13 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
                 if (k0 + u >= krows) break;
                 const int i = rt + kOwners * (k0 + u);
                 __syncwarp();
-                f(k0 + u, i < m ? i : -1, q[u], mi[u]);
+                Rec rec;
+                rec_ld(tmem0 + 16u * (unsigned)(k0 + u), rec);
+                if (!kWide) {
+#pragma unroll
+                    for (int e = 0; e < 9; ++e) mi[u][e] = rec_at(rec, 6 + e, Real());
+                }
+                f(k0 + u, i < m ? i : -1, q[u], mi[u], rec);
             }
         }
     };
@@ -386,13 +425,18 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
     // consumers' reads wait for too).
     auto push_rows = [&](unsigned tag) {
         if (!consumer) return;
+        int2 next[2];  // loaded while the barrier completes
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            next[u] = rt + u * kOwners < sends_n ? __ldg(P.send + send0 + rt + u * kOwners) : make_int2(-1, -1);
         asm volatile("bar.sync %0, %1;" ::"r"(kOwnBar), "r"(kOwners) : "memory");
-#pragma unroll 4
-        for (int e = rt; e < sends_n; e += kOwners) {
-            const int2 s = __ldg(P.send + send0 + e);
-            if ((unsigned)s.x < (unsigned)m && (unsigned)s.y < (unsigned)P.halo_count)
-                st_row(P.rows_in + (size_t)s.y * kRowBytes, get_d(s.x), tag);
-        }
+        auto push = [&](int2 e) {
+            if ((unsigned)e.x < (unsigned)m && (unsigned)e.y < (unsigned)P.halo_count)
+                st_row(P.rows_in + (size_t)e.y * kRowBytes, get_d(e.x), tag);
+        };
+        push(next[0]);
+        push(next[1]);
+        for (int e = rt + 2 * kOwners; e < sends_n; e += kOwners) push(__ldg(P.send + send0 + e));
     };
     auto exchange = [&](double (&v)[kTagSums], unsigned& bits) {
         return tag_exchange(P.sums_in, (int)gridDim.x, blk, ++xgen, v, bits, kConsumerWarps, P.flags, team, sh);
@@ -427,14 +471,17 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
                 for (int e = 0; e < 9; ++e) {
                     mi[e] = __ldg(P.minv + 9 * (size_t)c + e);
                     fin = fin && isfinite(mi[e]);
-                    __stcg(P.mrow + (size_t)e * P.n + row0 + i, mi[e]);
+                    if constexpr (kWide)
+                        __stcg(P.mrow + (size_t)e * P.n + row0 + i, mi[e]);
+                    else
+                        rec_set(rec, 6 + e, mi[e]);
                 }
                 const V3<Real> s = apply_minv(mi, b);
                 if (!finite3(b)) bad |= 1u;
                 if (!fin || !finite3(s)) bad |= 2u;
-                rec_put(rec, 6, b);
+                rec_put(rec, 3, b);
                 put_d(i, s);
-                rs_next += dot(b, s);
+                rs_next += dot_acc<double>(b, s);
             }
             __syncwarp();
             rec_st(tmem0 + 16u * (unsigned)k, rec);
@@ -491,13 +538,11 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
             phase_a(it, v[0], bits);
             if (s_fail) bits |= 8u;
             team.sync();  // q of all rows is written
-            each_row(true, [&](int k, int i, V3<Real> q, const Real(&mi)[9]) {
-                Rec rec;
-                rec_ld(tmem0 + 16u * (unsigned)k, rec);
+            each_row(true, [&](int, int i, V3<Real> q, const Real(&mi)[9], Rec& rec) {
                 if (i < 0) return;
-                const V3<Real> r = rec_get(rec, 6), s = apply_minv(mi, r), z = apply_minv(mi, q);
-                v[1] += dot(q, s) + dot(r, z);
-                v[2] += dot(q, z);
+                const V3<Real> r = rec_get<Real>(rec, 3), s = apply_minv(mi, r), z = apply_minv(mi, q);
+                v[1] += dot_acc<double>(q, s) + dot_acc<double>(r, z);
+                v[2] += dot_acc<double>(q, z);
             });
             v[3] = rs_next;
             if (!exchange(v, bits) || (bits & 8u)) {
@@ -524,16 +569,16 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
             sbad = 0;
             rs_next = 0.0;
             // x += alpha d, r -= alpha q, s = M^-1 r; with the prediction also d = s + beta d.
-            each_row(true, [&](int k, int i, V3<Real> q, const Real(&mi)[9]) {
-                Rec rec;
-                rec_ld(tmem0 + 16u * (unsigned)k, rec);
+            const Scale<Real> pa(alpha), na = pa.negated();
+            const Real bt = Real(beta);
+            each_row(true, [&](int k, int i, V3<Real> q, const Real(&mi)[9], Rec& rec) {
                 if (i >= 0) {
-                    const V3<Real> d = get_d(i), r = fma3(-alpha, q, rec_get(rec, 6)), s = apply_minv(mi, r);
-                    rec_put(rec, 0, fma3(alpha, d, rec_get(rec, 0)));
-                    rec_put(rec, 6, r);
+                    const V3<Real> d = get_d(i), r = na.axpy(q, rec_get<Real>(rec, 3)), s = apply_minv(mi, r);
+                    rec_put(rec, 0, pa.axpy(d, rec_get<Real>(rec, 0)));
+                    rec_put(rec, 3, r);
                     if (!finite3(s)) sbad = 2u;
-                    rs_next += dot(r, s);
-                    if (pending) put_d(i, fma3(beta, d, s));
+                    rs_next += dot_acc<double>(r, s);
+                    if (pending) put_d(i, fma3(bt, d, s));
                 }
                 __syncwarp();
                 rec_st(tmem0 + 16u * (unsigned)k, rec);
@@ -549,10 +594,9 @@ __global__ void __launch_bounds__(kThreads64, 1) pcg_slab64_kernel(const __grid_
                 if (!close(w[3], wb & 2u, it + 1) || it + 1 >= P.max_iterations || delta <= target) break;
                 beta = delta / old;
                 sbad = 0;
-                each_row(false, [&](int k, int i, V3<Real>, const Real(&mi)[9]) {
-                    Rec rec;
-                    rec_ld(tmem0 + 16u * (unsigned)k, rec);
-                    if (i >= 0) put_d(i, fma3(beta, get_d(i), apply_minv(mi, rec_get(rec, 6))));
+                const Real bc = Real(beta);
+                each_row(false, [&](int, int i, V3<Real>, const Real(&mi)[9], Rec& rec) {
+                    if (i >= 0) put_d(i, fma3(bc, get_d(i), apply_minv(mi, rec_get<Real>(rec, 3))));
                 });
             }
             push_rows((unsigned)it + 2u);
@@ -599,8 +643,8 @@ final_check:
             }
         };
         each_node([&](const Rec& rec, int c, int, V3<Real> xo, V3<Real> vo) {
-            const V3<Real> dv = have_x ? rec_get(rec, 0) : zero, r = rec_get(rec, 6);
-            v[0] += dot(r, r);
+            const V3<Real> dv = have_x ? rec_get<Real>(rec, 0) : zero, r = rec_get<Real>(rec, 3);
+            v[0] += dot_acc<double>(r, r);
             st3(P.x, c, dv);
             if (!finite3(dv)) bad |= 1u;
             if (P.integrate) {
@@ -623,7 +667,7 @@ final_check:
                 fl |= kFlagIntegrateAbort;
             } else {
                 each_node([&](const Rec& rec, int, int node, V3<Real> xo, V3<Real> vo) {
-                    const V3<Real> nv = vo + rec_get(rec, 0);
+                    const V3<Real> nv = vo + rec_get<Real>(rec, 0);
                     const V3<Real> nx = xo + nv * P.dt;
                     st3(P.node_v, node, nv);
                     st3(P.node_x, node, nx);
@@ -664,8 +708,8 @@ finish:
 // entry in stream order, gathered from the entry's upper block (element j = 3 c + i of a
 // transposed entry is element 3 i + c of the block; padding entries are zero).  A tile that
 // does not match its entry list (the host never builds one) is left alone.
-constexpr int kFill64Threads = 128;
-__global__ void __launch_bounds__(kFill64Threads) slab64_fill_kernel(Slab64FillArgs A)
+constexpr int kWideFillThreads = 128;
+__global__ void __launch_bounds__(kWideFillThreads) wide_fill_kernel(WideFillArgs A)
 {
     const int t = blockIdx.x;
     if (t >= A.tile_count) return;
@@ -673,19 +717,19 @@ __global__ void __launch_bounds__(kFill64Threads) slab64_fill_kernel(Slab64FillA
     const int e0 = __ldg(A.tile_entry0 + t), ne = __ldg(A.tile_entry0 + t + 1) - e0;
     const unsigned long long at = 16ull * (unsigned long long)d.x;
     if (e0 < 0 || ne <= 0 || e0 + ne > A.entries || d.x < 0 || (ne & 7) != 0 || (e0 & 7) != 0 ||
-        d.y != kSlabHeaderBytes + kSlab64EntryBytes * ne || at + (unsigned long long)d.y > A.stream_bytes)
+        d.y != kSlabHeaderBytes + kWideEntryBytes * ne || at + (unsigned long long)d.y > A.stream_bytes)
         return;
     unsigned char* out = A.stream + at;
     if (A.layout) {
         const float4* src = reinterpret_cast<const float4*>(A.layout + (size_t)kSlabHeaderBytes * t + 2 * (size_t)e0);
         float4* head = reinterpret_cast<float4*>(out);
         float4* cols = reinterpret_cast<float4*>(out + kSlabHeaderBytes + 72 * ne);
-        for (int i = threadIdx.x; i < kSlabHeaderBytes / 16 + ne / 8; i += kFill64Threads)
+        for (int i = threadIdx.x; i < kSlabHeaderBytes / 16 + ne / 8; i += kWideFillThreads)
             (i < kSlabHeaderBytes / 16 ? head[i] : cols[i - kSlabHeaderBytes / 16]) = __ldg(src + i);
         return;
     }
     double2* dst = reinterpret_cast<double2*>(out + kSlabHeaderBytes);
-    for (int f2 = threadIdx.x; f2 < 9 * ne / 2; f2 += kFill64Threads) {
+    for (int f2 = threadIdx.x; f2 < 9 * ne / 2; f2 += kWideFillThreads) {
         double v[2];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -701,34 +745,41 @@ __global__ void __launch_bounds__(kFill64Threads) slab64_fill_kernel(Slab64FillA
 
 }  // namespace
 
-int pcg_slab64_max_grid()
+template <class Real>
+int pcg_part_max_grid()
 {
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaFuncSetAttribute(pcg_slab64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlab64SmemLimit) !=
-            cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_slab64_kernel, kThreads64, kSlab64SmemLimit) !=
+        cudaFuncSetAttribute(pcg_part_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kPartSmemLimit) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_part_kernel<Real>, kPartThreads, kPartSmemLimit) !=
             cudaSuccess)
         return 0;
     return sms * per_sm < kTagMaxGroup ? sms * per_sm : kTagMaxGroup;
 }
 
-cudaError_t launch_pcg_slab64_kernel(const Slab64PcgArgs& args, int grid, cudaStream_t stream)
+template <class Real>
+cudaError_t launch_pcg_part_kernel(const PartPcgArgs<Real>& args, int grid, cudaStream_t stream)
 {
-    Slab64PcgArgs a = args;
+    PartPcgArgs<Real> a = args;
     void* kargs[] = {&a};
-    const size_t smem = args.ring_offset + size_t(args.stages) * kSlab64StageBytes + 16 * size_t(kSlab64MaxTiles);
-    const cudaError_t e =
-        cudaFuncSetAttribute(pcg_slab64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlab64SmemLimit);
+    const size_t smem = args.ring_offset + size_t(args.stages) * part_stage(sizeof(Real)) + part_table(sizeof(Real));
+    const cudaError_t e = cudaFuncSetAttribute(pcg_part_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)kPartSmemLimit);
     if (e != cudaSuccess) return e;
-    return cudaLaunchCooperativeKernel((const void*)pcg_slab64_kernel, dim3(grid), dim3(kThreads64), kargs, smem, stream);
+    return cudaLaunchCooperativeKernel((const void*)pcg_part_kernel<Real>, dim3(grid), dim3(kPartThreads), kargs, smem,
+                                       stream);
 }
+template int pcg_part_max_grid<float>();
+template int pcg_part_max_grid<double>();
+template cudaError_t launch_pcg_part_kernel<float>(const PartPcgArgs<float>&, int, cudaStream_t);
+template cudaError_t launch_pcg_part_kernel<double>(const PartPcgArgs<double>&, int, cudaStream_t);
 
-cudaError_t launch_slab64_fill_kernel(const Slab64FillArgs& args, cudaStream_t stream)
+cudaError_t launch_wide_fill_kernel(const WideFillArgs& args, cudaStream_t stream)
 {
     if (args.tile_count <= 0) return cudaSuccess;
-    slab64_fill_kernel<<<args.tile_count, kFill64Threads, 0, stream>>>(args);
+    wide_fill_kernel<<<args.tile_count, kWideFillThreads, 0, stream>>>(args);
     return cudaGetLastError();
 }
 

@@ -181,8 +181,8 @@ std::string build_layout(int n, const int* row_start, const int* col, const int*
 
     // Pass 1: tiles of consecutive owned rows, at most kSlabRows rows and kSlabCapE
     // entries (padded to a multiple of 8 so the arrays stay 16-byte aligned).
-    const int tile_rows = wide ? kSlab64Rows : kSlabRows, cap = wide ? kSlab64CapE : kSlabCapE;
-    const int entry_bytes = wide ? kSlab64EntryBytes : kSlabEntryBytes;
+    const int tile_rows = wide ? kWideRows : kSlabRows, cap = wide ? kWideCapE : kSlabCapE;
+    const int entry_bytes = wide ? kWideEntryBytes : kSlabEntryBytes;
     std::vector<int> part_tile0(parts + 1, 0);
     size_t stream_bytes = 0, entries = 0;
     for (int p = 0; p < parts; ++p) {
@@ -211,7 +211,7 @@ std::string build_layout(int n, const int* row_start, const int* col, const int*
             if (entries > 0x7fffffffu) return "stream too large";
             a = b;
         }
-        if (static_cast<int>(out.tile_desc.size() / 4) - part_tile0[p] > (wide ? kSlab64MaxTiles : kSlabMaxTiles))
+        if (static_cast<int>(out.tile_desc.size() / 4) - part_tile0[p] > (wide ? kWideMaxTiles : kSlabMaxTiles))
             return "a part has more tiles than the table holds";
     }
     part_tile0[parts] = static_cast<int>(out.tile_desc.size() / 4);
@@ -775,7 +775,7 @@ std::string build_slab_plan(int n, const int* row_start, const int* col, const i
     std::vector<int> len(n);
     for (int r = 0; r < n; ++r) len[r] = (row_start[r + 1] - row_start[r]) + (lt_start[r + 1] - lt_start[r]);
     for (int r = 0; r < n; ++r)
-        if (len[r] > (wide ? kSlab64CapE : kSlabCapE)) return "a row has more blocks than a tile holds";
+        if (len[r] > (wide ? kWideCapE : kSlabCapE)) return "a row has more blocks than a tile holds";
     std::vector<int> part_of(n, 0);
     std::vector<double> w(n);
     const double extra = row_weight_extra();
@@ -801,7 +801,7 @@ std::string build_slab_plan(int n, const int* row_start, const int* col, const i
     }
     out.part_body.assign(parts, 0);
     out.launch_start = {0, parts};
-    if (wide) add_sends(out);
+    if (!out.sym) add_sends(out);
     return "";
 }
 

@@ -92,14 +92,14 @@ static_assert(2 * (kSlabRows + 1) <= kSlabHeaderBytes, "header too small");
 constexpr int kSlabHaloWord = kSlabHeaderBytes / 2 - 1;
 static_assert(kSlabHaloWord >= kSlabRows + 1, "the halo word must not overlap the row offsets");
 
-// The FP64 form of the stream (pk_pcg_slab64.cu): the full rows in tiles of half as many rows,
+// The FP64 (wide) form of the stream (pk_pcg_part.cu): the full rows in tiles of half as many rows,
 // eight consumer lanes a row, 74 bytes an entry.
-constexpr int kSlab64Rows = 16, kSlab64Lanes = 8;
-constexpr int kSlab64EntryBytes = 74;   // 9 doubles + u16 column
-constexpr int kSlab64CapE = 256;
-constexpr int kSlab64StageBytes = 19072;
-constexpr int kSlab64MaxTiles = 256;
-static_assert(kSlabHeaderBytes + kSlab64CapE * kSlab64EntryBytes <= kSlab64StageBytes, "stage too small");
+constexpr int kWideRows = 16, kWideLanes = 8;
+constexpr int kWideEntryBytes = 74;   // 9 doubles + u16 column
+constexpr int kWideCapE = 256;
+constexpr int kWideStageBytes = 19072;
+constexpr int kWideMaxTiles = 256;
+static_assert(kSlabHeaderBytes + kWideCapE * kWideEntryBytes <= kWideStageBytes, "stage too small");
 
 struct SlabPlan {
     int n = 0;
@@ -116,7 +116,8 @@ struct SlabPlan {
     int max_window = 0, max_tiles = 0, max_rows = 0;
     // FP64 form: `stream` holds only the tiles' headers and columns, one after another (a tile's
     // at kSlabHeaderBytes x tile + 2 x its first entry); the whole stream has stream_bytes.
-    // send: what each part sends, part by part from send_start, {row of the part, halo_src index}.
+    // send (coupled full rows): what each part sends, part by part from send_start, {row of the
+    // part, halo_src index}.
     bool wide = false;
     size_t stream_bytes = 0;
     std::vector<int> send, send_start;

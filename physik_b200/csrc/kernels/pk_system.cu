@@ -251,10 +251,10 @@ struct pk_system {
     DevBuf slab_export;  // per slab row: held by another part's window
     int slab_fill_entries = 0;
     DevBuf slab_qs, slab_ss;
-    // part-resident PCG in FP64 (pk_pcg_slab64.cu): shares the buffers above
+    // coupled part-resident PCG (pk_pcg_part.cu): shares the buffers above
     bool wide_tried = false;
-    int wide_parts = 0, wide_window = 0, wide_halo = 0;
-    DevBuf wide_send, wide_send_start, wide_inbox, wide_mrow;
+    int part_parts = 0, part_window = 0, part_halo = 0;
+    DevBuf part_send, part_send_start, part_inbox, part_mrow;
     // resident PCG (pk_pcg_res.cu): the layout where the whole matrix fits on chip
     bool res_tried = false;
     int res_parts = 0;            // blocks of the launch (0: does not apply)
@@ -553,7 +553,7 @@ void reset_slab(pk_system* s)
     s->res_tried = false;
     s->res_parts = 0;
     s->wide_tried = false;
-    s->wide_parts = 0;
+    s->part_parts = 0;
 }
 
 // Copies the assembled upper blocks (and their transposes) into the slab stream.
@@ -703,6 +703,12 @@ int ensure_resident(pk_system* s, bool bodies)
     return PK_OK;
 }
 
+// The rows pushed between blocks (at most two packets each), then the blocks' inboxes.
+size_t part_inbox_bytes(int halo, int parts)
+{
+    return 32 * static_cast<size_t>(halo) + 2 * pk::kResSlotBytes * static_cast<size_t>(parts) * parts;
+}
+
 // Builds and uploads the part-resident kernel's layout if it has not been tried yet for
 // this pattern and grid (synchronous: never called while a stream capture is open).
 // Parts are cut by the rows' node positions at this moment.  Not applicable (too large
@@ -836,18 +842,23 @@ int ensure_slab(pk_system* s)
     s->slab_fill_entries = static_cast<int>(plan.fill_src.size());
     s->slab_halo_count = static_cast<int>(plan.halo_src.size());
     s->slab_parts = plan.parts;
+    s->part_parts = 0;
+    if (!bodies && !plan.sym && plan.parts <= pk::pcg_part_max_grid<float>()) {  // (else pcg_slab_kernel)
+        rc = upload_raw<int>(s->part_send, plan.send.data(), plan.send.size(), s->stream);
+        if (!rc) rc = upload_raw<int>(s->part_send_start, plan.send_start.data(), plan.send_start.size(), s->stream);
+        if (rc) return rc;
+        s->part_halo = s->slab_halo_count;
+        s->part_window = plan.max_window;
+        PK_CHECK(s->part_inbox.ensure(part_inbox_bytes(s->part_halo, plan.parts)));
+        s->part_parts = plan.parts;
+    }
     return PK_OK;
 }
 
-// FP64: the rows pushed between blocks (two packets each), then the blocks' inboxes.
-size_t wide_inbox_bytes(int halo, int parts)
-{
-    return 32 * static_cast<size_t>(halo) + 2 * pk::kResSlotBytes * static_cast<size_t>(parts) * parts;
-}
 // Writes the FP64 stream's blocks, or (layout, once) its headers and columns.
-int slab64_fill(pk_system* s, const unsigned char* layout)
+int wide_fill(pk_system* s, const unsigned char* layout)
 {
-    pk::Slab64FillArgs f{};
+    pk::WideFillArgs f{};
     f.values = s->values.as<double>();
     f.nnz = s->nnz;
     f.tile_desc = s->slab_tiles.as<int4>();
@@ -858,21 +869,21 @@ int slab64_fill(pk_system* s, const unsigned char* layout)
     f.layout = layout;
     f.stream = s->slab_stream.as<unsigned char>();
     f.stream_bytes = s->slab_stream_bytes;
-    PK_CHECK(pk::launch_slab64_fill_kernel(f, s->stream));
+    PK_CHECK(pk::launch_wide_fill_kernel(f, s->stream));
     s->launches += 1;
     return PK_OK;
 }
-// The same for the FP64 kernel, after the resident layout did not apply (coupled solves with
-// the kernel left to the library); where it does not apply either, wide_parts stays 0 and the
+// The same in FP64, after the resident layout did not apply (coupled solves with
+// the kernel left to the library); where it does not apply either, part_parts stays 0 and the
 // ring kernel solves.
-int ensure_slab64(pk_system* s)
+int ensure_wide(pk_system* s)
 {
     if (s->wide_tried || s->res_parts > 0 || requested_kernel() != -1 || s->kernel_choice > 0 || s->dyn_count <= 0 ||
         !s->have_pattern)
         return PK_OK;
     s->wide_tried = true;
-    s->wide_parts = 0;
-    int grid = pk::pcg_slab64_max_grid();
+    s->part_parts = 0;
+    int grid = pk::pcg_part_max_grid<double>();
     if (s->pcg_grid_override > 0) grid = std::min(grid, s->pcg_grid_override);
     grid = std::min(grid, std::max(1, s->dyn_count / 64));
     const int n = s->dyn_count;
@@ -891,68 +902,74 @@ int ensure_slab64(pk_system* s)
     if (!rc) rc = upload_raw<int>(s->slab_perm, plan.perm.data(), plan.perm.size(), s->stream);
     if (!rc) rc = upload_raw<unsigned>(s->slab_fill_src, plan.fill_src.data(), plan.fill_src.size(), s->stream);
     if (!rc) rc = upload_raw<int>(s->slab_tile_e0, plan.tile_entry0.data(), plan.tile_entry0.size(), s->stream);
-    if (!rc) rc = upload_raw<int>(s->wide_send, plan.send.data(), plan.send.size(), s->stream);
-    if (!rc) rc = upload_raw<int>(s->wide_send_start, plan.send_start.data(), plan.send_start.size(), s->stream);
+    if (!rc) rc = upload_raw<int>(s->part_send, plan.send.data(), plan.send.size(), s->stream);
+    if (!rc) rc = upload_raw<int>(s->part_send_start, plan.send_start.data(), plan.send_start.size(), s->stream);
     if (rc) return rc;
     PK_CHECK(s->slab_stream.ensure(plan.stream_bytes));
     PK_CHECK(s->slab_qs.ensure(4 * sizeof(double) * static_cast<size_t>(n)));
-    PK_CHECK(s->wide_mrow.ensure(9 * sizeof(double) * static_cast<size_t>(n)));
+    PK_CHECK(s->part_mrow.ensure(9 * sizeof(double) * static_cast<size_t>(n)));
     s->slab_stream_bytes = plan.stream_bytes;
     s->slab_tile_count = static_cast<int>(plan.tile_desc.size() / 4);
     s->slab_fill_entries = static_cast<int>(plan.fill_src.size());
-    s->wide_halo = static_cast<int>(plan.halo_src.size());
-    s->wide_window = plan.max_window;
-    PK_CHECK(s->wide_inbox.ensure(wide_inbox_bytes(s->wide_halo, plan.parts)));
-    rc = slab64_fill(s, layout.as<unsigned char>());
+    s->part_halo = static_cast<int>(plan.halo_src.size());
+    s->part_window = plan.max_window;
+    PK_CHECK(s->part_inbox.ensure(part_inbox_bytes(s->part_halo, plan.parts)));
+    rc = wide_fill(s, layout.as<unsigned char>());
     if (rc) return rc;
     PK_CHECK(cudaStreamSynchronize(s->stream));
-    s->wide_parts = plan.parts;
+    s->part_parts = plan.parts;
     return PK_OK;
 }
 
-int run_pcg_slab64(pk_system* s, const pk_step_params& p, int skip_on_flags)
+template <class Real>
+int run_pcg_part(pk_system* s, const pk_step_params& p, int skip_on_flags)
 {
     int rc = ensure_solver_buffers(s, 1);
-    if (!rc) rc = slab64_fill(s, nullptr);
+    if (!rc) {
+        if constexpr (std::is_same<Real, double>::value)
+            rc = wide_fill(s, nullptr);
+        else if (!s->slab_filled)
+            rc = slab_fill(s);
+    }
     if (rc) return rc;
     pk::DevStats* st = s->stats.as<pk::DevStats>();
-    pk::Slab64PcgArgs a{};
+    pk::PartPcgArgs<Real> a{};
     a.n = s->dyn_count;
     a.part_info = s->slab_part_info.as<int>();
-    a.send_start = s->wide_send_start.as<int>();
-    a.send = s->wide_send.as<int2>();
+    a.send_start = s->part_send_start.as<int>();
+    a.send = s->part_send.as<int2>();
     a.tile_desc = s->slab_tiles.as<int4>();
     a.tile_count = s->slab_tile_count;
-    a.halo_count = s->wide_halo;
+    a.halo_count = s->part_halo;
     a.stream = s->slab_stream.as<unsigned char>();
     a.stream_bytes = s->slab_stream_bytes;
-    a.win_cap = s->wide_window;
-    a.stages = pk::slab64_stages(a.win_cap);
-    a.ring_offset = static_cast<unsigned>(pk::slab64_ring_offset(a.win_cap));
-    a.rows_in = s->wide_inbox.as<unsigned char>();
-    a.sums_in = a.rows_in + 32 * static_cast<size_t>(s->wide_halo);
+    a.win_cap = s->part_window;
+    a.stages = pk::part_stages(sizeof(Real), a.win_cap);
+    a.ring_offset = static_cast<unsigned>(pk::part_ring_offset(sizeof(Real), a.win_cap));
+    a.rows_in = s->part_inbox.as<unsigned char>();
+    a.sums_in = a.rows_in + 4 * sizeof(Real) * static_cast<size_t>(s->part_halo);
     a.perm = s->slab_perm.as<int>();
-    a.b = s->rhs.as<double>();
-    a.minv = s->minv.as<double>();
-    a.x = s->px.as<double>();
-    a.qs = s->slab_qs.as<double>();
-    a.mrow = s->wide_mrow.as<double>();
+    a.b = s->rhs.as<Real>();
+    a.minv = s->minv.as<Real>();
+    a.x = s->px.as<Real>();
+    a.qs = s->slab_qs.as<Real>();
+    a.mrow = s->part_mrow.as<Real>();
     a.max_iterations = p.max_iterations;
-    a.tolerance = p.tolerance;
+    a.tolerance = static_cast<double>(static_cast<Real>(p.tolerance));
     a.skip_on_flags = skip_on_flags;
     a.integrate = p.integrate;
-    a.dt = p.dt;
+    a.dt = static_cast<Real>(p.dt);
     a.dyn_to_node = s->dyn_to_node.as<int>();
-    a.node_x = s->x.as<double>();
-    a.node_v = s->v.as<double>();
+    a.node_x = s->x.as<Real>();
+    a.node_v = s->v.as<Real>();
     a.flags = &st->flags;
     a.stats = st;
     // (no packet may carry a tag of the last solve)
-    PK_CHECK(cudaMemsetAsync(s->wide_inbox.p, 0, wide_inbox_bytes(s->wide_halo, s->wide_parts), s->stream));
-    PK_CHECK(pk::launch_pcg_slab64_kernel(a, s->wide_parts, s->stream));
+    PK_CHECK(cudaMemsetAsync(s->part_inbox.p, 0, part_inbox_bytes(s->part_halo, s->part_parts), s->stream));
+    PK_CHECK(pk::launch_pcg_part_kernel<Real>(a, s->part_parts, s->stream));
     s->launches += 1;
-    s->last_kernel = 0;
-    s->last_blocks = s->wide_parts;
+    s->last_kernel = std::is_same<Real, double>::value ? 0 : 3;
+    s->last_blocks = s->part_parts;
     return PK_OK;
 }
 
@@ -962,7 +979,7 @@ int ensure_slab_any(pk_system* s)
     if (s->precision == PK_PREC_MIXED) return ensure_slab<double>(s);
     if (batched_solve(s)) return PK_OK;
     const int rc = ensure_resident<double>(s, false);
-    return rc ? rc : ensure_slab64(s);
+    return rc ? rc : ensure_wide(s);
 }
 
 // The per-body round table for the next solve (slab_schedule_kernel) on `stream`.
@@ -1275,14 +1292,15 @@ int run_pcg(pk_system* s, const pk_step_params& p, int skip_on_flags)
         if (rc) return rc;
     } else {
         int rc = ensure_resident<double>(s, false);
-        if (!rc) rc = ensure_slab64(s);
+        if (!rc) rc = ensure_wide(s);
         if (rc) return rc;
     }
     const int kernel = solve_kernel(s);
     s->last_kernel = kernel;
     if (s->res_parts > 0 && kernel == (std::is_same<Real, float>::value ? 3 : 0))
         return run_pcg_resident<Real>(s, p, skip_on_flags);
-    if (std::is_same<Real, double>::value && kernel == 0 && s->wide_parts > 0) return run_pcg_slab64(s, p, skip_on_flags);
+    if (std::is_same<Real, double>::value && kernel == 0 && s->part_parts > 0) return run_pcg_part<Real>(s, p, skip_on_flags);
+    if (kernel == 3 && s->part_parts > 0) return run_pcg_part<Real>(s, p, skip_on_flags);
     if (kernel == 3) return run_pcg_slab<Real, Acc>(s, p, skip_on_flags);
     if (kernel == 0 && s->ring_tiles > 0) {
         int rc = ensure_solver_buffers(s, 1);
