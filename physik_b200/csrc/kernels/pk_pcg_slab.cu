@@ -1,4 +1,5 @@
-// pk_pcg_slab.cu -- the part-resident cooperative block-Jacobi PCG kernel.
+// pk_pcg_slab.cu -- the part-resident cooperative block-Jacobi PCG kernel of the per-body
+// solves and of the symmetric stream form (coupled full rows: pk_pcg_part.cu).
 //
 // The same solve as the other PCG kernels (SolvePreconditionedConjugateGradient,
 // src/Core/Solvers/Linear/ConjugateGradientSolver.cpp:114-241, with the SpMV of
