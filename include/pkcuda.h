@@ -272,7 +272,8 @@ PKCUDA_API int pk_system_set_refinement(pk_system* sys, int passes);
 /* The PCG kernel of the last solve: 0 ring-staged, 1 TMA-staged, 2 unstaged, 3
  * part-resident, 4 per-body batch kernel, 5 part-resident with one group of parts per body
  * (batched solve); where the whole matrix fits the SMs' on-chip memory, the resident
- * kernel runs as 3 and 5 (FP32 storage) and as 0 (FP64); -1 before the first solve (or a negative PK_ERR_*).
+ * kernel runs as 3 and 5 (FP32 storage) and as 0 (FP64); the part-resident kernel runs as 0
+ * in FP64 too; -1 before the first solve (or a negative PK_ERR_*).
  * blocks (may be NULL) receives the blocks it ran on. */
 PKCUDA_API int pk_system_pcg_kernel(pk_system* sys, int* blocks);
 /* Stream form of the part-resident kernel's layout in the last solve: 0 full symmetric

@@ -2,6 +2,7 @@
 #include "pk_res_plan.h"
 
 #include <algorithm>
+#include <atomic>
 #include <numeric>
 
 #include "pk_slab_plan.h"
@@ -160,11 +161,19 @@ std::string build_cut(int n, const int* row_start, const int* col, const int* lt
         }
     }
     // 4. halos
+    std::atomic<bool> failed{false};
     auto each_part = [&](const std::function<void(int, int)>& f) {
+        const auto guarded = [&](int p, int t) {
+            try {
+                f(p, t);
+            } catch (...) {  // nothing may leave a worker thread
+                failed = true;
+            }
+        };
         if (n >= 4096)
-            for_items(parts, f);
+            for_items(parts, guarded);
         else
-            for (int p = 0; p < parts; ++p) f(p, 0);
+            for (int p = 0; p < parts; ++p) guarded(p, 0);
     };
     std::vector<std::vector<int>> halos(parts);
     each_part([&](int p, int) {
@@ -179,6 +188,7 @@ std::string build_cut(int n, const int* row_start, const int* col, const int* lt
         std::sort(halo.begin(), halo.end());
         halo.erase(std::unique(halo.begin(), halo.end()), halo.end());
     });
+    if (failed) return "host memory exhausted while building the layout";
     out.part_info.assign((size_t)kResPartInts * parts, 0);
     for (int p = 0; p < parts; ++p) {
         int* pi = out.part_info.data() + (size_t)kResPartInts * p;
@@ -253,6 +263,7 @@ std::string build_cut(int n, const int* row_start, const int* col, const int* lt
             }
         }
     });
+    if (failed) return "host memory exhausted while building the layout";
     // 6. who sends which row where
     std::vector<std::vector<int>> sends(parts);
     for (int p = 0; p < parts; ++p) {

@@ -895,6 +895,13 @@ int ensure_wide(pk_system* s)
     const std::string why = pk::build_slab_plan(n, s->h_row_start.data(), in.col.data(), s->h_lts.data(), in.ltr.data(),
                                                 in.ltb.data(), in.coords.data(), grid, plan, pk::kSlabFull, true);
     if (!why.empty()) return PK_OK;
+    // Where the stream finds no room the ring kernel, which needs none, solves.
+    size_t free_bytes = 0, total_bytes = 0;
+    const size_t need = plan.stream_bytes + plan.stream.size() + 4 * plan.fill_src.size() +
+                        13 * sizeof(double) * static_cast<size_t>(n) +
+                        part_inbox_bytes(static_cast<int>(plan.halo_src.size()), plan.parts) + (size_t{64} << 20);
+    PK_CHECK(cudaMemGetInfo(&free_bytes, &total_bytes));
+    if (free_bytes < need) return PK_OK;
     DevBuf layout;
     rc = upload_raw<int>(s->slab_part_info, plan.part_info.data(), plan.part_info.size(), s->stream);
     if (!rc) rc = upload_raw<int>(s->slab_tiles, plan.tile_desc.data(), plan.tile_desc.size(), s->stream);
