@@ -61,6 +61,8 @@ __device__ __forceinline__ void bulk_g2s_first(void* dst, const void* src, unsig
         : "memory");
 }
 
+static_assert(kTagSlotBytes == kResSlotBytes, "the host sizes the inboxes");
+
 // A row record of sixteen 32-bit columns: x and r, in FP32 then M^-1 (column-major).
 struct Rec {
     unsigned w[16];
