@@ -632,6 +632,7 @@ __global__ void __launch_bounds__(kBlockThreads, sizeof(Real) == 4 ? 7 : 4)
         sum.c[2] = kscale3(sum.c[2], dt2);
         st9(mine, (size_t)lane, sum);
         const unsigned skip = __ballot_sync(0xffffffffu, diagonal);
+        __syncwarp();  // (a vote orders no memory; the lanes leave lists of different lengths)
         Real* dst = A.values + 9 * (size_t)(k - lane);
 #pragma unroll
         for (int j = 0; j < 9; ++j) {
