@@ -291,6 +291,8 @@ std::string build_res_plan(int n, const int* row_start, const int* col, const in
 {
     out = ResPlan{};
     if (n <= 0 || nseg <= 0 || limits.blocks <= 0 || seg[0] != 0 || seg[nseg] != n) return "empty system";
+    std::vector<double> held;
+    coords = finite_coords(n, coords, held);
     std::vector<int> len(n);
     int longest = 0, largest = 0;
     for (int r = 0; r < n; ++r) {

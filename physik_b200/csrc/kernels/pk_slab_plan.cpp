@@ -728,6 +728,18 @@ std::string build_layout_sym(int n, const int* row_start, const int* col, const 
 
 }  // namespace
 
+const double* finite_coords(int n, const double* coords, std::vector<double>& held)
+{
+    if (!coords) return nullptr;
+    const size_t count = 3 * static_cast<size_t>(n);
+    for (size_t i = 0; i < count; ++i) {
+        if (std::isfinite(coords[i])) continue;
+        if (held.empty()) held.assign(coords, coords + count);
+        held[i] = 0.0;
+    }
+    return held.empty() ? coords : held.data();
+}
+
 int plan_thread_count() { return plan_threads(); }
 void for_items(int count, const std::function<void(int, int)>& f) { parallel_items(count, f); }
 
@@ -771,6 +783,8 @@ std::string build_slab_plan(int n, const int* row_start, const int* col, const i
 {
     out = SlabPlan{};
     if (n <= 0 || parts <= 0) return "empty system";
+    std::vector<double> held;
+    coords = finite_coords(n, coords, held);
     parts = std::min(parts, n);
     std::vector<int> len(n);
     for (int r = 0; r < n; ++r) len[r] = (row_start[r + 1] - row_start[r]) + (lt_start[r + 1] - lt_start[r]);
@@ -812,6 +826,8 @@ std::string build_slab_plan_batched(int n, const int* row_start, const int* col,
     out = SlabPlan{};
     if (n <= 0 || nseg <= 0 || max_blocks <= 0) return "empty system";
     if (seg[0] != 0 || seg[nseg] != n) return "segments do not cover the rows";
+    std::vector<double> held;
+    coords = finite_coords(n, coords, held);
     std::vector<int> len(n);
     for (int r = 0; r < n; ++r) len[r] = (row_start[r + 1] - row_start[r]) + (lt_start[r + 1] - lt_start[r]);
     for (int r = 0; r < n; ++r)

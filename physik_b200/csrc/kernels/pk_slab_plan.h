@@ -136,6 +136,11 @@ std::string build_slab_plan(int n, const int* row_start, const int* col, const i
                             const int* lt_block, const double* coords, int parts, SlabPlan& out,
                             int form = kSlabAuto, bool wide = false);
 
+// The coordinates a layout is cut by: `coords` itself, or a copy in `held` with 0 in place of
+// every value that is not finite (a state may hold any; the cuts sort by them, and NaN has no
+// place in an order).
+const double* finite_coords(int n, const double* coords, std::vector<double>& held);
+
 // f(i, thread) for i in [0, count) on the layout builds' host threads (thread <
 // plan_thread_count()); each i must write only its own outputs.
 int plan_thread_count();

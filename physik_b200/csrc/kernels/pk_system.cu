@@ -286,8 +286,8 @@ struct pk_system {
     int graph_kernels = 0;
     // nodes; snap_x: positions at the start of the last substep (pk_system_snapshot_positions)
     DevBuf x, v, mass, node_to_dyn, snap_x;
-    // The positions first set after the nodes: what layouts are cut by, so that a layout (and
-    // the order of a solve's sums) does not depend on when it is built.
+    // The first finite positions set after the nodes: what layouts are cut by, so that a layout
+    // (and the order of a solve's sums) does not depend on when it is built.
     DevBuf layout_x;
     bool have_layout_x = false;
     DevBuf contact_count, contact_tet, contact_point;  // pk_system_sphere_contacts
@@ -711,8 +711,8 @@ size_t part_inbox_bytes(int halo, int parts)
 
 // Builds and uploads the part-resident kernel's layout if it has not been tried yet for
 // this pattern and grid (synchronous: never called while a stream capture is open).
-// Parts are cut by the rows' node positions at this moment.  Not applicable (too large
-// a window, too long a row) leaves slab_parts at 0 and the reason in slab_reason.
+// Parts are cut by the rows' node positions as first set (layout_inputs).  Not applicable (too
+// large a window, too long a row) leaves slab_parts at 0 and the reason in slab_reason.
 template <class Acc>
 int ensure_slab(pk_system* s)
 {
@@ -1756,6 +1756,22 @@ int download_real_any(pk_system* s, const DevBuf& buf, double* dst, size_t n)
                                         : download_real<float>(buf, dst, n, s->stream);
 }
 
+// x: what was just written to s->x.  A state that is not finite in the storage's type is not
+// kept: a layout built before a finite one is set is cut by the positions it finds.
+template <class T>
+int keep_layout_positions(pk_system* s, const T* x)
+{
+    if (s->have_layout_x) return PK_OK;
+    const bool narrow_type = s->precision != PK_PREC_FP64;
+    for (size_t i = 0; i < 3 * static_cast<size_t>(s->node_count); ++i)
+        if (!(narrow_type ? std::isfinite(static_cast<float>(x[i])) : std::isfinite(x[i]))) return PK_OK;
+    const size_t bytes = 3 * s->rsize() * static_cast<size_t>(s->node_count);
+    PK_CHECK(s->layout_x.ensure(bytes));
+    if (bytes) PK_CHECK(cudaMemcpyAsync(s->layout_x.p, s->x.p, bytes, cudaMemcpyDeviceToDevice, s->stream));
+    s->have_layout_x = true;
+    return PK_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1838,16 +1854,6 @@ PKCUDA_API int pk_system_set_nodes(pk_system* s, int node_count, const int* node
     return PK_OK;
 }
 
-static int keep_layout_positions(pk_system* s)
-{
-    if (s->have_layout_x) return PK_OK;
-    const size_t bytes = 3 * s->rsize() * static_cast<size_t>(s->node_count);
-    PK_CHECK(s->layout_x.ensure(bytes));
-    if (bytes) PK_CHECK(cudaMemcpyAsync(s->layout_x.p, s->x.p, bytes, cudaMemcpyDeviceToDevice, s->stream));
-    s->have_layout_x = true;
-    return PK_OK;
-}
-
 PKCUDA_API int pk_system_set_state_f64(pk_system* s, const double* x, const double* v)
 {
     if (!s || !s->have_nodes) return fail(PK_ERR_STATE, "set_state before set_nodes");
@@ -1862,7 +1868,7 @@ PKCUDA_API int pk_system_set_state_f64(pk_system* s, const double* x, const doub
         if (x) rc = upload_real_any(s, s->x, x, n);
         if (!rc && v) rc = upload_real_any(s, s->v, v, n);
     }
-    return !rc && x ? keep_layout_positions(s) : rc;
+    return !rc && x ? keep_layout_positions(s, x) : rc;
 }
 
 PKCUDA_API int pk_system_set_state_f32(pk_system* s, const float* x, const float* v)
@@ -1879,7 +1885,7 @@ PKCUDA_API int pk_system_set_state_f32(pk_system* s, const float* x, const float
     // float storage: copy straight from the caller's buffer (pinned buffers stay asynchronous)
     if (x) PK_CHECK(cudaMemcpyAsync(s->x.p, x, n * sizeof(float), cudaMemcpyHostToDevice, s->stream));
     if (v) PK_CHECK(cudaMemcpyAsync(s->v.p, v, n * sizeof(float), cudaMemcpyHostToDevice, s->stream));
-    return x ? keep_layout_positions(s) : PK_OK;
+    return x ? keep_layout_positions(s, x) : PK_OK;
 }
 
 PKCUDA_API int pk_system_get_state_f64(pk_system* s, double* x, double* v)
