@@ -369,9 +369,11 @@ PKCUDA_API int pk_slab_plan_batched_selfcheck(int n, const int* row_start, const
 
 /* CPU self-check of the resident PCG kernel's layout (its rows stay on chip for the whole
  * solve): builds it for the upper BSR of segment_count bodies on at most max_blocks blocks
- * in the precision's storage, checks what the kernel checks, and evaluates y = A x as its
- * lanes do.  info (may be NULL) receives {parts, most rows of a part, lanes per row, bytes
- * of shared memory}.  PK_ERR_UNSUPPORTED when the matrix does not fit on chip.  No
+ * and the thread-block clusters that fit them (max_blocks < 0: -max_blocks blocks, no
+ * clusters) in the precision's storage, checks what the kernel checks, and evaluates
+ * y = A x as its lanes do.  info (may be NULL) receives {parts, most rows of a part, lanes
+ * per row, bytes of shared memory, blocks of a cluster (0: none), threads x rows per
+ * thread}: six ints.  PK_ERR_UNSUPPORTED when the matrix does not fit on chip.  No
  * counterpart in the reference (it checks this library's own layout). */
 PKCUDA_API int pk_res_plan_selfcheck(int n, const int* row_start, const int* col_index, const double* values,
                                      const double* x, const double* coords, const int* segment_row_start,
