@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import unittest
 from dataclasses import dataclass
 from typing import Optional
 
@@ -38,6 +39,16 @@ def reference_library_path(precision: str) -> str:
 
 def reference_available(precision: str = "f32") -> bool:
     return os.path.exists(reference_library_path(precision))
+
+
+class ReferenceMissing(unittest.SkipTest):
+    """The reference has not been built here: a test that asks for it is skipped."""
+
+
+def _load_reference(precision: str):
+    if not reference_available(precision):
+        raise ReferenceMissing(f"{reference_library_path(precision)} is missing (make -C oracle ref)")
+    return C.CDLL(reference_library_path(precision))
 
 
 @dataclass
@@ -273,8 +284,7 @@ class Reference:
     """The reference itself (compiled from its sources), driven through ref_harness.cpp."""
 
     def __init__(self, scene, precision: str = "f32", substeps: int = 1):
-        path = reference_library_path(precision)
-        self.lib = C.CDLL(path)
+        self.lib = _load_reference(precision)
         L = self.lib
         L.ref_world_create.restype = _p
         L.ref_world_destroy.argtypes = [_p]
@@ -452,7 +462,7 @@ class Reference:
 
 
 def _ref_lib(precision="f32"):
-    return C.CDLL(reference_library_path(precision))
+    return _load_reference(precision)
 
 
 def reference_bsr_multiply(row_start, col, values, x, precision="f32"):
