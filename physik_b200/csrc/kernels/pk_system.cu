@@ -302,6 +302,7 @@ struct pk_system {
     DevBuf dm_inv64, params64, mass64, elem_u, elem_vx;
     bool rest64_ok = false;  // pk_system_set_rest64 matches the current tets and nodes
     bool lists_ok = false;  // the blocks' tets match the pattern, incidences, tets and node rows
+    bool lists_tried = false;  // they were built for these, or found no room
     // solver
     DevBuf px, pr, psd0, psd1, pq, part_a, part_b, part_bad, sync, stats;
     pk::DevStats* host_stats = nullptr;  // pinned; the second holds an adjoint's forward step
@@ -1513,15 +1514,24 @@ bool assembly_fold_enabled()
 }
 
 // The blocks' tets, built on the device after the pattern, the incidences, the tets or the
-// node rows changed.
+// node rows changed.  Where they find no room (64 bytes a tet, 8 a block) the rows are
+// assembled one thread each, which needs none.
 int ensure_block_lists(pk_system* s)
 {
-    if (s->lists_ok || s->dyn_count <= 0 || s->inc_count <= 0 || !s->have_tets || !block_rows_enabled())
+    if (s->lists_tried || s->dyn_count <= 0 || s->inc_count <= 0 || !s->have_tets || !block_rows_enabled())
         return PK_OK;
     if (s->tet_count >= (1 << 28) || s->inc_count >= (1 << 29)) return PK_OK;  // a list entry is 32 bits
-    PK_CHECK(s->blk_range.ensure(sizeof(int2) * static_cast<size_t>(s->nnz)));
-    PK_CHECK(s->blk_list.ensure(4 * sizeof(unsigned) * static_cast<size_t>(s->inc_count)));
-    PK_CHECK(s->blk_missing.ensure(sizeof(int)));
+    s->lists_tried = true;
+    cudaError_t e = s->blk_range.ensure(sizeof(int2) * static_cast<size_t>(s->nnz));
+    if (e == cudaSuccess) e = s->blk_list.ensure(4 * sizeof(unsigned) * static_cast<size_t>(s->inc_count));
+    if (e == cudaSuccess) e = s->blk_missing.ensure(sizeof(int));
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        s->blk_range.reset();
+        s->blk_list.reset();
+        return PK_OK;
+    }
+    PK_CHECK(e);
     PK_CHECK(cudaMemsetAsync(s->blk_missing.p, 0, sizeof(int), s->stream));
     PK_CHECK(pk::launch_block_list_kernel(s->dyn_count, s->row_start.as<int>(), s->col.as<int>(),
                                           s->inc_start.as<int>(), s->inc_list.as<int>(), s->tet_nodes.as<int4>(),
@@ -1837,7 +1847,7 @@ PKCUDA_API int pk_system_set_nodes(pk_system* s, int node_count, const int* node
     s->have_layout_x = false;
     s->have_snapshot = false;
     s->h_node_to_dyn.assign(node_to_dyn, node_to_dyn + node_count);
-    s->lists_ok = false;
+    s->lists_ok = s->lists_tried = false;
     s->h_mass.assign(mass, mass + node_count);
     s->adj_consts = false;
     int rc = upload_raw<int>(s->node_to_dyn, node_to_dyn, node_count, s->stream);
@@ -2130,7 +2140,7 @@ PKCUDA_API int pk_system_set_tets(pk_system* s, int tet_count, const int* tet_no
     for (long long i = 0; i < 4ll * tet_count; ++i)
         if (tet_nodes[i] < 0 || tet_nodes[i] >= s->node_count) return fail(PK_ERR_ARG, "tet node out of range");
     s->tet_count = tet_count;
-    s->lists_ok = false;
+    s->lists_ok = s->lists_tried = false;
     s->h_tet_nodes.assign(tet_nodes, tet_nodes + 4 * static_cast<size_t>(tet_count));
     s->h_enabled.assign(enabled, enabled + tet_count);
     s->h_damping.assign(damping, damping + tet_count);
@@ -2318,7 +2328,7 @@ PKCUDA_API int pk_system_set_pattern(pk_system* s, int dyn_count, const int* dyn
     s->nnz = nnz;
     s->lt_count = static_cast<int>(ltr.size());
     s->inc_count = inc;
-    s->lists_ok = false;
+    s->lists_ok = s->lists_tried = false;
     s->max_row = max_row;
     s->diag_first = diag_first;
     int rc = upload_raw<int>(s->dyn_to_node, dyn_to_node, dyn_count, s->stream);
