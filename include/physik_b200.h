@@ -254,7 +254,9 @@ PHYSIK_B200_API void PHYSIK_AddPointConnection(PhysikWorldHandle world, int node
                                                float stiffness, float damping);
 
 /* ---- extensions (no counterpart in the reference) --------------------- */
-#define PHYSIK_B200_PRECISION_FP32 0  /* the reference's scalar type: float storage and dot products */
+/* the reference's scalar type: float storage; dot products in float, or in double and judged as floats
+ * (a sum a float does not hold ends the solve, as in the reference) */
+#define PHYSIK_B200_PRECISION_FP32 0
 #define PHYSIK_B200_PRECISION_MIXED 1 /* float storage, double CG scalars, double polar for near-inverted tets */
 #define PHYSIK_B200_PRECISION_FP64 2  /* double everywhere */
 PHYSIK_B200_API void PHYSIK_B200_SetPrecision(PhysikWorldHandle world, int precision);

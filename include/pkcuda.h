@@ -39,7 +39,9 @@ extern "C" {
 #endif
 
 /* Precision of a system: storage / accumulation. */
-#define PK_PREC_FP32 0  /* float storage, float dot products (the reference's scalar type) */
+/* float storage (the reference's scalar type); dot products in float, or in double and judged as
+ * floats (the resident and part-resident kernels: a sum a float does not hold ends the solve) */
+#define PK_PREC_FP32 0
 #define PK_PREC_MIXED 1 /* float storage, double CG scalars and updates, double polar for near-inverted tets */
 #define PK_PREC_FP64 2  /* double everywhere */
 

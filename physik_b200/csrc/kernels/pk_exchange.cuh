@@ -98,6 +98,21 @@ struct Scale<double> {
     __device__ __forceinline__ V3<double> axpy(V3<double> b, V3<double> c) const { return fma3(a, b, c); }
 };
 
+// An FP32 system's sums are added in double here and judged as floats, so that a solve whose
+// sums a float does not hold ends as it does where they are added in float (the other kernels,
+// the reference): from 2^128 infinite, below 2^-150 zero.
+__device__ __forceinline__ double as_float_sum(double v)
+{
+    const int m = __double2hiint(v) & 0x7fffffff;
+    return m >= 0x47f00000 ? (double)INFINITY : m < 0x36900000 ? 0.0 : v;
+}
+// What alpha and beta may reach: the largest finite value of the sums' type.
+template <bool FS>
+constexpr double scalar_max()
+{
+    return FS ? 3.4028234663852886e38 : 1.7976931348623157e308;
+}
+
 // The exchange of a group of blocks through global memory: sums of four doubles and the OR
 // of a word.  A block pushes its sums into the inbox of every member (kTagSlotBytes a
 // sender), so that a reader polls lines nobody else reads.  The inbox of member j has

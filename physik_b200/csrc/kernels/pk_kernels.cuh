@@ -450,6 +450,7 @@ struct PartPcgArgs {
     Real* x;                   // per dynamic row: delta-v out
     Real* qs;                  // 4 per slab row
     Real* mrow;                // FP64: M^-1 in slab order, [9][n]
+    int float_sums;            // FP32 systems: the sums (in double) are judged as floats
     int max_iterations;
     double tolerance;
     int skip_on_flags, integrate;
@@ -501,6 +502,7 @@ struct ResPcgArgs {
     unsigned char* sums_in;          // [2][grid][sender] x kResSlotBytes: tagged sums
     size_t sums_stride;              // bytes of one block's inbox: the largest group's senders
     unsigned* epoch;                 // [grid] tag base of the group starting at each block
+    int float_sums;                  // FP32 systems: the sums (in double) are judged as floats
     int max_iterations;
     double tolerance;
     int skip_on_flags;

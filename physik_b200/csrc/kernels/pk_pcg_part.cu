@@ -130,7 +130,8 @@ __device__ __forceinline__ void st_q(double* p, V3<double> v)
     __stcg(p + 2, v.z);
 }
 
-template <class Real>
+// FS: the sums judged as floats (as_float_sum).
+template <class Real, bool FS>
 __global__ void __launch_bounds__(kPartThreads, 1) pcg_part_kernel(const __grid_constant__ PartPcgArgs<Real> P)
 {
     constexpr bool kWide = sizeof(Real) == 8;
@@ -441,7 +442,12 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_part_kernel(const __grid_
         for (int e = rt + 2 * kOwners; e < sends_n; e += kOwners) push(__ldg(P.send + send0 + e));
     };
     auto exchange = [&](double (&v)[kTagSums], unsigned& bits) {
-        return tag_exchange(P.sums_in, (int)gridDim.x, blk, ++xgen, v, bits, kConsumerWarps, P.flags, team, sh);
+        const bool ok = tag_exchange(P.sums_in, (int)gridDim.x, blk, ++xgen, v, bits, kConsumerWarps, P.flags, team, sh);
+        if constexpr (FS) {
+            v[0] = as_float_sum(v[0]);
+            v[3] = as_float_sum(v[3]);
+        }
+        return ok;
     };
 
     unsigned fl = 0, sbad = 0;
@@ -526,7 +532,8 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_part_kernel(const __grid_
             const double old = delta;
             delta = new_delta;
             // (the last test: delta / old overflows)
-            if (!isfinite(delta) || !isfinite(old) || old <= 0.0 || (old < 1.0 && fabs(delta) > DBL_MAX * old)) {
+            if (!isfinite(delta) || !isfinite(old) || old <= 0.0 ||
+                (old < 1.0 && fabs(delta) > scalar_max<FS>() * old)) {
                 fl |= kFlagBreakdown;
                 return false;
             }
@@ -559,7 +566,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_part_kernel(const __grid_
             const double dq = v[0], inv = 1.0 / dq;
             double alpha = delta * inv;
             alpha = fma(fma(-alpha, dq, delta), inv, alpha);
-            if ((bits & 1u) || !isfinite(dq) || dq <= 0.0 || !isfinite(alpha)) {
+            if ((bits & 1u) || !isfinite(dq) || dq <= 0.0 || !(FS ? fabs(alpha) <= scalar_max<FS>() : isfinite(alpha))) {
                 fl |= kFlagBreakdown;
                 break;
             }
@@ -747,17 +754,31 @@ __global__ void __launch_bounds__(kWideFillThreads) wide_fill_kernel(WideFillArg
 
 }  // namespace
 
+namespace {
+template <class Real>
+const void* part_kernel(bool float_sums)
+{
+    if constexpr (sizeof(Real) == 4)
+        if (float_sums) return (const void*)pcg_part_kernel<Real, true>;
+    return (const void*)pcg_part_kernel<Real, false>;
+}
+}  // namespace
+
 template <class Real>
 int pcg_part_max_grid()
 {
-    int dev = 0, sms = 0, per_sm = 0;
+    int dev = 0, sms = 0, per_sm = 1 << 20;
     if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaFuncSetAttribute(pcg_part_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kPartSmemLimit) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_part_kernel<Real>, kPartThreads, kPartSmemLimit) !=
-            cudaSuccess)
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return 0;
+    for (const bool float_sums : {false, true}) {
+        const void* k = part_kernel<Real>(float_sums);
+        int b = 0;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPartSmemLimit) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, kPartThreads, kPartSmemLimit) != cudaSuccess)
+            return 0;
+        per_sm = b < per_sm ? b : per_sm;
+    }
     return sms * per_sm < kTagMaxGroup ? sms * per_sm : kTagMaxGroup;
 }
 
@@ -767,10 +788,10 @@ cudaError_t launch_pcg_part_kernel(const PartPcgArgs<Real>& args, int grid, cuda
     PartPcgArgs<Real> a = args;
     void* kargs[] = {&a};
     const size_t smem = args.ring_offset + size_t(args.stages) * part_stage(sizeof(Real)) + part_table(sizeof(Real));
-    const cudaError_t e = cudaFuncSetAttribute(pcg_part_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)kPartSmemLimit);
+    const void* k = part_kernel<Real>(args.float_sums != 0);
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPartSmemLimit);
     if (e != cudaSuccess) return e;
-    return cudaLaunchCooperativeKernel((const void*)pcg_part_kernel<Real>, dim3(grid), dim3(kPartThreads), kargs, smem,
+    return cudaLaunchCooperativeKernel(k, dim3(grid), dim3(kPartThreads), kargs, smem,
                                        stream);
 }
 template int pcg_part_max_grid<float>();

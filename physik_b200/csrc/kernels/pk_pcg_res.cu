@@ -44,7 +44,7 @@
 //
 // All sums keep one fixed order: warp shuffles, then the block's warps, then the group's
 // blocks, the same in every block; a run repeats bit for bit.  Sums and scalars are FP64 in
-// every precision.  Every wait is bounded; one that gives up sets the timeout flag, which
+// every precision (an FP32 system's sums are judged as floats).  Every wait is bounded; one that gives up sets the timeout flag, which
 // ends the other blocks' waits.
 #include <cuda_runtime.h>
 #include <float.h>
@@ -166,8 +166,9 @@ __device__ __forceinline__ void words_set(Words& t, int i, double v)
 // MAXT: threads per block at most (256 leaves a thread twice the registers of 512).
 // CL: exchange inside a cluster (else through global memory).
 // R: rows per thread (2: one lane a row, rows tid and tid + T, whose entries alternate in the
-// slots).  TM: slots in tensor memory.
-template <class Real, int MAXT, bool CL, int R, bool TM>
+// slots).  TM: slots in tensor memory.  FS: the sums judged as floats (as_float_sum; a run-time
+// rule cost every precision 1.5 % of an iteration, these instances cost FP32 alone).
+template <class Real, int MAXT, bool CL, int R, bool TM, bool FS>
 __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
 {
     constexpr int KR = res_reg_slots(sizeof(Real), MAXT, R);
@@ -444,7 +445,7 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
         const double old = delta;
         delta = new_delta;
         // (the last test: delta / old overflows)
-        if (!isfinite(delta) || !isfinite(old) || old <= 0.0 || (old < 1.0 && fabs(delta) > DBL_MAX * old)) {
+        if (!isfinite(delta) || !isfinite(old) || old <= 0.0 || (old < 1.0 && fabs(delta) > scalar_max<FS>() * old)) {
             fl |= kFlagBreakdown;
             return false;
         }
@@ -759,6 +760,10 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
             }
         }
         if (timed_out) break;
+        if constexpr (FS) {
+            v[0] = as_float_sum(v[0]);
+            v[3] = as_float_sum(v[3]);
+        }
 
         double beta;
         if (turn == kEnd) {
@@ -822,7 +827,7 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
             const double dq = v[0], inv = 1.0 / dq;
             double alpha = delta * inv;
             alpha = fma(fma(-alpha, dq, delta), inv, alpha);
-            if ((bits & 1u) || !isfinite(dq) || dq <= 0.0 || !isfinite(alpha)) {
+            if ((bits & 1u) || !isfinite(dq) || dq <= 0.0 || !(FS ? fabs(alpha) <= scalar_max<FS>() : isfinite(alpha))) {
                 fl |= kFlagBreakdown;
                 converged = delta <= target;
                 continue;
@@ -941,21 +946,28 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
     if (CL) cluster_barrier();  // nobody's shared memory goes while a peer may still write to it
 }
 
-template <class Real>
+template <class Real, bool FS>
 const void* res_kernel(int threads, bool cluster, int rpt, bool tmem)
 {
     if (cluster)
-        return threads <= 256 ? (const void*)pcg_res_kernel<Real, 256, true, 1, false>
-                              : (const void*)pcg_res_kernel<Real, 512, true, 1, false>;
+        return threads <= 256 ? (const void*)pcg_res_kernel<Real, 256, true, 1, false, FS>
+                              : (const void*)pcg_res_kernel<Real, 512, true, 1, false, FS>;
     if (rpt == 1 && threads <= 256) {
         if constexpr (sizeof(Real) == 8)
-            if (tmem) return (const void*)pcg_res_kernel<Real, 256, false, 1, true>;
-        return (const void*)pcg_res_kernel<Real, 256, false, 1, false>;
+            if (tmem) return (const void*)pcg_res_kernel<Real, 256, false, 1, true, FS>;
+        return (const void*)pcg_res_kernel<Real, 256, false, 1, false, FS>;
     }
     if constexpr (sizeof(Real) == 4)
-        return (const void*)pcg_res_kernel<Real, kResPairThreads, false, 2, true>;  // (never asked for 512 threads)
+        return (const void*)pcg_res_kernel<Real, kResPairThreads, false, 2, true, FS>;  // (never asked for 512 threads)
     else
-        return (const void*)pcg_res_kernel<Real, 512, false, 1, false>;
+        return (const void*)pcg_res_kernel<Real, 512, false, 1, false, FS>;
+}
+template <class Real>
+const void* res_kernel(int threads, bool cluster, int rpt, bool tmem, bool float_sums)
+{
+    if constexpr (sizeof(Real) == 4)
+        if (float_sums) return res_kernel<Real, true>(threads, cluster, rpt, tmem);
+    return res_kernel<Real, false>(threads, cluster, rpt, tmem);
 }
 
 template <class Real>
@@ -970,8 +982,9 @@ ResLimits query_limits(int dev)
         bool cluster, tmem;
     } const kinds[] = {{256, 1, false, false}, {256, 1, false, true}, {256, 1, true, false}, {512, 1, true, false},
                        {sizeof(Real) == 4 ? kResPairThreads : 512, sizeof(Real) == 4 ? 2 : 1, false, false}};
-    for (const auto& kind : kinds) {
-        const void* k = res_kernel<Real>(kind.threads, kind.cluster, kind.rpt, kind.tmem);
+    for (int i = 0; i < 2 * int(sizeof(kinds) / sizeof(kinds[0])); ++i) {
+        const auto& kind = kinds[i / 2];
+        const void* k = res_kernel<Real>(kind.threads, kind.cluster, kind.rpt, kind.tmem, i % 2 != 0);
         int b = 0;
         if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmemLimit) != cudaSuccess ||
             (kind.cluster && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
@@ -994,7 +1007,7 @@ ResLimits query_limits(int dev)
             c.attrs = &a;
             c.numAttrs = 1;
             int k = 0;
-            if (cudaOccupancyMaxActiveClusters(&k, res_kernel<Real>(threads, true, 1, false), &c) != cudaSuccess) {
+            if (cudaOccupancyMaxActiveClusters(&k, res_kernel<Real>(threads, true, 1, false, false), &c) != cudaSuccess) {
                 cudaGetLastError();
                 k = 0;
             }
@@ -1042,7 +1055,8 @@ cudaError_t launch_pcg_res_kernel(const ResPcgArgs<Real>& args, int threads, int
     }
     c.attrs = &at;
     c.numAttrs = 1;
-    return cudaLaunchKernelExC(&c, res_kernel<Real>(threads, cluster > 0, rpt, args.tmem_slots > 0), kargs);
+    return cudaLaunchKernelExC(&c, res_kernel<Real>(threads, cluster > 0, rpt, args.tmem_slots > 0, args.float_sums != 0),
+                                kargs);
 }
 
 template cudaError_t launch_pcg_res_kernel<float>(const ResPcgArgs<float>&, int, int, int, int, cudaStream_t);
