@@ -1547,7 +1547,8 @@ int ensure_block_lists(pk_system* s)
 template <class Real>
 int run_step(pk_system* s, const pk_step_params& p)
 {
-    if (const int rc = ensure_block_lists(s)) return rc;
+    if (!p.explicit_mode)
+        if (const int rc = ensure_block_lists(s)) return rc;
     PK_CHECK(cudaMemsetAsync(s->stats.p, 0, sizeof(pk::DevStats), s->stream));
     // A per-body part-resident layout from an earlier step: its round table for this solve
     // is built on the side stream while the step assembles.
@@ -1662,7 +1663,7 @@ int run_step_graph(pk_system* s, const pk_step_params& p)
         // Everything built lazily (allocations, uploads) must exist before the capture.
         int prc = ensure_batch_parts_any(s);
         if (!prc) prc = ensure_slab_any(s);
-        if (!prc) prc = ensure_block_lists(s);
+        if (!prc && !p.explicit_mode) prc = ensure_block_lists(s);
         if (prc) return prc;
         const bool timing = s->timing;
         const long long launches = s->launches;
