@@ -72,15 +72,18 @@ def measured_peaks():
 
 
 KERNEL_NAMES = {
-    "slab": "pcg_part_kernel (cooperative, one block per part: search directions resident in shared memory, "
-            "full symmetric rows streamed by TMA, block-Jacobi, one exchange per iteration, integrate)",
-    "ring": "pcg_ring_kernel (cooperative: TMA-staged upper BSR rows, L2 gathers of lower blocks and records, "
-            "block-Jacobi, dots, integrate)",
-    "staged": "pcg_kernel (cooperative, TMA-staged tiles)",
-    "plain": "pcg_kernel (cooperative, unstaged)",
-    "batched": "pcg_batch_kernel (cooperative per-body PCG: symmetric BSR SpMV + block-Jacobi + dots + integrate)",
-    "slab-batched": "pcg_slab_kernel with one group of parts per body (per-body CG scalars and exchanges; "
-                    "bodies packed into a few cooperative launches)",
+    "pcg_res_kernel": "pcg_res_kernel (the matrix on chip for the whole solve, block-Jacobi, one exchange per "
+                      "iteration, integrate)",
+    "pcg_part_kernel": "pcg_part_kernel (cooperative, one block per part: search directions resident in shared "
+                       "memory, full symmetric rows streamed by TMA, block-Jacobi, one exchange per iteration, "
+                       "integrate)",
+    "pcg_slab_kernel": "pcg_slab_kernel (cooperative, one group of parts per body or the symmetric stream: search "
+                       "directions resident in shared memory, rows streamed by TMA, per-body CG scalars and exchanges)",
+    "pcg_ring_kernel": "pcg_ring_kernel (cooperative: TMA-staged upper BSR rows, L2 gathers of lower blocks and "
+                       "records, block-Jacobi, dots, integrate)",
+    "pcg_kernel": "pcg_kernel (cooperative, TMA-staged tiles or unstaged)",
+    "pcg_batch_kernel": "pcg_batch_kernel (cooperative per-body PCG: symmetric BSR SpMV + block-Jacobi + dots + "
+                        "integrate)",
 }
 
 
@@ -323,6 +326,7 @@ def run_ours(args, scene, rank, world, local, pg):
             w.step()
         w.synchronize()
         pcg_kernel, pcg_blocks = w.pcg_kernel()
+        launched = w.pcg_launched()
 
         # --- device-resident timed region ---------------------------------
         w.enable_timing(True)
@@ -414,7 +418,7 @@ def run_ours(args, scene, rank, world, local, pg):
         verr = float(np.linalg.norm(vm - vr) / max(np.linalg.norm(vr), 1e-300))
         fp64 = {"steps_per_s": k / (ref_ms / 1e3), "ms_per_step": ref_ms / k, "steps": k,
                 "solve": "one coupled PCG over all bodies, FP64 storage and arithmetic",
-                "pcg_kernel": ref_kernel, "pcg_blocks": ref_blocks, "cg_iterations": ref_stats["iterations"],
+                "pcg_kernel": ref_kernel, "pcg_launched": ref.pcg_launched(), "pcg_blocks": ref_blocks, "cg_iterations": ref_stats["iterations"],
                 "pcg_ms": ref_solve_ms, "assemble_ms": ref_tm["assemble_ms"] / max(1, ref_tm["steps"]),
                 "algorithmic_bytes_per_solve": ref_bytes,
                 "spmv_gbs": ref_achieved,
@@ -431,14 +435,14 @@ def run_ours(args, scene, rank, world, local, pg):
     traffic = None
     tpi = traffic_per_iteration()
     if (tpi and tpi.get("workload") == args.workload and tpi.get("precision") == args.precision
-            and tpi.get("kernel") == pcg_kernel and not batched):
+            and tpi.get("kernel") == launched and not batched):
         traffic = float(tpi["dram_bytes_per_iteration"]) * stats["iterations"]
     return dict(
         value=value, ms_per_step=elapsed_ms / args.steps, e2e_s=e2e_s, n=n, nnz=nnz, nodes=n_nodes,
         iters=stats["iterations"], converged=stats["converged"], flags=stats["flags"], assemble_ms=assemble_ms,
         solve_ms=solve_ms, launches=tm["launches"], achieved=achieved, peak=peak, peak_kind=peak_kind,
         traffic=traffic, clocks=clock, bytes_per_solve=bytes_per_solve, h2d=2 * 12 * n_nodes, d2h=2 * 12 * n_nodes,
-        tuned=tuned, fp64=fp64, batched=batched, pcg_kernel=pcg_kernel, pcg_blocks=pcg_blocks)
+        tuned=tuned, fp64=fp64, batched=batched, pcg_kernel=pcg_kernel, launched=launched, pcg_blocks=pcg_blocks)
 
 
 def reference_sample(args, scene):
@@ -584,8 +588,9 @@ def main():
         traffic_src = ("profiles/pcg_dram_traffic.json: DRAM bytes per CG iteration of an ncu capture of this "
                        "kernel on this workload, times this run's iterations" if r["traffic"] is not None else
                        "no ncu capture of this kernel and workload committed")
-        kernel = KERNEL_NAMES.get(r["pcg_kernel"], r["pcg_kernel"]) + f", {r['pcg_blocks']} blocks"
-        roof = {"bound": "hbm", "achieved": r["achieved"], "peak": r["peak"], "unit": "GB/s",
+        kernel = KERNEL_NAMES.get(r["launched"], r["launched"]) + f", {r['pcg_blocks']} blocks"
+        resident = r["launched"] == "pcg_res_kernel"
+        roof = {"bound": "latency" if resident else "hbm", "achieved": r["achieved"], "peak": r["peak"], "unit": "GB/s",
                 "frac": r["achieved"] / r["peak"], "traffic": r["traffic"], "traffic_source": traffic_src,
                 "kernel": kernel,
                 "peak_source": f"{r['peak_kind']} hbm_gbs (MEASURED_PEAKS.json)",
@@ -594,7 +599,8 @@ def main():
                                  "76U + 4(n+1) + 48n + 264n (FP64)"}
     cfg_out = dict(base_config, dynamic_rows=r["n"], upper_blocks=r["nnz"], cg_iterations=r["iters"],
                    converged=r["converged"], assemble_ms=r["assemble_ms"], pcg_ms=r["solve_ms"],
-                   autotuned_candidate=r["tuned"][0], pcg_kernel=r["pcg_kernel"], pcg_blocks=r["pcg_blocks"],
+                   autotuned_candidate=r["tuned"][0], pcg_kernel=r["pcg_kernel"], pcg_launched=r["launched"],
+                   pcg_blocks=r["pcg_blocks"],
                    batched_per_body_solve=r["batched"],
                    cuda_graph=r["batched"])
     if r["fp64"] is not None:
@@ -608,7 +614,7 @@ def main():
         cfg_out["batched256"] = {
             "workload": bdesc, "steps_per_s": b["value"], "ms_per_step": b["ms_per_step"],
             "e2e_steps_per_s": args.steps / b["e2e_s"], "pcg_ms": b["solve_ms"], "assemble_ms": b["assemble_ms"],
-            "pcg_kernel": b["pcg_kernel"], "pcg_blocks": b["pcg_blocks"], "max_body_cg_iterations": b["iters"],
+            "pcg_kernel": b["pcg_kernel"], "pcg_launched": b["launched"], "pcg_blocks": b["pcg_blocks"], "max_body_cg_iterations": b["iters"],
             "algorithmic_bytes_per_solve": b["bytes_per_solve"], "spmv_gbs": b["achieved"],
             "frac": (b["achieved"] / b["peak"]) if b["achieved"] else None, "cuda_graph": True,
             "gpu_launches": b["launches"], "clocks": b["clocks"]}

@@ -325,6 +325,8 @@ PHYSIK_B200_API int PHYSIK_B200_Autotune(PhysikWorldHandle world, int repeats, d
  * TMA-staged, 2 unstaged, 3 part-resident, 4 batched) or -1; blocks (may be NULL)
  * receives the blocks it ran on. */
 PHYSIK_B200_API int PHYSIK_B200_GetPcgKernel(PhysikWorldHandle world, int* blocks);
+/* The kernel function that solve launched (see pk_system_pcg_launched); "" before the first. */
+PHYSIK_B200_API const char* PHYSIK_B200_GetPcgLaunchedKernel(PhysikWorldHandle world);
 /* The part-resident kernel's stream form in the last step's solve (pk_system_slab_form:
  * 0 full rows, 1 symmetric form, -1 another kernel).  No counterpart in the reference. */
 PHYSIK_B200_API int PHYSIK_B200_GetPcgStreamForm(PhysikWorldHandle world);

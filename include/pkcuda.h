@@ -278,6 +278,12 @@ PKCUDA_API int pk_system_set_refinement(pk_system* sys, int passes);
  * in FP64 too; -1 before the first solve (or a negative PK_ERR_*).
  * blocks (may be NULL) receives the blocks it ran on. */
 PKCUDA_API int pk_system_pcg_kernel(pk_system* sys, int* blocks);
+/* The kernel that the last solve launched, by the name of its function (the numbers above
+ * stand for several): "pcg_res_kernel" (resident), "pcg_part_kernel" (part-resident,
+ * coupled), "pcg_slab_kernel" (part-resident, per body or symmetric stream),
+ * "pcg_ring_kernel", "pcg_kernel" (staged or unstaged), "pcg_batch_kernel"; "" before the
+ * first solve.  A string that is never freed. */
+PKCUDA_API const char* pk_system_pcg_launched(pk_system* sys);
 /* Stream form of the part-resident kernel's layout in the last solve: 0 full symmetric
  * rows, 1 the symmetric form (each in-sub-part block streamed once); -1 when the last
  * solve did not run on the part-resident kernel. */

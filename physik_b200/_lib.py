@@ -98,6 +98,7 @@ _SIGS = {
     "pk_system_adjoint_step": (_i, [_p, C.POINTER(PkStepParams), _p, _p, _p, _p, _p]),
     "pk_system_autotune": (_i, [_p, C.POINTER(PkStepParams), _i, _p, _p]),
     "pk_system_pcg_kernel": (_i, [_p, _p]),
+    "pk_system_pcg_launched": (C.c_char_p, [_p]),
     "pk_system_set_refinement": (_i, [_p, _i]),
     "pk_system_set_connections": (_i, [_p, _i, _p, _p, _p, _p]),
     "pk_system_set_masses": (_i, [_p, _p]),
@@ -187,6 +188,7 @@ _SIGS = {
     "PHYSIK_B200_GetTetCount": (_i, [_p]),
     "PHYSIK_B200_Autotune": (_i, [_p, _i, _p]),
     "PHYSIK_B200_GetPcgKernel": (_i, [_p, _p]),
+    "PHYSIK_B200_GetPcgLaunchedKernel": (C.c_char_p, [_p]),
     "PHYSIK_B200_GetPcgStreamForm": (_i, [_p]),
     "PHYSIK_B200_GetDeviceSystem": (_p, [_p]),
     "pk_system_sphere_contacts": (_i, [_p, _p, C.c_double, _i, _p, _p]),

@@ -985,6 +985,12 @@ PHYSIK_B200_API int PHYSIK_B200_GetPcgKernel(PhysikWorldHandle world, int* block
     return Guard([&] { return w->GetPcgKernel(blocks); }, -1);
 }
 
+PHYSIK_B200_API const char* PHYSIK_B200_GetPcgLaunchedKernel(PhysikWorldHandle world)
+{
+    World* w = AsWorld(world);
+    return w ? w->GetPcgLaunchedKernel() : "";
+}
+
 PHYSIK_B200_API int PHYSIK_B200_GetPcgStreamForm(PhysikWorldHandle world)
 {
     World* w = AsWorld(world);

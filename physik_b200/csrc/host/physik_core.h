@@ -723,6 +723,7 @@ public:
     int Autotune(int repeats, double* bestMs);
     // PCG kernel of the last solve (see pk_system_pcg_kernel) and its block count.
     int GetPcgKernel(int* blocks) const;
+    const char* GetPcgLaunchedKernel() const;  // its function's name (see pk_system_pcg_launched)
     // Stream form of the part-resident kernel in the last solve (pk_system_slab_form).
     int GetPcgStreamForm() const;
 

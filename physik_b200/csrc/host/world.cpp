@@ -1539,6 +1539,11 @@ int World::GetPcgKernel(int* blocks) const
     return pk_system_pcg_kernel(scene->sys, blocks);
 }
 
+const char* World::GetPcgLaunchedKernel() const
+{
+    return scene && scene->sys ? pk_system_pcg_launched(scene->sys) : "";
+}
+
 int World::GetPcgStreamForm() const
 {
     if (!scene || !scene->sys) return -1;

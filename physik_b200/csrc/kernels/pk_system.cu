@@ -270,6 +270,7 @@ struct pk_system {
     int kernel_choice = -1;
     int last_kernel = -1;         // kernel of the last solve (4: batched), blocks it ran on
     int last_blocks = 0;
+    const char* last_launched = "";  // its __global__ function
     int staged_rows = 0;          // rows per staged tile (0: chosen from the grid)
     std::vector<int> h_row_start, h_lts;  // host copies for re-tiling
     // host copies for the adjoint step's assembly of node sensitivities
@@ -536,6 +537,7 @@ int run_pcg_ring(pk_system* s, const pk_step_params& p, int skip_on_flags)
     a.stats = st;
     PK_CHECK(pk::launch_pcg_ring_kernel<Real, Acc>(a, grid, s->stream));
     s->launches += 1;
+    s->last_launched = "pcg_ring_kernel";
     s->last_blocks = grid;
     return PK_OK;
 }
@@ -977,6 +979,7 @@ int run_pcg_part(pk_system* s, const pk_step_params& p, int skip_on_flags)
     PK_CHECK(cudaMemsetAsync(s->part_inbox.p, 0, part_inbox_bytes(s->part_halo, s->part_parts), s->stream));
     PK_CHECK(pk::launch_pcg_part_kernel<Real>(a, s->part_parts, s->stream));
     s->launches += 1;
+    s->last_launched = "pcg_part_kernel";
     s->last_kernel = std::is_same<Real, double>::value ? 0 : 3;
     s->last_blocks = s->part_parts;
     return PK_OK;
@@ -1091,6 +1094,7 @@ int run_pcg_slab(pk_system* s, const pk_step_params& p, int skip_on_flags)
         a.part_body = s->slab_part_body.as<int>();
         PK_CHECK(pk::launch_pcg_slab_kernel<Acc>(a, s->slab_grid, s->stream));
         s->launches += 1;
+        s->last_launched = "pcg_slab_kernel";
         s->last_kernel = bodies ? 5 : 3;
         s->last_blocks = s->slab_parts;
         return PK_OK;
@@ -1146,6 +1150,7 @@ int run_pcg_resident(pk_system* s, const pk_step_params& p, int skip_on_flags)
     PK_CHECK(pk::launch_pcg_res_kernel<Real>(a, s->res_plan.threads, s->res_plan.rpt, s->res_plan.cluster, s->res_parts,
                                              s->stream));
     s->launches += 1;
+    s->last_launched = "pcg_res_kernel";
     s->last_blocks = s->res_parts;
     return PK_OK;
 }
@@ -1258,6 +1263,7 @@ int run_pcg_batch(pk_system* s, const pk_step_params& p, int skip_on_flags)
     a.body_stats = s->body_stats.as<pk::BatchBodyStats>();
     PK_CHECK(pk::launch_pcg_batch_kernel<Real, Acc>(a, grid, s->stream));
     s->launches += 1;
+    s->last_launched = "pcg_batch_kernel";
     s->last_blocks = grid;
     return PK_OK;
 }
@@ -1331,6 +1337,7 @@ int run_pcg(pk_system* s, const pk_step_params& p, int skip_on_flags)
     PK_CHECK(pk::launch_pcg_kernel<Real, Acc>(a, grid, pk::kPcgThreads, s->stream));
     s->launches += 1;
     s->last_kernel = a.ntiles > 0 ? 1 : 2;
+    s->last_launched = "pcg_kernel";
     s->last_blocks = grid;
     return PK_OK;
 }
@@ -2599,6 +2606,8 @@ PKCUDA_API int pk_system_pcg_kernel(pk_system* s, int* blocks)
     if (blocks) *blocks = s->last_blocks;
     return s->last_kernel;
 }
+
+PKCUDA_API const char* pk_system_pcg_launched(pk_system* s) { return s ? s->last_launched : ""; }
 
 PKCUDA_API int pk_system_set_graph(pk_system* s, int on)
 {

@@ -179,6 +179,10 @@ class SimWorld:
         k = self.X.PHYSIK_B200_GetPcgKernel(self.h, C.byref(blocks))
         return self.PCG_KERNELS.get(k, "none"), blocks.value
 
+    def pcg_launched(self) -> str:
+        """The kernel function that the last step's solve launched."""
+        return self.X.PHYSIK_B200_GetPcgLaunchedKernel(self.h).decode()
+
     def pcg_stream_form(self) -> str:
         """Stream form of the part-resident kernel in the last solve: "full", "sym" or "none"."""
         return {0: "full", 1: "sym"}.get(self.X.PHYSIK_B200_GetPcgStreamForm(self.h), "none")
