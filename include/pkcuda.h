@@ -366,6 +366,18 @@ PKCUDA_API int pk_slab_plan_selfcheck(int n, const int* row_start, const int* co
                                       const double* x, const double* coords, int parts, int form, double* y,
                                       int* info);
 
+/* CPU self-check of the coupled part-resident kernel's layout: full symmetric rows in the
+ * precision's stream form (FP64: tiles of half as many rows, headers and columns only), cut
+ * as above, with the lists of the rows that each part sends to the others' windows.  Checks
+ * what the kernel checks before it uses a part or a tile, that every halo row is sent once
+ * and every block placed once, and evaluates y = A x as its lanes read it, the halo from the
+ * rows sent.  info (may be NULL) receives {parts, largest window, most tiles in a part,
+ * stream KiB, halo rows}.  No counterpart in the reference (it checks this library's own
+ * layout). */
+PKCUDA_API int pk_part_plan_selfcheck(int n, const int* row_start, const int* col_index, const double* values,
+                                      const double* x, const double* coords, int parts, int precision, double* y,
+                                      int* info);
+
 /* The same for the per-body (batched) layout: rows in segments (bodies), every body cut
  * into parts that fit, bodies packed into launches of at most max_blocks parts; also
  * checks that every part's group is its body's consecutive parts within one launch.

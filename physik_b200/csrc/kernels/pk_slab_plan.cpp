@@ -1172,4 +1172,135 @@ void slab_spmv_host(const SlabPlan& plan, int nnz, const double* values, const d
     }
 }
 
+namespace {
+// Where a tile's header lies in SlabPlan::stream, and its columns.
+size_t part_tile_at(const SlabPlan& plan, int ti)
+{
+    return plan.wide ? (size_t)kSlabHeaderBytes * ti + 2 * (size_t)plan.tile_entry0[ti]
+                     : 16 * (size_t)plan.tile_desc[4 * (size_t)ti];
+}
+size_t part_cols_at(const SlabPlan& plan, int ti)
+{
+    const size_t ne = plan.tile_entry0[ti + 1] - plan.tile_entry0[ti];
+    return part_tile_at(plan, ti) + kSlabHeaderBytes + (plan.wide ? 0 : 36 * ne);
+}
+}  // namespace
+
+std::string part_check(const SlabPlan& plan, int nnz)
+{
+    if (plan.sym) return "the symmetric form has no sends";
+    const int cap = plan.wide ? kWideCapE : kSlabCapE, rows = plan.wide ? kWideRows : kSlabRows;
+    const int entry = plan.wide ? kWideEntryBytes : kSlabEntryBytes;
+    const int stage = plan.wide ? kWideStageBytes : kSlabStageBytes;
+    const int tiles = static_cast<int>(plan.tile_desc.size() / 4), halo = static_cast<int>(plan.halo_src.size());
+    if (static_cast<int>(plan.tile_entry0.size()) != tiles + 1 ||
+        plan.tile_entry0[tiles] != static_cast<int>(plan.fill_src.size()))
+        return "bad entry lists";
+    if (static_cast<int>(plan.send_start.size()) != plan.parts + 1 || plan.send_start[0] != 0 ||
+        plan.send_start[plan.parts] != halo || static_cast<int>(plan.send.size()) != 2 * halo)
+        return "bad send lists";
+    std::vector<int> owner(plan.n, -1), sent(halo, 0);
+    std::vector<unsigned char> placed(nnz, 0), listed(plan.n, 0);
+    for (int p = 0; p < plan.parts; ++p) {
+        const int* pi = plan.part_info.data() + (size_t)kSlabPartInts * p;
+        if (pi[1] < 0 || pi[1] > kSlabMaxRows || pi[3] < 0 || pi[1] + pi[3] > plan.max_window ||
+            plan.max_window > kSlabWinCap || pi[0] < 0 || pi[0] + pi[1] > plan.n || pi[2] < 0 || pi[2] + pi[3] > halo ||
+            pi[4] < 0 || pi[5] < 0 || pi[4] + pi[5] > tiles || pi[5] > (plan.wide ? kWideMaxTiles : kSlabMaxTiles))
+            return "bad part";
+        for (int g = pi[0]; g < pi[0] + pi[1]; ++g) {
+            if (owner[g] >= 0 || plan.perm[g] < 0 || plan.perm[g] >= plan.n || listed[plan.perm[g]]++) return "a row owned twice";
+            owner[g] = p;
+        }
+    }
+    unsigned long long at = 0;
+    for (int p = 0; p < plan.parts; ++p) {
+        const int* pi = plan.part_info.data() + (size_t)kSlabPartInts * p;
+        int row = 0;
+        for (int ti = pi[4]; ti < pi[4] + pi[5]; ++ti) {
+            const int* d = plan.tile_desc.data() + 4 * (size_t)ti;
+            const int e0 = plan.tile_entry0[ti], ne = plan.tile_entry0[ti + 1] - e0;
+            if (ne <= 0 || ne > cap || ne % 8 != 0 || e0 % 8 != 0 || d[1] != kSlabHeaderBytes + entry * ne || d[1] > stage ||
+                d[1] % 16 != 0 || 16ull * (unsigned long long)d[0] != at || at + d[1] > plan.stream_bytes)
+                return "bad tile";
+            at += d[1];
+            if (d[2] != row || d[3] < 1 || d[3] > rows || d[2] + d[3] > pi[1]) return "bad tile rows";
+            row += d[3];
+            const size_t head = part_tile_at(plan, ti), cols = part_cols_at(plan, ti);
+            if (cols + 2 * (size_t)ne > plan.stream.size()) return "a tile beyond the stream";
+            int last = 0;
+            bool flag = false;
+            for (int i = 0; i < d[3]; ++i) {
+                const int j0 = get_u16(plan.stream, head + 2 * (size_t)i), j1 = get_u16(plan.stream, head + 2 * (size_t)i + 2);
+                if (j0 != last || j1 < j0 || j1 > ne) return "bad row offsets";
+                last = j1;
+                for (int j = j0; j < j1; ++j) {
+                    const unsigned s = plan.fill_src[(size_t)e0 + j], k = s & ~kSlabLowerBit,
+                                   bit = (s & kSlabLowerBit) ? 2u : 1u;
+                    if (s == kSlabNoPos || k >= (unsigned)nnz || (placed[k] & bit)) return "a block placed twice";
+                    placed[k] |= bit;
+                    const int c = get_u16(plan.stream, cols + 2 * (size_t)j);
+                    if (c >= pi[1] + pi[3]) return "a column outside the window";
+                    flag = flag || c >= pi[1];
+                }
+            }
+            for (int j = last; j < ne; ++j)
+                if (plan.fill_src[(size_t)e0 + j] != kSlabNoPos) return "a padding entry with a block";
+            if ((get_u16(plan.stream, head + 2 * (size_t)kSlabHaloWord) != 0) != flag) return "a tile's halo flag";
+        }
+        if (row != pi[1]) return "rows without a tile";
+        for (int e = plan.send_start[p]; e < plan.send_start[p + 1]; ++e) {
+            const int r = plan.send[2 * (size_t)e], place = plan.send[2 * (size_t)e + 1];
+            if (r < 0 || r >= pi[1] || place < 0 || place >= halo || sent[place]++ || plan.halo_src[place] != pi[0] + r)
+                return "a row sent to the wrong place";
+        }
+        for (int i = 0; i < pi[3]; ++i) {
+            const int g = plan.halo_src[pi[2] + i];
+            if (g < 0 || g >= plan.n || owner[g] == p) return "a halo row of the part's own";
+        }
+    }
+    if (at != plan.stream_bytes) return "bytes without a tile";
+    for (int i = 0; i < halo; ++i)
+        if (!sent[i]) return "a halo row nobody sends";
+    for (int k = 0; k < nnz; ++k)
+        if (!(placed[k] & 1)) return "a block not placed";
+    return "";
+}
+
+void part_spmv_host(const SlabPlan& plan, const double* values, const double* x, double* y)
+{
+    // the rows in flight, as their owners send them
+    std::vector<double> rows_in(3 * plan.halo_src.size(), std::nan(""));
+    for (int p = 0; p < plan.parts; ++p)
+        for (int e = plan.send_start[p]; e < plan.send_start[p + 1]; ++e) {
+            const int g = plan.part_info[(size_t)kSlabPartInts * p] + plan.send[2 * (size_t)e];
+            for (int a = 0; a < 3; ++a)
+                rows_in[3 * (size_t)plan.send[2 * (size_t)e + 1] + a] = x[3 * (size_t)plan.perm[g] + a];
+        }
+    for (int p = 0; p < plan.parts; ++p) {
+        const int* pi = plan.part_info.data() + (size_t)kSlabPartInts * p;
+        const int g0 = pi[0], m = pi[1], h = pi[3];
+        std::vector<double> win(3 * (size_t)(m + h));
+        for (int i = 0; i < m + h; ++i)
+            for (int a = 0; a < 3; ++a)
+                win[3 * (size_t)i + a] =
+                    i < m ? x[3 * (size_t)plan.perm[g0 + i] + a] : rows_in[3 * (size_t)(pi[2] + i - m) + a];
+        for (int ti = pi[4]; ti < pi[4] + pi[5]; ++ti) {
+            const int* d = plan.tile_desc.data() + 4 * (size_t)ti;
+            const size_t head = part_tile_at(plan, ti), cols = part_cols_at(plan, ti);
+            for (int i = 0; i < d[3]; ++i) {
+                double* out = y + 3 * (size_t)plan.perm[g0 + d[2] + i];
+                out[0] = out[1] = out[2] = 0.0;
+                const int j1 = get_u16(plan.stream, head + 2 * (size_t)i + 2);
+                for (int j = get_u16(plan.stream, head + 2 * (size_t)i); j < j1; ++j) {
+                    const unsigned s = plan.fill_src[(size_t)plan.tile_entry0[ti] + j];
+                    const double* v = values + 9 * (size_t)(s & ~kSlabLowerBit);
+                    const double* q = win.data() + 3 * (size_t)get_u16(plan.stream, cols + 2 * (size_t)j);
+                    for (int a = 0; a < 3; ++a)
+                        for (int c = 0; c < 3; ++c) out[a] += v[(s & kSlabLowerBit) ? 3 * a + c : 3 * c + a] * q[c];
+                }
+            }
+        }
+    }
+}
+
 }  // namespace pk

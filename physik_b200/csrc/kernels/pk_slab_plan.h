@@ -160,6 +160,15 @@ std::string build_slab_plan_batched(int n, const int* row_start, const int* col,
 // the kernel's clamps), in double: the CPU self-check of a plan.
 void slab_spmv_host(const SlabPlan& plan, int nnz, const double* values, const double* x, double* y);
 
+// The coupled part-resident kernel's layout (full rows, either stream form): the conditions it
+// checks before it uses a part or a tile, that tiles and entry lists lie one after another,
+// that every halo row is sent once, by its owner, to its place, and that every block is placed
+// once (its transpose once, off the diagonal).  "" when they hold.
+std::string part_check(const SlabPlan& plan, int nnz);
+// y = A x through that layout as the kernel's lanes read it (the entries' blocks by the fill
+// list, the window from the rows that are sent), in double.
+void part_spmv_host(const SlabPlan& plan, const double* values, const double* x, double* y);
+
 // The full form's halo order, checked on the host: inside every part the interior rows
 // (every block's column in the part) precede the others, and a tile's header flags a halo
 // column exactly when one of its blocks has its column in the halo.  "" when it holds.

@@ -3132,6 +3132,39 @@ PKCUDA_API int pk_slab_plan_selfcheck(int n, const int* row_start, const int* co
     return PK_OK;
 }
 
+PKCUDA_API int pk_part_plan_selfcheck(int n, const int* row_start, const int* col_index, const double* values,
+                                      const double* x, const double* coords, int parts, int precision, double* y,
+                                      int* info)
+{
+    if (n <= 0 || parts <= 0 || !row_start || !col_index || !values || !x || !y)
+        return fail(PK_ERR_ARG, "part selfcheck");
+    if (row_start[0] != 0) return fail(PK_ERR_ARG, "row_start[0] != 0");
+    for (int r = 0; r < n; ++r) {
+        if (row_start[r + 1] < row_start[r]) return fail(PK_ERR_ARG, "row_start not monotone");
+        for (int k = row_start[r]; k < row_start[r + 1]; ++k) {
+            if (col_index[k] < r || col_index[k] >= n) return fail(PK_ERR_ARG, "column outside [row, n)");
+            if (k > row_start[r] && col_index[k] <= col_index[k - 1]) return fail(PK_ERR_ARG, "columns not sorted");
+        }
+    }
+    std::vector<int> lts, ltr, ltb;
+    build_transpose(n, row_start, col_index, lts, ltr, ltb);
+    pk::SlabPlan plan;
+    std::string why = pk::build_slab_plan(n, row_start, col_index, lts.data(), ltr.data(), ltb.data(), coords, parts,
+                                          plan, pk::kSlabFull, precision == PK_PREC_FP64);
+    if (!why.empty()) return fail(PK_ERR_UNSUPPORTED, "part layout: " + why);
+    why = pk::part_check(plan, row_start[n]);
+    if (!why.empty()) return fail(PK_ERR_STATE, "part layout: " + why);
+    pk::part_spmv_host(plan, values, x, y);
+    if (info) {
+        info[0] = plan.parts;
+        info[1] = plan.max_window;
+        info[2] = plan.max_tiles;
+        info[3] = static_cast<int>(plan.stream_bytes / 1024);
+        info[4] = static_cast<int>(plan.halo_src.size());
+    }
+    return PK_OK;
+}
+
 PKCUDA_API int pk_ring_tiling_selfcheck(int precision, int n, const int* row_start, const int* col_index,
                                         const double* values, const double* x, double* y, int* tiles, int* max_span)
 {
