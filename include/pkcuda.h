@@ -340,6 +340,16 @@ PKCUDA_API const char* pk_pcg_noalloc_last_error(void);
  * missing > 0) -- the launch still ends normally and the context stays usable.  No
  * counterpart in the reference (it checks this library's failure path). */
 PKCUDA_API int pk_exchange_wait_selftest(int device, int blocks, int missing, unsigned long long limit, double* out);
+/* The same for the exchange of tagged packets (resident and part-resident kernels): out
+ * receives 4 doubles per block {completed, two sums, a shared-memory word that nothing sets
+ * was seen}; every wait gives up after `limit` polls. */
+PKCUDA_API int pk_tag_wait_selftest(int device, int blocks, int missing, unsigned limit, double* out);
+/* One solve of a fixed band system (700 rows: 20 I on the diagonal, -I towards the next five
+ * rows, right-hand side sin(3 r + component)) in double on four blocks of the resident kernel
+ * (kernel 0), of its cluster form (1) or of the part-resident kernel (2).  With `lost` the
+ * first part sends none of its rows: the waits for them give up after `limit` polls and the
+ * solve returns PK_ERR_TIMEOUT.  x receives 3 x 700 doubles. */
+PKCUDA_API int pk_pcg_wait_selftest(int device, int kernel, int lost, unsigned limit, double* x, int* iterations);
 
 /* Host-only consistency check of the ring-staged PCG kernel's tiling (no device needed):
  * builds its tiles for the upper BSR (values 9 per block, x 3 per row), replays the

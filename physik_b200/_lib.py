@@ -121,6 +121,8 @@ _SIGS = {
     "PHYSIK_SetNodeFixed": (_v, [_p, _i, _i]),
     "PHYSIK_IsNodeFixed": (_i, [_p, _i]),
     "pk_exchange_wait_selftest": (_i, [_i, _i, _i, C.c_ulonglong, _p]),
+    "pk_tag_wait_selftest": (_i, [_i, _i, _i, C.c_uint, _p]),
+    "pk_pcg_wait_selftest": (_i, [_i, _i, _i, C.c_uint, _p, _p]),
     "PHYSIK_GenerateTetMesh": (_p, [_p, _i, _p, _i]),
     "PHYSIK_IsGeneratedTetMeshHandleValid": (_i, [_p]),
     "PHYSIK_DestroyGeneratedTetMesh": (_v, [_p]),

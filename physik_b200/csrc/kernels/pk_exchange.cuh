@@ -125,7 +125,6 @@ constexpr int kTagSums = 4;
 constexpr int kTagSlotBytes = 16 * kTagSums;
 constexpr int kTagMaxGroup = 160;
 constexpr int kTagPoll = kTagMaxGroup / 32;
-constexpr unsigned kTagSpinLimit = 1u << 22;  // polls of one wait: seconds
 struct TagShared {
     double part[2][kTagSums * 16];  // the warps' partials, by exchange parity
     double sum[2][kTagSums];
@@ -194,7 +193,7 @@ __device__ __forceinline__ void tag_publish(unsigned char* inbox, int size, int 
 // four of eight or more warps (all of four) read one sum each, lane i of them the members i, i + 32, ...
 __device__ __forceinline__ bool tag_finish(const unsigned char* inbox, int size, int me, unsigned gen,
                                            double (&v)[kTagSums], unsigned& bits, unsigned* flags, TagTeam team,
-                                           TagShared& sh, unsigned long long limit = kTagSpinLimit)
+                                           TagShared& sh, unsigned limit)
 {
     if (size <= 1) return sh.fail == 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = team.warps;
@@ -248,17 +247,17 @@ __device__ __forceinline__ bool tag_finish(const unsigned char* inbox, int size,
 }
 __device__ __forceinline__ bool tag_exchange(unsigned char* inbox, int size, int me, unsigned gen, double (&v)[kTagSums],
                                              unsigned& bits, int value_warps, unsigned* flags, TagTeam team, TagShared& sh,
-                                             unsigned long long limit = kTagSpinLimit)
+                                             unsigned limit)
 {
     tag_publish(inbox, size, me, gen, v, bits, value_warps, team, sh);
     return tag_finish(inbox, size, me, gen, v, bits, flags, team, sh, limit);
 }
 
 // Waits (bounded) until the shared-memory word holds `want`; false when it gave up.
-__device__ __forceinline__ bool wait_shared(const int* flag, int want)
+__device__ __forceinline__ bool wait_shared(const int* flag, int want, unsigned long long limit = kBarrierSpinLimit)
 {
     for (unsigned long long spins = 0; *(const volatile int*)flag != want; ++spins) {
-        if (spins > kBarrierSpinLimit) return false;
+        if (spins > limit) return false;
         __nanosleep(32);
     }
     __threadfence_block();

@@ -414,6 +414,9 @@ struct SlabPcgArgs {
     int sym;
 };
 
+// Polls of one wait of the part-resident and resident kernels for another block: seconds.
+constexpr unsigned kTagSpinLimit = 1u << 22;
+
 // ------------------------------------------------------------------ part-resident PCG, coupled
 // pk_pcg_part.cu: the window, a ring of as many stages as fit, the table.
 constexpr size_t kPartSmemLimit = 224 * 1024;
@@ -442,6 +445,7 @@ struct PartPcgArgs {
     unsigned long long stream_bytes;
     int stages, win_cap;
     unsigned ring_offset;
+    unsigned spin_limit;         // polls of one wait for another block
     unsigned char* rows_in;      // a packet (FP64: two) per halo row; zero at launch
     unsigned char* sums_in;      // the blocks' inboxes; zero at launch
     const int* perm;             // slab index -> dynamic row
@@ -502,6 +506,7 @@ struct ResPcgArgs {
     unsigned char* sums_in;          // [2][grid][sender] x kResSlotBytes: tagged sums
     size_t sums_stride;              // bytes of one block's inbox: the largest group's senders
     unsigned* epoch;                 // [grid] tag base of the group starting at each block
+    unsigned spin_limit;             // polls of one wait for another block
     int float_sums;                  // FP32 systems: the sums (in double) are judged as floats
     int max_iterations;
     double tolerance;

@@ -63,7 +63,6 @@ namespace {
 constexpr int kResMaxWarps = kResMaxThreads / 32;
 constexpr int kResSums = 4;  // d.q, q.s + r.z, q.z, r.s; at the end r.r in the first
 constexpr int kResSendRegs = 2;
-constexpr unsigned kResSpinLimit = 1u << 22;  // polls of one wait: seconds
 
 // ------------------------------------------------------------------ cluster exchange
 __device__ __forceinline__ unsigned cluster_map(const void* p, unsigned rank)
@@ -101,9 +100,9 @@ constexpr unsigned row_tx_bytes()
     return sizeof(Real) == 4 ? 16 : 24;
 }
 // Bounded wait for the phase with the given parity, seeing what cluster peers wrote.
-__device__ __forceinline__ bool cluster_wait(unsigned long long* bar, unsigned parity)
+__device__ __forceinline__ bool cluster_wait(unsigned long long* bar, unsigned parity, unsigned limit)
 {
-    for (unsigned i = 0; i < kMbarSpinLimit; ++i) {
+    for (unsigned i = 0; i < limit; ++i) {
         unsigned ok;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -661,7 +660,7 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
                 }
             }
             if (CL && gsize > 1) {
-                if (!cluster_wait(&sh_bar[gen & 1u], ((gen - 1u) >> 1) & 1u)) s_fail = 1;
+                if (!cluster_wait(&sh_bar[gen & 1u], ((gen - 1u) >> 1) & 1u, P.spin_limit)) s_fail = 1;
                 __syncthreads();
                 const unsigned char* in = sums_in + (size_t)(gen & 1u) * kResMaxCluster * kResSlotBytes +
                                           16 * (lane >> 3);
@@ -726,7 +725,7 @@ __global__ void __launch_bounds__(MAXT, 1) pcg_res_kernel(ResPcgArgs<Real> P)
                     for (int j = 0; j < kResSlotPoll; ++j)
                         if (((todo >> j) & 1u) && packet_tag(pk[j]) == tag) got |= 1u << j;
                     todo &= ~got;
-                    if (spins > kResSpinLimit) {
+                    if (spins > P.spin_limit) {
                         atomicOr(P.flags, kFlagBarrierTimeout);
                         s_fail = 1;
                         break;

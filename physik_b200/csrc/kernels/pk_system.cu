@@ -967,6 +967,7 @@ int run_pcg_part(pk_system* s, const pk_step_params& p, int skip_on_flags)
     a.max_iterations = p.max_iterations;
     a.tolerance = static_cast<double>(static_cast<Real>(p.tolerance));
     a.float_sums = s->precision == PK_PREC_FP32 ? 1 : 0;
+    a.spin_limit = pk::kTagSpinLimit;
     a.skip_on_flags = skip_on_flags;
     a.integrate = p.integrate;
     a.dt = static_cast<Real>(p.dt);
@@ -1135,6 +1136,7 @@ int run_pcg_resident(pk_system* s, const pk_step_params& p, int skip_on_flags)
     a.max_iterations = p.max_iterations;
     a.tolerance = static_cast<double>(static_cast<Real>(p.tolerance));
     a.float_sums = s->precision == PK_PREC_FP32 ? 1 : 0;
+    a.spin_limit = pk::kTagSpinLimit;
     a.skip_on_flags = skip_on_flags;
     a.integrate = p.integrate;
     a.dt = static_cast<Real>(p.dt);
