@@ -21,7 +21,8 @@
 // A launch exchanges in one of two ways.  Groups of at most kResMaxCluster blocks run as
 // thread-block clusters of `cluster` blocks (a group never straddles two; blocks a cluster
 // has left over have no part) and write into each other's shared memory; such a launch may
-// have more clusters than fit the GPU at once, since clusters do not wait for each other.
+// have more clusters than fit the GPU at once, since clusters do not wait for each other
+// (the runtime asks for a layout only where the whole matrix is within the SMs' memory).
 // Larger groups exchange through global memory and must all be resident (cluster = 0, a
 // cooperative launch).
 // Plain C++ (no CUDA), shared by the runtime and its CPU self-check.

@@ -653,10 +653,15 @@ int ensure_resident(pk_system* s, bool bodies)
     }
     const int grid = limits.blocks;
     const int n = s->dyn_count;
-    // Blocks of a row before padding: a matrix that cannot fit is refused without a layout.
+    // A matrix above the SMs' memory is refused without a layout.  A coupled one cannot fit; a
+    // batch could still run as clusters in waves, which the rule leaves to the stream because
+    // neither is the better one throughout (ms a solve, stream / waves: 300 bodies of 650 rows
+    // 2.35 / 1.71, 1,500 of 360 5.50 / 3.12, 600 of 640 2.92 / 3.47, 150 of 3,900 3.69 / 4.90,
+    // 600 of 1,570 4.89 / 6.85).  (Blocks of a row before padding.)
     const size_t entries = 2 * static_cast<size_t>(s->nnz);
-    if (grid <= 0 || entries > static_cast<size_t>(n) &&
-                         (entries - n) * (9 * sizeof(Real) + 2) > static_cast<size_t>(grid) * 2 * pk::kResSmemLimit)
+    if (grid <= 0 ||
+        (entries > static_cast<size_t>(n) &&
+         (entries - n) * (9 * sizeof(Real) + 2) > static_cast<size_t>(grid) * 2 * pk::kResSmemLimit))
         return PK_OK;
     LayoutInputs in;
     int rc = layout_inputs<Real>(s, in);
