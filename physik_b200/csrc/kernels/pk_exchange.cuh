@@ -193,7 +193,7 @@ __device__ __forceinline__ void tag_publish(unsigned char* inbox, int size, int 
 // four of eight or more warps (all of four) read one sum each, lane i of them the members i, i + 32, ...
 __device__ __forceinline__ bool tag_finish(const unsigned char* inbox, int size, int me, unsigned gen,
                                            double (&v)[kTagSums], unsigned& bits, unsigned* flags, TagTeam team,
-                                           TagShared& sh, unsigned limit)
+                                           TagShared& sh, unsigned limit = kTagSpinLimit)
 {
     if (size <= 1) return sh.fail == 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = team.warps;
@@ -247,7 +247,7 @@ __device__ __forceinline__ bool tag_finish(const unsigned char* inbox, int size,
 }
 __device__ __forceinline__ bool tag_exchange(unsigned char* inbox, int size, int me, unsigned gen, double (&v)[kTagSums],
                                              unsigned& bits, int value_warps, unsigned* flags, TagTeam team, TagShared& sh,
-                                             unsigned limit)
+                                             unsigned limit = kTagSpinLimit)
 {
     tag_publish(inbox, size, me, gen, v, bits, value_warps, team, sh);
     return tag_finish(inbox, size, me, gen, v, bits, flags, team, sh, limit);

@@ -442,8 +442,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_part_kernel(const __grid_
         for (int e = rt + 2 * kOwners; e < sends_n; e += kOwners) push(__ldg(P.send + send0 + e));
     };
     auto exchange = [&](double (&v)[kTagSums], unsigned& bits) {
-        const bool ok = tag_exchange(P.sums_in, (int)gridDim.x, blk, ++xgen, v, bits, kConsumerWarps, P.flags, team, sh,
-                                     P.spin_limit);
+        const bool ok = tag_exchange(P.sums_in, (int)gridDim.x, blk, ++xgen, v, bits, kConsumerWarps, P.flags, team, sh);
         if constexpr (FS) {
             v[0] = as_float_sum(v[0]);
             v[3] = as_float_sum(v[3]);
