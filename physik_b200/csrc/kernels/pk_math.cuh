@@ -177,12 +177,12 @@ __host__ __device__ inline M3<T> polar_rotation(const M3<T>& f, int* iterations,
             const V3<T> d = next.c[col] - r.c[col];
             diff += dot(d, d);
         }
-        // The identity exits, off the common path.  With 0.01 < |det r| < 100 and r^-T within 4
+        // The identity exits, off the common path.  With |det r| > 0.01 and r^-T within 4
         // (Frobenius) of r, every row of r is below 4.5 (its product with the same row of r^-T
-        // is 1 up to rounding), so the determinant of r^-T is 1 / det r to 0.2 % in float, far
-        // above the limit, and nothing is infinite or NaN.  A bound on det r alone does not do:
-        // at conditions above 1e6 the two determinants need not agree.
-        if (!(fabs(dr) > T(0.01) && fabs(dr) < T(100)) || !(diff <= T(4))) {
+        // is 1 up to rounding), so |det r| < 92, the determinant of r^-T is 1 / det r to 0.2 % in
+        // float, far above the limit, and nothing is infinite or NaN.  A bound on det r alone
+        // does not do: at conditions above 1e6 the two determinants need not agree.
+        if (!(fabs(dr) > T(0.01) && diff <= T(4))) {
             if (!finite9(ti) || fabs(det(ti)) <= min_det || !finite9(next)) {
                 *fallback = true;
                 return mident<T>();
