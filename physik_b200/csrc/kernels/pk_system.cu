@@ -253,6 +253,18 @@ struct pk_system {
     DevBuf slab_qs, slab_ss;
     // coupled part-resident PCG (pk_pcg_part.cu): shares the buffers above
     bool wide_tried = false;
+    // FP64 layouts of patterns with transient blocks (layout_waits)
+    bool nodes_solved = false;    // a solve ran since the nodes were set
+    bool replaced = false;        // the pattern replaced one that had been solved
+    int pattern_solves = 0;       // solves on this pattern
+    bool waited = false;          // some of them without the layout it may get
+    // The pattern of the FP64 layout last built, whose buffers stay as they are while another
+    // pattern waits, so that a pattern which returns needs no second build.
+    struct {
+        bool valid = false;
+        int res_parts = 0, part_parts = 0;
+        std::vector<int> row_start, col, dyn_to_node;
+    } kept;
     int part_parts = 0, part_window = 0, part_halo = 0;
     DevBuf part_send, part_send_start, part_inbox, part_mrow;
     // resident PCG (pk_pcg_res.cu): the layout where the whole matrix fits on chip
@@ -557,6 +569,7 @@ void reset_slab(pk_system* s)
     s->res_parts = 0;
     s->wide_tried = false;
     s->part_parts = 0;
+    s->kept.valid = false;
 }
 
 // Copies the assembled upper blocks (and their transposes) into the slab stream.
@@ -637,6 +650,37 @@ bool resident_allowed(const pk_system* s)
     return s->precision == PK_PREC_FP64 ? rk == -1 : (rk == -1 || rk == 3) && requested_slab_form() == pk::kSlabFull;
 }
 
+// A pattern with the blocks of connections or host-emitted contributions that replaces a solved
+// one may last a frame (a drag, contacts), and a layout takes the host 0.2 to 0.7 us a row: an
+// FP64 step with new connections at 36 k rows took 29.9 ms with the layout against 3.4 on the ring
+// kernel, which needs none; at 18 k rows 6.6 against 3.4, at 648 0.84 against 0.62.  Such a
+// pattern is first solved on the ring kernel, about as many times as the layout is worth (it
+// saves 10 to 20 us an iteration).  The bodies' own pattern never waits, so that a solve does not depend on
+// the steps before it; FP32 storage has no kernel as fast without a layout.
+bool layout_waits(const pk_system* s)
+{
+    return s->precision == PK_PREC_FP64 && s->replaced && (s->conn_count > 0 || s->ext_on) &&
+           s->pattern_solves <= s->dyn_count / 8192;
+}
+
+// The current pattern (columns `col`) is the one whose layout is kept, and it may have one.
+bool layout_returns(const pk_system* s, const int* col)
+{
+    return s->kept.row_start == s->h_row_start && s->kept.dyn_to_node == s->h_dyn_to_node &&
+           std::equal(s->kept.col.begin(), s->kept.col.end(), col) && requested_kernel() == -1 &&
+           (s->kept.res_parts > 0 ? resident_allowed(s) : s->kernel_choice <= 0);
+}
+// An FP64 layout's buffers hold the current pattern's (of the columns `col`).
+void keep_layout(pk_system* s, std::vector<int>& col)
+{
+    s->kept.res_parts = s->res_parts;
+    s->kept.part_parts = s->part_parts;
+    s->kept.row_start = s->h_row_start;
+    s->kept.dyn_to_node = s->h_dyn_to_node;
+    s->kept.col.swap(col);
+    s->kept.valid = true;
+}
+
 // Builds and uploads the resident kernel's layout (one group per body when `bodies`) if it
 // has not been tried yet; where it does not apply res_parts stays 0.  Synchronous.
 template <class Real>
@@ -663,6 +707,7 @@ int ensure_resident(pk_system* s, bool bodies)
         (entries > static_cast<size_t>(n) &&
          (entries - n) * (9 * sizeof(Real) + 2) > static_cast<size_t>(grid) * 2 * pk::kResSmemLimit))
         return PK_OK;
+    s->kept.valid = false;
     LayoutInputs in;
     int rc = layout_inputs<Real>(s, in);
     if (rc) return rc;
@@ -708,6 +753,7 @@ int ensure_resident(pk_system* s, bool bodies)
     s->res_plan.max_group = plan.max_group;
     s->res_plan.max_halo = plan.max_halo;
     s->res_plan.smem_bytes = plan.smem_bytes;
+    if (sizeof(Real) == 8) keep_layout(s, in.col);
     return PK_OK;
 }
 
@@ -896,6 +942,7 @@ int ensure_wide(pk_system* s)
     grid = std::min(grid, std::max(1, s->dyn_count / 64));
     const int n = s->dyn_count;
     if (grid <= 0 || n > static_cast<long long>(grid) * pk::kSlabMaxRows) return PK_OK;
+    s->kept.valid = false;
     LayoutInputs in;
     int rc = layout_inputs<double>(s, in);
     if (rc) return rc;
@@ -933,6 +980,7 @@ int ensure_wide(pk_system* s)
     if (rc) return rc;
     PK_CHECK(cudaStreamSynchronize(s->stream));
     s->part_parts = plan.parts;
+    keep_layout(s, in.col);
     return PK_OK;
 }
 
@@ -996,6 +1044,10 @@ int ensure_slab_any(pk_system* s)
     if (s->precision == PK_PREC_FP32) return ensure_slab<float>(s);
     if (s->precision == PK_PREC_MIXED) return ensure_slab<double>(s);
     if (batched_solve(s)) return PK_OK;
+    if (layout_waits(s)) {
+        s->waited = true;
+        return PK_OK;
+    }
     const int rc = ensure_resident<double>(s, false);
     return rc ? rc : ensure_wide(s);
 }
@@ -1314,9 +1366,10 @@ int run_pcg(pk_system* s, const pk_step_params& p, int skip_on_flags)
         int rc = ensure_slab<Acc>(s);
         if (rc) return rc;
     } else {
-        int rc = ensure_resident<double>(s, false);
-        if (!rc) rc = ensure_wide(s);
+        const int rc = ensure_slab_any(s);
         if (rc) return rc;
+        ++s->pattern_solves;
+        s->nodes_solved = true;
     }
     const int kernel = solve_kernel(s);
     s->last_kernel = kernel;
@@ -1672,6 +1725,12 @@ int run_step_graph(pk_system* s, const pk_step_params& p)
         drop_graph(s);
         return run_step<Real>(s, p);
     }
+    // (a step captured while its layout waited is captured again with it)
+    if (s->waited && !layout_waits(s)) {
+        s->waited = false;
+        drop_graph(s);
+    }
+    const int solves = s->pattern_solves + (p.explicit_mode || s->precision != PK_PREC_FP64 ? 0 : 1);
     if (!s->graph_exec || !same_params(p, s->graph_params)) {
         drop_graph(s);
         // Everything built lazily (allocations, uploads) must exist before the capture.
@@ -1719,6 +1778,7 @@ int run_step_graph(pk_system* s, const pk_step_params& p)
     }
     s->launches += s->graph_kernels;
     s->stats_pending = true;
+    s->pattern_solves = solves;  // (a capture counts its solve too)
     return PK_OK;
 }
 
@@ -1862,6 +1922,8 @@ PKCUDA_API int pk_system_set_nodes(pk_system* s, int node_count, const int* node
     PK_CHECK(cudaSetDevice(s->device));
     s->node_count = node_count;
     s->have_layout_x = false;
+    s->nodes_solved = false;
+    s->kept.valid = false;
     s->have_snapshot = false;
     s->h_node_to_dyn.assign(node_to_dyn, node_to_dyn + node_count);
     s->lists_ok = s->lists_tried = false;
@@ -2346,6 +2408,9 @@ PKCUDA_API int pk_system_set_pattern(pk_system* s, int dyn_count, const int* dyn
     s->lt_count = static_cast<int>(ltr.size());
     s->inc_count = inc;
     s->lists_ok = s->lists_tried = false;
+    s->replaced = s->nodes_solved;
+    s->pattern_solves = 0;
+    s->waited = false;
     s->max_row = max_row;
     s->diag_first = diag_first;
     int rc = upload_raw<int>(s->dyn_to_node, dyn_to_node, dyn_count, s->stream);
@@ -2375,7 +2440,14 @@ PKCUDA_API int pk_system_set_pattern(pk_system* s, int dyn_count, const int* dyn
     s->h_row_start.assign(row_start, row_start + dyn_count + 1);
     s->h_dyn_to_node.assign(dyn_to_node, dyn_to_node + dyn_count);
     s->h_lts = lts;
+    const bool kept = s->kept.valid;
     reset_slab(s);
+    s->kept.valid = kept;
+    if (kept && layout_returns(s, col_index)) {
+        s->res_tried = s->wide_tried = true;
+        s->res_parts = s->kept.res_parts;
+        s->part_parts = s->kept.part_parts;
+    }
     // Ring-staged PCG tiles (the kernel used where the part-resident one does not apply).
     s->ring_tiles = 0;
     const int rk = requested_kernel();
@@ -2665,6 +2737,7 @@ PKCUDA_API int pk_system_autotune(pk_system* s, const pk_step_params* p, int rep
         return fail(PK_ERR_STATE, "autotune needs an assembled system (step once first)");
     PK_CHECK(cudaSetDevice(s->device));
     if (const int rc = fetch_stats(s)) return rc;  // the timed solves overwrite them
+    s->replaced = false;  // the candidates are those of a pattern that stays
     PK_CHECK(cudaStreamSynchronize(s->stream));
     drop_graph(s);
     repeats = std::max(1, repeats);
