@@ -1734,10 +1734,12 @@ int run_step_graph(pk_system* s, const pk_step_params& p)
     if (!s->graph_exec || !same_params(p, s->graph_params)) {
         drop_graph(s);
         // Everything built lazily (allocations, uploads) must exist before the capture.
-        int prc = ensure_batch_parts_any(s);
-        if (!prc) prc = ensure_slab_any(s);
-        if (!prc && !p.explicit_mode) prc = ensure_block_lists(s);
-        if (prc) return prc;
+        if (!p.explicit_mode) {
+            int prc = ensure_batch_parts_any(s);
+            if (!prc) prc = ensure_slab_any(s);
+            if (!prc) prc = ensure_block_lists(s);
+            if (prc) return prc;
+        }
         const bool timing = s->timing;
         const long long launches = s->launches;
         s->timing = false;

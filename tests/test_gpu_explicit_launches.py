@@ -1,5 +1,6 @@
 """An explicit step launches its two kernels and nothing else (GPU): the block lists that
-implicit steps read are not built for it, and are once an implicit step follows."""
+implicit steps read and the solve's layout are not built for it, and are once an implicit step
+follows."""
 import pytest
 
 from physik_b200 import meshes
@@ -10,9 +11,11 @@ pytest.importorskip("physik_b200._lib")
 from physik_b200.world import SimWorld  # noqa: E402
 
 
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
 @pytest.mark.parametrize("graph", [False, True])
-def test_an_explicit_step_is_two_launches(graph):
-    w = SimWorld(meshes.small_box(4, 3, 2), precision="fp32", implicit=False)
+def test_an_explicit_step_is_two_launches(graph, precision, monkeypatch):
+    monkeypatch.setenv("PK_PCG_RESIDENT", "0")  # (the part kernel's FP64 layout is a launch)
+    w = SimWorld(meshes.small_box(4, 3, 2), precision=precision, implicit=False)
     w.prepare(True)
     w.set_graph(graph)
     w.enable_timing(True)
