@@ -1,20 +1,27 @@
 // pk_kernels.cu -- sm_100a kernels of PhysiK's implicit soft-body step.
 //
-//   tet_kernel   per tet: F = Ds * DmInv, polar rotation R, corotated stress; stores
-//                R and S = R * V * sigma so that node a's elastic force is -S g_a.
+//   tet_kernel   per tet: F = Ds * DmInv, polar rotation R, corotated stress; stores the
+//                corners' P = sqrt(V mu) R g, from which blocks are built, and their part of the
+//                right-hand side, or the explicit step's forces (TetView::rec).
 //                (FEMModel::ComputeCorotationalElasticForces, FEMModel.cpp:635-679;
 //                 ExtractRotationPolar :115-163; ComputeElasticForcesAndStiffness :377-424)
-//   row_kernel   per dynamic row: gathers its tets (incidence list, tet order), builds the
-//                row's upper blocks dt^2 * sum R Ke_ab R^T (+ m I on the diagonal), the
-//                right-hand side dt*(f + m g) - dt^2 * sum K_ab v_b, and the block-Jacobi
-//                inverse of its diagonal block.  Deterministic: one thread owns a row and
-//                sums in tet order, no atomics.
+//   block_list_kernel, block_rows_kernel
+//                after a pattern change, per stored block its tets and corner pairs; then each
+//                step a thread per off-diagonal block and four lanes per row: the upper blocks
+//                dt^2 * sum R Ke_ab R^T (+ m I on the diagonal), the right-hand side
+//                dt*(f + m g) - dt^2 * sum K_ab v_b, and the block-Jacobi inverse of the
+//                diagonal block.  Deterministic: fixed orders, no atomics.
 //                (TetMeshPhysicsComponent::UpdateSystem, TetMeshPhysicsComponent.cpp:293-354;
 //                 SolverData::AssembleImplicitMatrixAndRhs, SolverData.cpp:308-465;
 //                 SolverData::BuildInversePreconditioner, SolverData.cpp:260-306)
+//   row_kernel   the same with one thread per row over its tets, where there are no lists.
+//   extra_rows_kernel
+//                connections and host-emitted contributions added to the rows.
+//   explicit_row_kernel
+//                the explicit step from the tets' forces (World::IntegrateExplicitEuler).
 //   spmv_kernel  y = A x for the upper-stored symmetric BSR (SparseBlockMatrix::Multiply,
 //                SparseBlockMatrix.cpp:209-268).
-// The PCG kernel lives in pk_pcg.cu.
+// The PCG kernels live in pk_pcg*.cu.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -939,7 +946,7 @@ __global__ void embedded_vertex_kernel(const int* __restrict__ nodes, const floa
 }
 
 // ------------------------------------------------------------------ row kernel
-// The rows without block lists (kept for comparisons): one thread per row over its tets.
+// The rows without block lists (which found no room or do not apply): one thread per row over its tets.
 // MAXU > 0: accumulate the row's upper blocks in shared memory (MAXU slots per thread and the
 // diagonal's other three partial sums, joined as the block-list kernel joins them); MAXU == 0:
 // accumulate in place in the values array (rows of any length).

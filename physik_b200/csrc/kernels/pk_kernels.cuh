@@ -67,12 +67,13 @@ struct TetView {
     const Real* dm_inv;              // 9 per tet, column-major
     const Real* params;              // 4 per tet: rest volume, lambda, mu, damping
     // tet_rec() values per tet, written by the tet kernel each step and read by the row
-    // kernels (one aligned record per tet): four corners of four values P_k = R g_k and V
-    // lambda, then four of B_k and V mu, with B_k = T g_k - dt c v_k the tet's right-hand side
-    // at corner k (T = -(dt S + dt^2 Q), S = R V sigma, Q g_a the tet's sum_b K_ab v_b); in
-    // FP64 then g_a.g_b (10) and R R^T (6).  A tet that is not folded so has NaN in place of
-    // P_k's V lambda, and its form in place of B_0's V mu: kFormForces, B_k = -S g_k (V lambda
-    // and V mu in B_1 and B_3); kFormPlain (FP32, a rotation whose iteration ran out), R in
+    // kernels (one aligned record per tet): four corners of four values P_k = sqrt(V mu) R g_k
+    // and lambda / mu, then four of B_k and 0, with B_k = T g_k - dt c v_k the tet's right-hand
+    // side at corner k (T = -(dt S + dt^2 Q), S = R V sigma, Q g_a the tet's sum_b K_ab v_b); in
+    // FP64 then V mu g_a.g_b (10) and R R^T (6).  A tet that is not folded so has NaN in place
+    // of every lambda / mu, and its form in place of B_0's 0: kFormForces, B_k = -S g_k (lambda
+    // / mu in place of the other zeros); kFormPlain (blocks that might overflow, V mu too small
+    // for its root, lambda / mu too large, or in FP32 a rotation whose iteration ran out), R in
     // the first three corners and S in the next three; kFormSkip, no part in this step.
     // Explicit step: kTetForces values per tet, four corners of the force -S g_k and the damping.
     Real* rec;

@@ -35,8 +35,8 @@
 //   go on from solve to solve (epoch), so nothing is cleared between solves.
 //
 // Measured per CG iteration against the streaming kernels (part-resident stream for FP32
-// storage, ring for FP64): 8x8x8 box FP32 1.8 us (7.2), 32x8x8 beam FP64 3.0 us (13.3),
-// 64x16x16 beam 3.3 us mixed (10.9) and 4.2 us FP64 (18.5), 61x47x29 block mixed (594 rows a
+// storage, ring for FP64): 8x8x8 box FP32 2.3 us (7.2), 32x8x8 beam FP64 3.0 us (13.3),
+// 64x16x16 beam 3.5 us mixed (10.9) and 4.3 us FP64 (18.5), 61x47x29 block mixed (594 rows a
 // part) 7.0 us (19.3).  What is left is a chain of
 // latencies: about 3,000 cycles of a block's own work (product, two sets of FP64 sums by
 // shuffles, the scalars, the updates; 8.6 cycles an FP64 add, 24 a shuffle, 45 a barrier of
