@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <new>
 #include <numeric>
 
 #include "pk_slab_plan.h"
@@ -188,7 +189,7 @@ std::string build_cut(int n, const int* row_start, const int* col, const int* lt
         std::sort(halo.begin(), halo.end());
         halo.erase(std::unique(halo.begin(), halo.end()), halo.end());
     });
-    if (failed) return "host memory exhausted while building the layout";
+    if (failed) return kNoMemory;
     out.part_info.assign((size_t)kResPartInts * parts, 0);
     for (int p = 0; p < parts; ++p) {
         int* pi = out.part_info.data() + (size_t)kResPartInts * p;
@@ -263,7 +264,7 @@ std::string build_cut(int n, const int* row_start, const int* col, const int* lt
             }
         }
     });
-    if (failed) return "host memory exhausted while building the layout";
+    if (failed) return kNoMemory;
     // 6. who sends which row where
     std::vector<std::vector<int>> sends(parts);
     for (int p = 0; p < parts; ++p) {
@@ -288,7 +289,7 @@ std::string build_cut(int n, const int* row_start, const int* col, const int* lt
 std::string build_res_plan(int n, const int* row_start, const int* col, const int* lt_start, const int* lt_row,
                            const int* lt_block, const double* coords, const int* seg, int nseg,
                            const ResLimits& limits, int real, ResPlan& out)
-{
+try {
     out = ResPlan{};
     if (n <= 0 || nseg <= 0 || limits.blocks <= 0 || seg[0] != 0 || seg[nseg] != n) return "empty system";
     std::vector<double> held;
@@ -359,6 +360,8 @@ std::string build_res_plan(int n, const int* row_start, const int* col, const in
         if (why.empty()) return why;
     }
     return why.empty() ? "a part's rows exceed on-chip memory" : why;
+} catch (const std::bad_alloc&) {
+    return kNoMemory;
 }
 
 std::string res_check(const ResPlan& plan, int nnz, const ResLimits& limits, int real)

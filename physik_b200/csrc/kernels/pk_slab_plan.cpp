@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <new>
 #include <numeric>
 #include <thread>
 
@@ -290,7 +291,7 @@ std::string build_layout(int n, const int* row_start, const int* col, const int*
         try {
             build_part(p, t);
         } catch (...) {  // nothing may leave a worker thread
-            errors[p] = "host memory exhausted while building the layout";
+            errors[p] = kNoMemory;
         }
     });
     for (int p = 0; p < parts; ++p)
@@ -579,7 +580,7 @@ std::string build_layout_sym(int n, const int* row_start, const int* col, const 
             }
             errors[p] = why.empty() ? why : first_why;  // the one-sub-part-per-group reason
         } catch (...) {
-            errors[p] = "host memory exhausted while building the layout";
+            errors[p] = kNoMemory;
         }
     });
     for (int p = 0; p < parts; ++p)
@@ -635,7 +636,7 @@ std::string build_layout_sym(int n, const int* row_start, const int* col, const 
         try {
             build_part(p, t);
         } catch (...) {
-            errors[p] = "host memory exhausted while building the layout";
+            errors[p] = kNoMemory;
         }
     });
     for (int p = 0; p < parts; ++p)
@@ -780,7 +781,7 @@ std::string build_layout_form(int n, const int* row_start, const int* col, const
 
 std::string build_slab_plan(int n, const int* row_start, const int* col, const int* lt_start, const int* lt_row,
                             const int* lt_block, const double* coords, int parts, SlabPlan& out, int form, bool wide)
-{
+try {
     out = SlabPlan{};
     if (n <= 0 || parts <= 0) return "empty system";
     std::vector<double> held;
@@ -817,12 +818,14 @@ std::string build_slab_plan(int n, const int* row_start, const int* col, const i
     out.launch_start = {0, parts};
     if (!out.sym) add_sends(out);
     return "";
+} catch (const std::bad_alloc&) {
+    return kNoMemory;
 }
 
 std::string build_slab_plan_batched(int n, const int* row_start, const int* col, const int* lt_start,
                                     const int* lt_row, const int* lt_block, const double* coords, const int* seg,
                                     int nseg, int max_blocks, SlabPlan& out, int form)
-{
+try {
     out = SlabPlan{};
     if (n <= 0 || nseg <= 0 || max_blocks <= 0) return "empty system";
     if (seg[0] != 0 || seg[nseg] != n) return "segments do not cover the rows";
@@ -995,6 +998,8 @@ std::string build_slab_plan_batched(int n, const int* row_start, const int* col,
     out.part_body = part_body;
     out.launch_start = launch_start;
     return "";
+} catch (const std::bad_alloc&) {
+    return kNoMemory;
 }
 
 namespace {

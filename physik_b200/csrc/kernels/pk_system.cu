@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <string>
 #include <type_traits>
 #include <memory>
@@ -685,7 +686,7 @@ void keep_layout(pk_system* s, std::vector<int>& col)
 // has not been tried yet; where it does not apply res_parts stays 0.  Synchronous.
 template <class Real>
 int ensure_resident(pk_system* s, bool bodies)
-{
+try {
     if (s->res_tried || !resident_allowed(s)) return PK_OK;
     s->res_tried = true;
     s->res_parts = 0;
@@ -755,6 +756,9 @@ int ensure_resident(pk_system* s, bool bodies)
     s->res_plan.smem_bytes = plan.smem_bytes;
     if (sizeof(Real) == 8) keep_layout(s, in.col);
     return PK_OK;
+} catch (const std::bad_alloc&) {  // no room on the host for it: the kernels without one
+    s->res_parts = 0;
+    return PK_OK;
 }
 
 // The rows pushed between blocks (at most two packets each), then the blocks' inboxes.
@@ -769,7 +773,7 @@ size_t part_inbox_bytes(int halo, int parts)
 // large a window, too long a row) leaves slab_parts at 0 and the reason in slab_reason.
 template <class Acc>
 int ensure_slab(pk_system* s)
-{
+try {
     const bool bodies = batched_solve(s);
     if (s->slab_tried && s->slab_for_bodies != bodies) reset_slab(s);  // batched mode changed
     if (s->slab_tried || !slab_allowed(s)) return PK_OK;
@@ -907,6 +911,9 @@ int ensure_slab(pk_system* s)
         s->part_parts = plan.parts;
     }
     return PK_OK;
+} catch (const std::bad_alloc&) {  // no room on the host for it: the kernels without one
+    s->slab_parts = s->part_parts = 0;
+    return PK_OK;
 }
 
 // Writes the FP64 stream's blocks, or (layout, once) its headers and columns.
@@ -931,7 +938,7 @@ int wide_fill(pk_system* s, const unsigned char* layout)
 // the kernel left to the library); where it does not apply either, part_parts stays 0 and the
 // ring kernel solves.
 int ensure_wide(pk_system* s)
-{
+try {
     if (s->wide_tried || s->res_parts > 0 || requested_kernel() != -1 || s->kernel_choice > 0 || s->dyn_count <= 0 ||
         !s->have_pattern)
         return PK_OK;
@@ -981,6 +988,9 @@ int ensure_wide(pk_system* s)
     PK_CHECK(cudaStreamSynchronize(s->stream));
     s->part_parts = plan.parts;
     keep_layout(s, in.col);
+    return PK_OK;
+} catch (const std::bad_alloc&) {  // no room on the host for it: the kernels without one
+    s->part_parts = 0;
     return PK_OK;
 }
 
@@ -3101,7 +3111,7 @@ extern "C" {
 PKCUDA_API int pk_slab_plan_batched_selfcheck(int n, const int* row_start, const int* col_index, const double* values,
                                               const double* x, const double* coords, const int* segment_row_start,
                                               int segment_count, int max_blocks, int form, double* y, int* info)
-{
+try {
     if (n <= 0 || segment_count <= 0 || max_blocks <= 0 || !row_start || !col_index || !values || !x || !y ||
         !segment_row_start)
         return fail(PK_ERR_ARG, "slab batched selfcheck");
@@ -3145,12 +3155,14 @@ PKCUDA_API int pk_slab_plan_batched_selfcheck(int n, const int* row_start, const
         info[5] = plan.sym ? 1 : 0;
     }
     return PK_OK;
+} catch (const std::bad_alloc&) {
+    return fail(PK_ERR_UNSUPPORTED, pk::kNoMemory);
 }
 
 PKCUDA_API int pk_res_plan_selfcheck(int n, const int* row_start, const int* col_index, const double* values,
                                      const double* x, const double* coords, const int* segment_row_start,
                                      int segment_count, int max_blocks, int precision, double* y, int* info)
-{
+try {
     if (n <= 0 || segment_count <= 0 || max_blocks == 0 || !row_start || !col_index || !values || !x || !y ||
         !coords || !segment_row_start)
         return fail(PK_ERR_ARG, "resident selfcheck");
@@ -3180,11 +3192,13 @@ PKCUDA_API int pk_res_plan_selfcheck(int n, const int* row_start, const int* col
         info[5] = plan.threads * plan.rpt;
     }
     return PK_OK;
+} catch (const std::bad_alloc&) {
+    return fail(PK_ERR_UNSUPPORTED, pk::kNoMemory);
 }
 
 PKCUDA_API int pk_slab_plan_selfcheck(int n, const int* row_start, const int* col_index, const double* values,
                                       const double* x, const double* coords, int parts, int form, double* y, int* info)
-{
+try {
     if (n <= 0 || parts <= 0 || !row_start || !col_index || !values || !x || !y)
         return fail(PK_ERR_ARG, "slab selfcheck");
     if (row_start[0] != 0) return fail(PK_ERR_ARG, "row_start[0] != 0");
@@ -3212,12 +3226,14 @@ PKCUDA_API int pk_slab_plan_selfcheck(int n, const int* row_start, const int* co
         info[4] = plan.sym ? 1 : 0;
     }
     return PK_OK;
+} catch (const std::bad_alloc&) {
+    return fail(PK_ERR_UNSUPPORTED, pk::kNoMemory);
 }
 
 PKCUDA_API int pk_part_plan_selfcheck(int n, const int* row_start, const int* col_index, const double* values,
                                       const double* x, const double* coords, int parts, int precision, double* y,
                                       int* info)
-{
+try {
     if (n <= 0 || parts <= 0 || !row_start || !col_index || !values || !x || !y)
         return fail(PK_ERR_ARG, "part selfcheck");
     if (row_start[0] != 0) return fail(PK_ERR_ARG, "row_start[0] != 0");
@@ -3245,6 +3261,8 @@ PKCUDA_API int pk_part_plan_selfcheck(int n, const int* row_start, const int* co
         info[4] = static_cast<int>(plan.halo_src.size());
     }
     return PK_OK;
+} catch (const std::bad_alloc&) {
+    return fail(PK_ERR_UNSUPPORTED, pk::kNoMemory);
 }
 
 PKCUDA_API int pk_ring_tiling_selfcheck(int precision, int n, const int* row_start, const int* col_index,
