@@ -141,8 +141,9 @@ std::string build_slab_plan(int n, const int* row_start, const int* col, const i
 // place in an order).
 const double* finite_coords(int n, const double* coords, std::vector<double>& held);
 
-// Why a layout whose build ran out of host memory does not apply.
-constexpr const char* kNoMemory = "host memory exhausted while building the layout";
+// Why a layout whose build ran out of host memory does not apply (short: a std::string of it
+// must need no memory).
+constexpr const char* kNoMemory = "no host memory";
 
 // f(i, thread) for i in [0, count) on the layout builds' host threads (thread <
 // plan_thread_count()); each i must write only its own outputs.

@@ -1,56 +1,90 @@
-"""Layouts that find no host memory (CPU): a status, no exception through the C ABI.
+"""Layouts that find no host memory (CPU): a reason, no exception.
 
-A child process lowers its address-space limit to a little above what it uses, more at every
-call, and asks the self-checks for layouts of a band of 120,000 rows: whatever allocation fails, the
-call must return, with an error until the layout fits.
+The planners are compiled with an `operator new` that fails once a chosen number of allocations has
+succeeded.  For every such number, up to the one with which the layout is built, each planner
+must return a reason; the runtime then solves without the layout, and nothing leaves a C entry.
 """
+import os
 import subprocess
-import sys
-
-import pytest
 
 from physik_b200 import _lib as L
 
-CHILD = r"""
-import ctypes as C, os, resource, sys
-# one thread: the C library ends a process whose new thread finds no memory for its local data
-os.sched_setaffinity(0, {min(os.sched_getaffinity(0))})
-sys.path.insert(0, sys.argv[1])
-import numpy as np
-from physik_b200 import _lib as L
-kind = sys.argv[2]
-n = 120000 if kind != "resident" else 60000
-width = np.minimum(8, n - np.arange(n))
-rs = np.concatenate([[0], np.cumsum(width)]).astype(np.int32)
-col = (np.arange(rs[-1]) - np.repeat(rs[:-1], width) + np.repeat(np.arange(n), width)).astype(np.int32)
-vals, x, y = np.ones(9 * len(col)), np.ones((n, 3)), np.zeros((n, 3))
-coords, seg, info = np.zeros((n, 3)), np.array([0, n], np.int32), np.zeros(8, np.int32)
-coords[:, 0] = np.arange(n)
-p = lambda a: a.ctypes.data_as(C.c_void_p)
-head = (n, p(rs), p(col), p(vals), p(x), p(coords))
-calls = {
-    "part64": lambda: L.PK.pk_part_plan_selfcheck(*head, 148, 2, p(y), p(info)),
-    "part32": lambda: L.PK.pk_part_plan_selfcheck(*head, 148, 1, p(y), p(info)),
-    "slab": lambda: L.PK.pk_slab_plan_selfcheck(*head, 148, 0, p(y), p(info)),
-    "batched": lambda: L.PK.pk_slab_plan_batched_selfcheck(*head, p(seg), 1, 148, 0, p(y), p(info)),
-    "resident": lambda: L.PK.pk_res_plan_selfcheck(*head, p(seg), 1, 148, 1, p(y), p(info)),
+SOURCE = r"""
+#include "pk_res_plan.h"
+#include "pk_slab_plan.h"
+#include <atomic>
+#include <cstdio>
+#include <cstdlib>
+#include <new>
+static std::atomic<long> left{-1};
+void* operator new(std::size_t size)
+{
+    if (left.load() >= 0 && left.fetch_sub(1) <= 0) {
+        left = 0;  // and all later ones
+        throw std::bad_alloc();
+    }
+    if (void* p = std::malloc(size ? size : 1)) return p;
+    throw std::bad_alloc();
 }
-used = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
-hard = resource.getrlimit(resource.RLIMIT_AS)[1]
-results = []
-for mb in list(range(1, 40, 3)) + [60, 90, 130, 180, 260]:
-    resource.setrlimit(resource.RLIMIT_AS, (used + (mb << 20), hard))
-    results.append(calls[kind]())
-resource.setrlimit(resource.RLIMIT_AS, (hard, hard))
-results.append(calls[kind]())
-print(*results)
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, std::size_t) noexcept { std::free(p); }
+
+int main()
+{
+    constexpr int n = 5000, band = 6;
+    std::vector<int> rs(1, 0), col, lts(n + 1, 0), ltr, ltb;
+    for (int r = 0; r < n; ++r) {
+        for (int c = r; c < n && c < r + band; ++c) col.push_back(c);
+        rs.push_back((int)col.size());
+    }
+    for (int r = 0; r < n; ++r) {
+        for (int c = r > band - 1 ? r - band + 1 : 0; c < r; ++c) {
+            ltr.push_back(c);
+            ltb.push_back(rs[c] + r - c);
+        }
+        lts[r + 1] = (int)ltr.size();
+    }
+    std::vector<double> xyz(3 * n, 0.0);
+    for (int r = 0; r < n; ++r) xyz[3 * r] = r;
+    const int seg[2] = {0, n};
+    for (int kind = 0; kind < 6; ++kind) {
+        long refused = 0;
+        for (long k = 0;; k += 1 + k / 40) {
+            std::string why;
+            {
+                pk::SlabPlan slab;
+                pk::ResPlan res;
+                pk::ResLimits limits;
+                limits.blocks = 148;
+                left = k;
+                if (kind < 3)
+                    why = pk::build_slab_plan(n, rs.data(), col.data(), lts.data(), ltr.data(), ltb.data(), xyz.data(),
+                                              16, slab, kind == 1 ? pk::kSlabSym : pk::kSlabFull, kind == 2);
+                else if (kind == 3)
+                    why = pk::build_slab_plan_batched(n, rs.data(), col.data(), lts.data(), ltr.data(), ltb.data(),
+                                                      xyz.data(), seg, 1, 16, slab, pk::kSlabFull);
+                else
+                    why = pk::build_res_plan(n, rs.data(), col.data(), lts.data(), ltr.data(), ltb.data(), xyz.data(),
+                                             seg, 1, limits, kind == 4 ? 4 : 8, res);
+                left = -1;
+            }
+            if (why.empty()) break;
+            ++refused;
+        }
+        std::printf("%ld\n", refused);
+    }
+}
 """
 
 
-@pytest.mark.parametrize("kind", ["part64", "part32", "slab", "batched", "resident"])
-def test_a_call_without_memory_returns_an_error(kind):
-    child = subprocess.run([sys.executable, "-c", CHILD, L.ROOT, kind], capture_output=True, text=True, timeout=300)
-    assert child.returncode == 0, (child.returncode, child.stderr[-500:])
-    results = [int(r) for r in child.stdout.split()]
-    assert results[-1] == 0 and any(r < 0 for r in results)
-    assert set(results) <= {0, L.PK_ERR_UNSUPPORTED}, results
+def test_a_layout_without_memory_gives_a_reason(tmp_path):
+    kernels = os.path.join(L.ROOT, "physik_b200", "csrc", "kernels")
+    source, program = tmp_path / "plans.cpp", tmp_path / "plans"
+    source.write_text(SOURCE)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-I", kernels, str(source),
+                    os.path.join(kernels, "pk_slab_plan.cpp"), os.path.join(kernels, "pk_res_plan.cpp"), "-o",
+                    str(program)], check=True)
+    run = subprocess.run([str(program)], capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, (run.returncode, run.stderr[-500:])
+    refused = [int(r) for r in run.stdout.split()]
+    assert len(refused) == 6 and min(refused) > 10, refused
