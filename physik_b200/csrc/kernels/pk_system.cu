@@ -254,7 +254,9 @@ struct pk_system {
     DevBuf slab_qs, slab_ss;
     // coupled part-resident PCG (pk_pcg_part.cu): shares the buffers above
     bool wide_tried = false;
-    // FP64 layouts of patterns with transient blocks (layout_waits)
+    // FP64 layouts of patterns that may be short-lived (layout_waits)
+    bool solved = false;          // a solve ran
+    bool rebuilt = false;         // the nodes were set again after one, and no layout since
     bool nodes_solved = false;    // a solve ran since the nodes were set
     bool replaced = false;        // the pattern replaced one that had been solved
     int pattern_solves = 0;       // solves on this pattern
@@ -651,17 +653,18 @@ bool resident_allowed(const pk_system* s)
     return s->precision == PK_PREC_FP64 ? rk == -1 : (rk == -1 || rk == 3) && requested_slab_form() == pk::kSlabFull;
 }
 
-// A pattern with the blocks of connections or host-emitted contributions that replaces a solved
-// one may last a frame (a drag, contacts), and a layout takes the host 0.2 to 0.7 us a row: an
-// FP64 step with new connections at 36 k rows took 29.9 ms with the layout against 3.4 on the ring
-// kernel, which needs none; at 18 k rows 6.6 against 3.4, at 648 0.84 against 0.62.  Such a
+// A pattern may last a frame: one with the blocks of connections or host-emitted contributions
+// that replaces a solved one (a drag, contacts), or the first of a scene set again (tets cut away).
+// A layout takes the host 0.2 to 0.7 us a row: an FP64 step with new connections at 36 k rows took
+// 29.9 ms with the layout against 3.4 on the ring kernel, which needs none (at 18 k rows 6.6
+// against 3.4, at 648 0.84 against 0.62), one after a node was cut away 47 against 20.  Such a
 // pattern is first solved on the ring kernel, about as many times as the layout is worth (it
-// saves 10 to 20 us an iteration).  The bodies' own pattern never waits, so that a solve does not depend on
-// the steps before it; FP32 storage has no kernel as fast without a layout.
+// saves 10 to 20 us an iteration).  Otherwise the bodies' own pattern does not wait, so that the
+// end of a connection leaves no trace; FP32 storage has no kernel as fast without a layout.
 bool layout_waits(const pk_system* s)
 {
-    return s->precision == PK_PREC_FP64 && s->replaced && (s->conn_count > 0 || s->ext_on) &&
-           s->pattern_solves <= s->dyn_count / 8192;
+    return s->precision == PK_PREC_FP64 && s->pattern_solves <= s->dyn_count / 8192 &&
+           (s->rebuilt || (s->replaced && (s->conn_count > 0 || s->ext_on)));
 }
 
 // The current pattern (columns `col`) is the one whose layout is kept, and it may have one.
@@ -1058,6 +1061,7 @@ int ensure_slab_any(pk_system* s)
         s->waited = true;
         return PK_OK;
     }
+    s->rebuilt = false;
     const int rc = ensure_resident<double>(s, false);
     return rc ? rc : ensure_wide(s);
 }
@@ -1379,7 +1383,7 @@ int run_pcg(pk_system* s, const pk_step_params& p, int skip_on_flags)
         const int rc = ensure_slab_any(s);
         if (rc) return rc;
         ++s->pattern_solves;
-        s->nodes_solved = true;
+        s->nodes_solved = s->solved = true;
     }
     const int kernel = solve_kernel(s);
     s->last_kernel = kernel;
@@ -1934,6 +1938,7 @@ PKCUDA_API int pk_system_set_nodes(pk_system* s, int node_count, const int* node
     PK_CHECK(cudaSetDevice(s->device));
     s->node_count = node_count;
     s->have_layout_x = false;
+    s->rebuilt = s->solved;
     s->nodes_solved = false;
     s->kept.valid = false;
     s->have_snapshot = false;
@@ -2749,7 +2754,7 @@ PKCUDA_API int pk_system_autotune(pk_system* s, const pk_step_params* p, int rep
         return fail(PK_ERR_STATE, "autotune needs an assembled system (step once first)");
     PK_CHECK(cudaSetDevice(s->device));
     if (const int rc = fetch_stats(s)) return rc;  // the timed solves overwrite them
-    s->replaced = false;  // the candidates are those of a pattern that stays
+    s->replaced = s->rebuilt = false;  // the candidates are those of a pattern that stays
     PK_CHECK(cudaStreamSynchronize(s->stream));
     drop_graph(s);
     repeats = std::max(1, repeats);

@@ -3,8 +3,8 @@
 Point connections join the pattern; dragged from node to node they give every step another one.
 A layout for the resident or the part-resident kernel costs the host more than such a step, so
 a joined pattern that replaces a solved one starts on the ring kernel and gets its layout when it
-has lasted; a world's first pattern and the bodies' own get it at once, the latter kept while others
-wait.  The kernels differ in the order of sums
+has lasted; so does the first of a scene set again when tets were cut away.  A world's first pattern
+and the bodies' own get it at once, the latter kept while others wait.  The kernels differ in the order of sums
 only: against a world that always steps on the ring kernel within the FP64 tolerances of
 test_gpu_resident.py, and with and without a captured step bit for bit.
 """
@@ -74,6 +74,33 @@ def test_the_bodies_own_layout_is_kept_while_others_wait(monkeypatch):
         assert u.pcg_launched() == "pcg_part_kernel"
     for p, q in zip(w.state(f64=True), plain.state(f64=True)):
         np.testing.assert_array_equal(p, q)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_a_scene_set_again_waits_for_its_layout(graph, monkeypatch):
+    scene = meshes.small_box(9, 8, 7)
+    tets, pinned = scene.bodies[0].tets, scene.bodies[0].pinned
+    counts = np.bincount(tets.ravel())
+    corners = [n for n in np.argsort(counts, kind="stable") if not pinned[n]][:2]
+
+    def run(w):
+        names = []
+        for k in range(7):
+            if k in (2, 3):  # a corner node leaves the solve with its tets
+                for t in np.nonzero((tets == corners[k - 2]).any(1))[0]:
+                    w.X.PHYSIK_SetTetActive(w.h, w.components[0], int(t), 0)
+            w.step()
+            assert w.cg_stats()["flags"] & L.FLAG_INTEGRATED
+            names.append(w.pcg_launched())
+        return names, w.state(f64=True)
+
+    w = SimWorld(scene, precision="fp64")
+    w.set_graph(graph)
+    names, (x, v) = run(w)
+    assert names == ["pcg_res_kernel"] * 2 + [RING] * 2 + ["pcg_res_kernel"] * 3
+    monkeypatch.setenv("PK_PCG_KERNEL", "ring")
+    _, (x2, v2) = run(SimWorld(scene, precision="fp64"))
+    assert rel(x, x2) <= 1e-12 and rel(v, v2) <= 1e-10
 
 
 def test_the_wait_grows_with_the_rows():
